@@ -330,47 +330,6 @@ __global__ void __launch_bounds__(256) k_norm2(const typename C2<R>::T* __restri
   block_reduce_store<256>(a, d_part, blockIdx.x);
 }
 
-// Re(w * conj(a) b), w in {1, -i, -1, i} indexed by wk (0..3): conj(a)b = R + iI
-__device__ __forceinline__ double re_wab(int wk, double ar, double ai, double br, double bi) {
-  double R = ar * br + ai * bi, I = ar * bi - ai * br;
-  switch (wk & 3) {
-    case 0: return R;
-    case 1: return I;   // -i*(R+iI) = I - iR
-    case 2: return -R;
-    default: return -I; //  i*(R+iI) = -I + iR
-  }
-}
-
-// <psi|P|psi>, (P psi)_i = (-i)^ny (-1)^popc(i&z) psi_{i^x}
-template <typename R>
-__global__ void __launch_bounds__(256) k_pauli(const typename C2<R>::T* __restrict__ s, uint64_t N, uint64_t xm,
-                                               uint64_t zm, int ny, double* d_part) {
-  DD acc{0, 0};
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  if (xm == 0) {
-    // diagonal: (-1)^popc(i & z) p_i   (ny = 0 when x = 0)
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
-      double p = p_of<R>(s[i]);
-      two_sum_acc(acc, (__popcll(i & zm) & 1) ? -p : p);
-    }
-  } else {
-    const int hb = 63 - __clzll(xm);
-    const uint64_t half = N >> 1;
-    for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < half; q += stride) {
-      uint64_t i = ((q >> hb) << (hb + 1)) | (q & ((1ULL << hb) - 1));
-      uint64_t j = i ^ xm;
-      auto a = s[i];
-      auto b = s[j];
-      // term i: Re(conj(a_i) w_i a_j), term j: Re(conj(a_j) w_j a_i)
-      int wi = ny + ((__popcll(i & zm) & 1) ? 2 : 0);
-      int wj = ny + ((__popcll(j & zm) & 1) ? 2 : 0);
-      double v = re_wab(wi, a.x, a.y, b.x, b.y) + re_wab(wj, b.x, b.y, a.x, a.y);
-      two_sum_acc(acc, v);
-    }
-  }
-  block_reduce_store<256>(acc, d_part, blockIdx.x);
-}
-
 template <typename R>
 __global__ void __launch_bounds__(256) k_expect1q(const typename C2<R>::T* __restrict__ s, uint64_t N, int bit,
                                                   Mat<double> o, double* d_part) {
@@ -853,15 +812,6 @@ cudaError_t launch_norm2(const void* s, int precision, int n, double* d_part, in
   uint64_t N = 1ULL << n;
   if (precision == QG_C64) k_norm2<float><<<nblocks, 256, 0, st>>>((const float2*)s, N, d_part);
   else k_norm2<double><<<nblocks, 256, 0, st>>>((const double2*)s, N, d_part);
-  counted();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pauli_expect(const void* s, int precision, int n, uint64_t xmask, uint64_t zmask, int ny,
-                                double* d_part, int nblocks, cudaStream_t st) {
-  uint64_t N = 1ULL << n;
-  if (precision == QG_C64) k_pauli<float><<<nblocks, 256, 0, st>>>((const float2*)s, N, xmask, zmask, ny, d_part);
-  else k_pauli<double><<<nblocks, 256, 0, st>>>((const double2*)s, N, xmask, zmask, ny, d_part);
   counted();
   return cudaGetLastError();
 }

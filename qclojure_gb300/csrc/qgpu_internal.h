@@ -314,8 +314,19 @@ struct ReduceScratch {
 };
 cudaError_t launch_probabilities(const void* s, int precision, int n, double* d_p, cudaStream_t st);
 cudaError_t launch_norm2(const void* s, int precision, int n, double* d_part, int nblocks, cudaStream_t st);
-cudaError_t launch_pauli_expect(const void* s, int precision, int n, uint64_t xmask, uint64_t zmask, int ny,
-                                double* d_part, int nblocks, cudaStream_t st);
+// Expectations of many Pauli strings of one state in one launch (pauli.cu). build() groups
+// `count` concatenated strings of n characters by what they sum (false: a character outside
+// IXYZ); `table` goes to the device, d_partial holds partial_bytes, and d_out[order[k]]
+// receives string k's value.
+struct PauliPlan {
+  int ngroups = 0, nstrings = 0, nchunks = 1;
+  size_t string_bytes = 0, partial_bytes = 0;
+  std::vector<int> order;
+  std::vector<unsigned char> table;
+  bool build(int n, int count, const char* text);
+};
+cudaError_t launch_pauli_plan(const void* s, int precision, int n, const PauliPlan& p, const void* d_table,
+                              void* d_partial, double* d_out, cudaStream_t st);
 cudaError_t launch_expect_1q(const void* s, int precision, int n, int bit, const double* o8, double* d_part,
                              int nblocks, cudaStream_t st);
 cudaError_t launch_inner(const void* a, const void* b, int precision, int n, double* d_part, int nblocks,

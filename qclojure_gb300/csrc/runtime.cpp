@@ -438,22 +438,50 @@ static int st_norm2(State* s, double* out, std::string* err) {
   return fetch_dd(s, s->d_part, s->nblocks, out, err);
 }
 
-static int st_pauli(State* s, const char* pauli, double* out, std::string* err) {
-  uint64_t xm = 0, zm = 0;
-  int ny = 0;
-  for (int q = 0; q < s->n; ++q) {
-    uint64_t b = 1ULL << (s->n - 1 - q);
-    char ch = pauli[q];
-    if (ch == 'X') xm |= b;
-    else if (ch == 'Y') { xm |= b; zm |= b; ++ny; }
-    else if (ch == 'Z') zm |= b;
-    else if (ch != 'I') {
+// values[k] = <psi|P_k|psi> of `count` concatenated Pauli strings, kPauliBatch strings per launch.
+constexpr int kPauliBatch = 4096;
+static int st_pauli_strings(State* s, int count, const char* text, double* values, std::string* err) {
+  for (int at = 0; at < count; at += kPauliBatch) {
+    const int k = std::min(kPauliBatch, count - at);
+    PauliPlan plan;
+    if (!plan.build(s->n, k, text + (size_t)at * s->n)) {
       *err = "Pauli strings use the characters I, X, Y, Z";
       return QG_ERR_INVALID_ARG;
     }
+    const size_t table = (plan.table.size() + 255) / 256 * 256, sums = (plan.partial_bytes + 255) / 256 * 256;
+    unsigned char* d = nullptr;
+    std::vector<double> got((size_t)k);
+    CK(cudaMallocAsync((void**)&d, table + sums + sizeof(double) * k, s->stream), "alloc pauli");
+    double* d_out = reinterpret_cast<double*>(d + table + sums);
+    cudaError_t e = cudaMemcpyAsync(d, plan.table.data(), plan.table.size(), cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = launch_pauli_plan(s->d, s->prec, s->n, plan, d, d + table, d_out, s->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(got.data(), d_out, sizeof(double) * k, cudaMemcpyDeviceToHost, s->stream);
+    const cudaError_t se = cudaStreamSynchronize(s->stream);
+    cudaFreeAsync(d, s->stream);
+    if (e != cudaSuccess || se != cudaSuccess) return cuda_fail(err, e != cudaSuccess ? e : se, "pauli");
+    for (int i = 0; i < k; ++i) values[at + i] = got[(size_t)plan.order[i]];
   }
-  CK(launch_pauli_expect(s->d, s->prec, s->n, xm, zm, ny & 3, s->d_part, s->nblocks, s->stream), "pauli");
-  return fetch_dd(s, s->d_part, s->nblocks, out, err);
+  return QG_OK;
+}
+
+// sum_k c_k <P_k>, added in string order like (reduce + ...); values (count of them) may be null
+static int st_hamiltonian(State* s, int count, const double* coeffs, const char* text, double* values, double* out,
+                          std::string* err) {
+  std::vector<double> own;
+  if (!values) {
+    own.resize((size_t)std::max(count, 1));
+    values = own.data();
+  }
+  const int rc = st_pauli_strings(s, count, text, values, err);
+  if (rc != QG_OK) return rc;
+  double energy = 0;
+  for (int k = 0; k < count; ++k) {
+    const double term = coeffs[k] * values[k];
+    energy = k == 0 ? term : energy + term;
+  }
+  *out = energy;
+  return QG_OK;
 }
 
 static int st_expect1q(State* s, const double* o8, int target, double* out, std::string* err) {
@@ -912,13 +940,7 @@ static int job_results(Ctx* c, Job* j, std::unique_ptr<State> st, cudaStream_t s
   if (rc == QG_OK && (sp.flags & QG_RES_HAMILTONIAN)) {
     j->term_values.assign(sp.n_terms, 0.0);
     double energy = 0;
-    for (int k = 0; rc == QG_OK && k < sp.n_terms; ++k) {
-      double v;
-      rc = st_pauli(st.get(), sp.paulis.data() + (size_t)k * j->n, &v, &err);
-      j->term_values[k] = v;
-      double term = sp.coeffs[k] * v;
-      energy = (k == 0) ? term : energy + term;  // (reduce + ...) in term order
-    }
+    rc = st_hamiltonian(st.get(), sp.n_terms, sp.coeffs.data(), sp.paulis.data(), j->term_values.data(), &energy, &err);
     j->energy = energy;
     if (rc == QG_OK) j->has |= QG_RES_HAMILTONIAN;
   }
@@ -2369,7 +2391,7 @@ int qg_state_pauli_expectation(void* state, const char* pauli, double* out) {
   State* s = (State*)state;
   cudaSetDevice(s->ctx->device);
   std::string err;
-  return state_err(s, st_pauli(s, pauli, out, &err), err);
+  return state_err(s, st_pauli_strings(s, 1, pauli, out, &err), err);
 }
 
 int qg_state_hamiltonian(void* state, int32_t n_terms, const double* coeffs, const char* paulis, double* out) {
@@ -2378,13 +2400,8 @@ int qg_state_hamiltonian(void* state, int32_t n_terms, const double* coeffs, con
   cudaSetDevice(s->ctx->device);
   std::string err;
   double energy = 0;
-  for (int k = 0; k < n_terms; ++k) {
-    double v;
-    int rc = st_pauli(s, paulis + (size_t)k * s->n, &v, &err);
-    if (rc != QG_OK) return state_err(s, rc, err);
-    double term = coeffs[k] * v;
-    energy = k == 0 ? term : energy + term;
-  }
+  const int rc = st_hamiltonian(s, n_terms, coeffs, paulis, nullptr, &energy, &err);
+  if (rc != QG_OK) return state_err(s, rc, err);
   *out = energy;
   return QG_OK;
 }
@@ -3283,15 +3300,11 @@ static int sweep_energies(Sweep* sw, const int32_t* term_offsets, const double* 
     for (size_t m = 0; m < g.members.size(); ++m) {
       const int ci = g.members[m];
       double energy = 0;
-      for (int t = term_offsets[ci]; t < term_offsets[ci + 1]; ++t) {
-        double v;
-        const int rc = st_pauli(g.views[m].get(), pauli_strings + char_off[ci] + (int64_t)(t - term_offsets[ci]) * g.n,
-                                &v, err);
-        if (rc != QG_OK) return rc;
-        const double term = coefficients[t] * v;
-        energy = (t == term_offsets[ci]) ? term : energy + term;
-        ++*launches;
-      }
+      const int t0 = term_offsets[ci], nt = term_offsets[ci + 1] - t0;
+      const int rc = st_hamiltonian(g.views[m].get(), nt, coefficients + t0, pauli_strings + char_off[ci], nullptr,
+                                    &energy, err);
+      if (rc != QG_OK) return rc;
+      *launches += 2 * ((nt + kPauliBatch - 1) / kPauliBatch);
       energies[ci] = energy;
     }
   }
