@@ -21,8 +21,11 @@
 
 namespace qg {
 
-struct dfc {  // complex double-float: (re.hi, re.lo, im.hi, im.lo)
-  float rh, rl, ih, il;
+// complex double-float. The leading floats of both parts lie side by side, and so do the
+// trailing ones: each couple is one operand of the packed FP32 instructions (f32x2), and
+// 16 bytes in memory are (re.hi, im.hi, re.lo, im.lo).
+struct dfc {
+  float rh, ih, rl, il;
 };
 
 // IEEE double -> (hi, lo): hi keeps the leading 24 significand bits (truncated),

@@ -943,7 +943,7 @@ class PassGen {
       const std::string F = "F" + std::to_string(cr);
       std::string lit;  // the phase as a value of the register type
       if (t.cls == PH_GENERAL)
-        lit = df_ ? "dfc{" + h(t, 0) + ", " + l(t, 0) + ", " + h(t, 1) + ", " + l(t, 1) + "}"
+        lit = df_ ? "dfc{" + h(t, 0) + ", " + h(t, 1) + ", " + l(t, 0) + ", " + l(t, 1) + "}"
                   : "make_float2(" + h(t, 0) + ", " + h(t, 1) + ")";
       else
         lit = rot(unit_power(t), one);

@@ -10,8 +10,8 @@
 //     16-byte stores), with the pass geometry supplied by P;
 //   - the complex arithmetic of the two policies the generator emits:
 //       complex128 as double-float pairs (hi + lo floats, about 48 bits) on the
-//       FP32 pipes, with error-free products (FMA) and sums (TwoSum); results
-//       are left unnormalised (the pair (s, t) of a rounded sum and its
+//       FP32 pipes, with error-free products (FMA) and sums (TwoSum), real and
+//       imaginary part together in packed instructions; results are left unnormalised (the pair (s, t) of a rounded sum and its
 //       collected error) and renormalised by the generated code after a few
 //       operations on a register and before it is stored;
 //       complex64 in FP32 with FMA contraction.
@@ -48,55 +48,149 @@ __device__ __forceinline__ int swz(int l) {
 }
 
 // ---------------------------------------------------------------------------
-// double-float scalars. A value is the unevaluated sum h + l of two floats.
-// tprod: a * x with a a constant pair (ah, al) -> (p, e), p = fl(ah*xh) and e
-// its exact error plus the cross terms ah*xl and al*xh (AL = false: al == 0).
+// Packed FP32 (f32x2): one instruction works on two floats. It has the same rate per float as
+// the scalar form (a probe on GB300: 123 of 128 floats per clock and SM either way) for half
+// the issue slots, and the double-float passes are bound by issue and by the latency of their
+// chains, not by the FP32 lanes: the two halves of an operand are the real and the imaginary
+// part, which every gate treats alike. Each lane does the operations of the scalar form
+// (products, FMA error terms, TwoSum) in the same order, so results are the same bits.
+// There is no packed negation: differences and negated constants take its place. ptxas contracts
+// a packed product into the packed sums that use it when nothing else does (unlike the scalar
+// .rn forms), which would break a TwoSum of it: mul2 is for products whose FMA error term uses
+// the rounded product too, and for exact ones; mul2_rn rounds lane by lane.
 // ---------------------------------------------------------------------------
-template <bool AL>
-__device__ __forceinline__ void tprod(float ah, float al, float xh, float xl, float& p, float& e) {
-  p = ah * xh;
-  e = fmaf(ah, xh, -p);
-  e = fmaf(ah, xl, e);
-  if (AL) e = fmaf(al, xh, e);
+__device__ __forceinline__ u64 pk(float a, float b) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
+__device__ __forceinline__ void unpk(u64 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 sub2(u64 a, u64 b) {
+  u64 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+  u64 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 mul2_rn(u64 a, u64 b) {
+  float ax, ay, bx, by;
+  unpk(a, ax, ay);
+  unpk(b, bx, by);
+  return pk(__fmul_rn(ax, bx), __fmul_rn(ay, by));
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a complex double-float as two operands: leading floats (re, im), trailing floats (re, im)
+struct cp {
+  u64 h, l;
+};
+__device__ __forceinline__ cp pack(const dfc& x) { return cp{pk(x.rh, x.ih), pk(x.rl, x.il)}; }
+__device__ __forceinline__ cp pack_swapped(const dfc& x) { return cp{pk(x.ih, x.rh), pk(x.il, x.rl)}; }
+__device__ __forceinline__ dfc unpack(const cp& x) {
+  dfc y;
+  unpk(x.h, y.rh, y.ih);
+  unpk(x.l, y.rl, y.il);
+  return y;
+}
+// a constant pair per lane (re lane: ah + al, im lane: bh + bl) and its negation
+struct kp {
+  u64 h, l, nh, nl;
+};
+__device__ __forceinline__ kp konst(float ah, float al, float bh, float bl) {
+  return kp{pk(ah, bh), pk(al, bl), pk(-ah, -bh), pk(-al, -bl)};
+}
+__device__ __forceinline__ kp konst(float h, float l) { return konst(h, l, h, l); }
+
 // Knuth's TwoSum: s = fl(a + b), e = (a + b) - s exactly.
-__device__ __forceinline__ void tsum(float a, float b, float& s, float& e) {
-  s = a + b;
-  const float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
+__device__ __forceinline__ void tsum(u64 a, u64 b, u64& s, u64& e) {
+  s = add2(a, b);
+  const u64 bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+// the same for a - b
+__device__ __forceinline__ void tdiff(u64 a, u64 b, u64& s, u64& e) {
+  s = sub2(a, b);
+  const u64 bb = sub2(s, a);
+  e = sub2(sub2(a, sub2(s, bb)), add2(b, bb));
+}
+// k * x: p = fl(kh * xh) and n = -(its exact error plus the cross terms kh * xl and kl * xh)
+template <bool KL>
+__device__ __forceinline__ void tprod(const kp& k, const cp& x, u64& p, u64& n) {
+  p = mul2(k.h, x.h);
+  n = fma2(k.nh, x.h, p);
+  n = fma2(k.nh, x.l, n);
+  if (KL) n = fma2(k.nl, x.h, n);
+}
+// the same with the signs exchanged: n = -fl(kh * xh), e = +(error and cross terms)
+template <bool KL>
+__device__ __forceinline__ void tprod_neg(const kp& k, const cp& x, u64& n, u64& e) {
+  n = mul2(k.nh, x.h);
+  e = fma2(k.h, x.h, n);
+  e = fma2(k.h, x.l, e);
+  if (KL) e = fma2(k.l, x.h, e);
+}
+// k * x
+template <bool KL>
+__device__ __forceinline__ cp prod(const kp& k, const cp& x) {
+  u64 n, e;
+  tprod_neg<KL>(k, x, n, e);
+  return cp{mul2_rn(k.h, x.h), e};
 }
 // a*x + b*y, unnormalised
 template <bool AL, bool BL>
-__device__ __forceinline__ void dot2(float ah, float al, float xh, float xl, float bh, float bl, float yh, float yl,
-                                     float& sh, float& sl) {
-  float p1, e1, p2, e2, err;
-  tprod<AL>(ah, al, xh, xl, p1, e1);
-  tprod<BL>(bh, bl, yh, yl, p2, e2);
-  tsum(p1, p2, sh, err);
-  sl = (e1 + e2) + err;
+__device__ __forceinline__ cp dot2(const kp& a, const cp& x, const kp& b, const cp& y) {
+  u64 p1, n1, p2, n2, s, err;
+  tprod<AL>(a, x, p1, n1);
+  tprod<BL>(b, y, p2, n2);
+  tsum(p1, p2, s, err);
+  return cp{s, sub2(err, add2(n1, n2))};
 }
-// x + y, unnormalised
-__device__ __forceinline__ void add2(float xh, float xl, float yh, float yl, float& sh, float& sl) {
-  float err;
-  tsum(xh, yh, sh, err);
-  sl = (xl + yl) + err;
+// x + y and x - y, unnormalised
+__device__ __forceinline__ cp sum(const cp& x, const cp& y) {
+  u64 s, err;
+  tsum(x.h, y.h, s, err);
+  return cp{s, add2(add2(x.l, y.l), err)};
+}
+__device__ __forceinline__ cp diff(const cp& x, const cp& y) {
+  u64 s, err;
+  tdiff(x.h, y.h, s, err);
+  return cp{s, add2(sub2(x.l, y.l), err)};
+}
+// x + k*y, unnormalised
+template <bool KL>
+__device__ __forceinline__ cp axpy(const kp& k, const cp& x, const cp& y) {
+  u64 n, e, s, err;
+  tprod_neg<KL>(k, y, n, e);
+  tdiff(x.h, n, s, err);
+  return cp{s, add2(add2(x.l, e), err)};
+}
+// k*y - x, unnormalised
+template <bool KL>
+__device__ __forceinline__ cp axmy(const kp& k, const cp& x, const cp& y) {
+  u64 p, n, s, err;
+  tprod<KL>(k, y, p, n);
+  tdiff(p, x.h, s, err);
+  return cp{s, sub2(err, add2(x.l, n))};
 }
 // Fast2Sum: bring the collected error back under the leading float. The
 // generated code applies it to a register after a few products (and before a
 // register goes to shared memory): left to grow, the low float random-walks to
 // a sizeable fraction of the high one and its roundings no longer average out
 // (the state's norm then drifts by ~1e-11 over a thousand gates).
-__device__ __forceinline__ void fast2(float& h, float& l) {
-  const float s = h + l;
-  l = l - (s - h);
-  h = s;
-}
-// normalised pair (|l| <= ulp(h)/2) for the conversion to IEEE doubles
-__device__ __forceinline__ void norm2(float& h, float& l) {
-  float s, e;
-  tsum(h, l, s, e);
-  h = s;
-  l = e;
+__device__ __forceinline__ cp fast2(const cp& x) {
+  const u64 s = add2(x.h, x.l);
+  return cp{s, sub2(x.l, sub2(s, x.h))};
 }
 
 // ---- complex double-float ------------------------------------------------
@@ -108,145 +202,85 @@ struct DF {
     return dfc{v.x, v.y, v.z, v.w};
   }
   static __device__ __forceinline__ void st_work(unsigned char* b, int pos, const V& v) {
-    reinterpret_cast<float4*>(b)[pos] = make_float4(v.rh, v.rl, v.ih, v.il);
+    reinterpret_cast<float4*>(b)[pos] = make_float4(v.rh, v.ih, v.rl, v.il);
   }
   static __device__ __forceinline__ V ld_doubles(const unsigned char* b, int pos) {
     return qg::load_dfc(reinterpret_cast<const double2*>(b)[pos]);
   }
-  static __device__ __forceinline__ void st_doubles(unsigned char* b, int pos, V v) {
-    norm2(v.rh, v.rl);
-    norm2(v.ih, v.il);
-    reinterpret_cast<double2*>(b)[pos] = qg::store_dfc(v);
+  // normalised pairs (|l| <= ulp(h)/2) for the conversion to IEEE doubles
+  static __device__ __forceinline__ void st_doubles(unsigned char* b, int pos, const V& v) {
+    const cp x = pack(v);
+    cp y;
+    tsum(x.h, x.l, y.h, y.l);
+    reinterpret_cast<double2*>(b)[pos] = qg::store_dfc(unpack(y));
   }
-  static __device__ __forceinline__ V renorm(V v) {
-    fast2(v.rh, v.rl);
-    fast2(v.ih, v.il);
-    return v;
-  }
+  static __device__ __forceinline__ V renorm(const V& v) { return unpack(fast2(pack(v))); }
   static __device__ __forceinline__ V zero() { return dfc{0.f, 0.f, 0.f, 0.f}; }
-  static __device__ __forceinline__ V neg(const V& x) { return dfc{-x.rh, -x.rl, -x.ih, -x.il}; }
-  static __device__ __forceinline__ V mul_i(const V& x) { return dfc{-x.ih, -x.il, x.rh, x.rl}; }
-  static __device__ __forceinline__ V mul_mi(const V& x) { return dfc{x.ih, x.il, -x.rh, -x.rl}; }
+  static __device__ __forceinline__ V neg(const V& x) { return dfc{-x.rh, -x.ih, -x.rl, -x.il}; }
+  static __device__ __forceinline__ V mul_i(const V& x) { return dfc{-x.ih, x.rh, -x.il, x.rl}; }
+  static __device__ __forceinline__ V mul_mi(const V& x) { return dfc{x.ih, -x.rh, x.il, -x.rl}; }
 };
 
-// (gr + i gi) * x
+// (gr + i gi) * x: re = gr xr + (-gi) xi, im = gr xi + gi xr
+template <bool RL, bool IL>
+__device__ __forceinline__ cp df_cmul_p(float grh, float grl, float gih, float gil, const dfc& x) {
+  return dot2<RL, IL>(konst(grh, grl), pack(x), konst(-gih, -gil, gih, gil), pack_swapped(x));
+}
 template <bool RL, bool IL>
 __device__ __forceinline__ dfc df_cmul(float grh, float grl, float gih, float gil, const dfc& x) {
-  dfc y;
-  dot2<RL, IL>(grh, grl, x.rh, x.rl, -gih, -gil, x.ih, x.il, y.rh, y.rl);
-  dot2<RL, IL>(grh, grl, x.ih, x.il, gih, gil, x.rh, x.rl, y.ih, y.il);
-  return y;
+  return unpack(df_cmul_p<RL, IL>(grh, grl, gih, gil, x));
 }
-// (a + i a) x (NEG = false) or (a - i a) x (NEG = true), a a constant pair: the sum and
-// the difference of x's parts first, then one product each (a T-gate phase)
+// (a + i a) x (NEG = false) or (a - i a) x (NEG = true), a a constant pair: x + i x or
+// x - i x first, then one product each (a T-gate phase)
 template <bool AL, bool NEG>
 __device__ __forceinline__ dfc df_cmul_diag(float ah, float al, const dfc& x) {
-  float dh, dl, sh, sl;
-  dfc y;
-  if (!NEG) {  // a (xr - xi) + i a (xr + xi)
-    add2(x.rh, x.rl, -x.ih, -x.il, dh, dl);
-    add2(x.rh, x.rl, x.ih, x.il, sh, sl);
-  } else {  // a (xr + xi) + i a (xi - xr)
-    add2(x.rh, x.rl, x.ih, x.il, dh, dl);
-    add2(x.ih, x.il, -x.rh, -x.rl, sh, sl);
-  }
-  tprod<AL>(ah, al, dh, dl, y.rh, y.rl);
-  tprod<AL>(ah, al, sh, sl, y.ih, y.il);
-  return y;
+  return unpack(prod<AL>(konst(ah, al), sum(pack(x), pack(NEG ? DF::mul_mi(x) : DF::mul_i(x)))));
 }
 // a real scalar times x
 template <bool AL>
 __device__ __forceinline__ dfc df_scale(float ah, float al, const dfc& x) {
-  dfc y;
-  tprod<AL>(ah, al, x.rh, x.rl, y.rh, y.rl);
-  tprod<AL>(ah, al, x.ih, x.il, y.ih, y.il);
-  return y;
+  return unpack(prod<AL>(konst(ah, al), pack(x)));
 }
 // y = a*x0 + b*x1 for complex constants a, b (8 floats: a.re h/l, a.im h/l, b.re h/l, b.im h/l)
 __device__ __forceinline__ dfc df_row(float arh, float arl, float aih, float ail, float brh, float brl, float bih,
                                       float bil, const dfc& x0, const dfc& x1) {
-  dfc y;
-  float uh, ul, vh, vl;
-  dot2<true, true>(arh, arl, x0.rh, x0.rl, -aih, -ail, x0.ih, x0.il, uh, ul);
-  dot2<true, true>(brh, brl, x1.rh, x1.rl, -bih, -bil, x1.ih, x1.il, vh, vl);
-  add2(uh, ul, vh, vl, y.rh, y.rl);
-  dot2<true, true>(arh, arl, x0.ih, x0.il, aih, ail, x0.rh, x0.rl, uh, ul);
-  dot2<true, true>(brh, brl, x1.ih, x1.il, bih, bil, x1.rh, x1.rl, vh, vl);
-  add2(uh, ul, vh, vl, y.ih, y.il);
-  return y;
+  return unpack(sum(df_cmul_p<true, true>(arh, arl, aih, ail, x0), df_cmul_p<true, true>(brh, brl, bih, bil, x1)));
 }
 // real 2x2 [[a, b], [c, d]]
 template <bool AL, bool BL, bool CL, bool DL>
 __device__ __forceinline__ void df_real(float ah, float al, float bh, float bl, float ch, float cl, float dh, float dl,
                                         dfc& x0, dfc& x1) {
-  dfc y0, y1;
-  dot2<AL, BL>(ah, al, x0.rh, x0.rl, bh, bl, x1.rh, x1.rl, y0.rh, y0.rl);
-  dot2<AL, BL>(ah, al, x0.ih, x0.il, bh, bl, x1.ih, x1.il, y0.ih, y0.il);
-  dot2<CL, DL>(ch, cl, x0.rh, x0.rl, dh, dl, x1.rh, x1.rl, y1.rh, y1.rl);
-  dot2<CL, DL>(ch, cl, x0.ih, x0.il, dh, dl, x1.ih, x1.il, y1.ih, y1.il);
-  x0 = y0;
-  x1 = y1;
+  const cp u = pack(x0), v = pack(x1);
+  x0 = unpack(dot2<AL, BL>(konst(ah, al), u, konst(bh, bl), v));
+  x1 = unpack(dot2<CL, DL>(konst(ch, cl), u, konst(dh, dl), v));
 }
 // [[c, c], [c, -c]] (Hadamard-shaped): the sum and difference first, one product each
 template <bool CL>
 __device__ __forceinline__ void df_hadamard(float ch, float cl, dfc& x0, dfc& x1) {
-  float sh, sl, dh, dl;
-  dfc y0, y1;
-  add2(x0.rh, x0.rl, x1.rh, x1.rl, sh, sl);
-  add2(x0.rh, x0.rl, -x1.rh, -x1.rl, dh, dl);
-  tprod<CL>(ch, cl, sh, sl, y0.rh, y0.rl);
-  tprod<CL>(ch, cl, dh, dl, y1.rh, y1.rl);
-  add2(x0.ih, x0.il, x1.ih, x1.il, sh, sl);
-  add2(x0.ih, x0.il, -x1.ih, -x1.il, dh, dl);
-  tprod<CL>(ch, cl, sh, sl, y0.ih, y0.il);
-  tprod<CL>(ch, cl, dh, dl, y1.ih, y1.il);
-  x0 = y0;
-  x1 = y1;
+  const cp u = pack(x0), v = pack(x1);
+  const kp c = konst(ch, cl);
+  x0 = unpack(prod<CL>(c, sum(u, v)));
+  x1 = unpack(prod<CL>(c, diff(u, v)));
 }
 // [[1, 1], [1, -1]]: a Hadamard whose 1/sqrt 2 is applied later with the global factors
 __device__ __forceinline__ void df_sumdiff(dfc& x0, dfc& x1) {
-  dfc y0, y1;
-  add2(x0.rh, x0.rl, x1.rh, x1.rl, y0.rh, y0.rl);
-  add2(x0.rh, x0.rl, -x1.rh, -x1.rl, y1.rh, y1.rl);
-  add2(x0.ih, x0.il, x1.ih, x1.il, y0.ih, y0.il);
-  add2(x0.ih, x0.il, -x1.ih, -x1.il, y1.ih, y1.il);
-  x0 = y0;
-  x1 = y1;
-}
-// x + k*y for a constant pair k, unnormalised
-template <bool KL>
-__device__ __forceinline__ void axpy(float kh, float kl, float xh, float xl, float yh, float yl, float& zh, float& zl) {
-  float p, e, err;
-  tprod<KL>(kh, kl, yh, yl, p, e);
-  tsum(xh, p, zh, err);
-  zl = (xl + e) + err;
+  const cp u = pack(x0), v = pack(x1);
+  x0 = unpack(sum(u, v));
+  x1 = unpack(diff(u, v));
 }
 // [[1, b], [c, S]] (S = +-1): a real rotation with its diagonal factored out
 template <bool BL, bool CL, bool NEG>
 __device__ __forceinline__ void df_realunit(float bh, float bl, float ch, float cl, dfc& x0, dfc& x1) {
-  dfc y0, y1;
-  axpy<BL>(bh, bl, x0.rh, x0.rl, x1.rh, x1.rl, y0.rh, y0.rl);
-  axpy<BL>(bh, bl, x0.ih, x0.il, x1.ih, x1.il, y0.ih, y0.il);
-  if (NEG) {
-    axpy<CL>(ch, cl, -x1.rh, -x1.rl, x0.rh, x0.rl, y1.rh, y1.rl);
-    axpy<CL>(ch, cl, -x1.ih, -x1.il, x0.ih, x0.il, y1.ih, y1.il);
-  } else {
-    axpy<CL>(ch, cl, x1.rh, x1.rl, x0.rh, x0.rl, y1.rh, y1.rl);
-    axpy<CL>(ch, cl, x1.ih, x1.il, x0.ih, x0.il, y1.ih, y1.il);
-  }
-  x0 = y0;
-  x1 = y1;
+  const cp u = pack(x0), v = pack(x1);
+  x0 = unpack(axpy<BL>(konst(bh, bl), u, v));
+  x1 = unpack(NEG ? axmy<CL>(konst(ch, cl), v, u) : axpy<CL>(konst(ch, cl), v, u));
 }
 // [[1, i b], [i c, 1]]: an RX-shaped rotation with its diagonal factored out
 template <bool BL, bool CL>
 __device__ __forceinline__ void df_rxunit(float bh, float bl, float ch, float cl, dfc& x0, dfc& x1) {
-  dfc y0, y1;
-  axpy<BL>(-bh, -bl, x0.rh, x0.rl, x1.ih, x1.il, y0.rh, y0.rl);
-  axpy<BL>(bh, bl, x0.ih, x0.il, x1.rh, x1.rl, y0.ih, y0.il);
-  axpy<CL>(-ch, -cl, x1.rh, x1.rl, x0.ih, x0.il, y1.rh, y1.rl);
-  axpy<CL>(ch, cl, x1.ih, x1.il, x0.rh, x0.rl, y1.ih, y1.il);
-  x0 = y0;
-  x1 = y1;
+  const cp u = pack(x0), us = pack_swapped(x0), v = pack(x1), vs = pack_swapped(x1);
+  x0 = unpack(axpy<BL>(konst(-bh, -bl, bh, bl), u, vs));
+  x1 = unpack(axpy<CL>(konst(-ch, -cl, ch, cl), v, us));
 }
 // x * w^T, the chunks the run needs selected at compile time
 template <bool A, bool B, bool C>
@@ -255,33 +289,33 @@ __device__ __forceinline__ dfc df_root_mul_impl(unsigned T, const dfc& x) {
   bool have = false;
   if (A) {
     const float4 v = qgp_roots[(T >> 20) & 1023u];
-    g = dfc{v.x, v.y, v.z, v.w};
+    g = dfc{v.x, v.z, v.y, v.w};
     have = true;
   }
   if (B) {
     const float4 v = qgp_roots[1024 + ((T >> 10) & 1023u)];
-    g = have ? df_cmul<true, true>(v.x, v.y, v.z, v.w, g) : dfc{v.x, v.y, v.z, v.w};
+    g = have ? df_cmul<true, true>(v.x, v.y, v.z, v.w, g) : dfc{v.x, v.z, v.y, v.w};
     have = true;
   }
   if (C) {
     const float4 v = qgp_roots[2048 + (T & 1023u)];
-    g = have ? df_cmul<true, true>(v.x, v.y, v.z, v.w, g) : dfc{v.x, v.y, v.z, v.w};
+    g = have ? df_cmul<true, true>(v.x, v.y, v.z, v.w, g) : dfc{v.x, v.z, v.y, v.w};
   }
   return df_cmul<true, true>(g.rh, g.rl, g.ih, g.il, x);
 }
 // x times a power of two (exact)
-__device__ __forceinline__ dfc df_pow2(float c, const dfc& x) { return dfc{x.rh * c, x.rl * c, x.ih * c, x.il * c}; }
+__device__ __forceinline__ dfc df_pow2(float c, const dfc& x) {
+  const cp v = pack(x);
+  const u64 k = pk(c, c);
+  return unpack(cp{mul2(k, v.h), mul2(k, v.l)});
+}
 // [[a, i b], [i c, d]] with a, b, c, d real (RX-shaped)
 template <bool AL, bool BL, bool CL, bool DL>
 __device__ __forceinline__ void df_rxlike(float ah, float al, float bh, float bl, float ch, float cl, float dh, float dl,
                                           dfc& x0, dfc& x1) {
-  dfc y0, y1;
-  dot2<AL, BL>(ah, al, x0.rh, x0.rl, -bh, -bl, x1.ih, x1.il, y0.rh, y0.rl);
-  dot2<AL, BL>(ah, al, x0.ih, x0.il, bh, bl, x1.rh, x1.rl, y0.ih, y0.il);
-  dot2<DL, CL>(dh, dl, x1.rh, x1.rl, -ch, -cl, x0.ih, x0.il, y1.rh, y1.rl);
-  dot2<CL, DL>(ch, cl, x0.rh, x0.rl, dh, dl, x1.ih, x1.il, y1.ih, y1.il);
-  x0 = y0;
-  x1 = y1;
+  const cp u = pack(x0), us = pack_swapped(x0), v = pack(x1), vs = pack_swapped(x1);
+  x0 = unpack(dot2<AL, BL>(konst(ah, al), u, konst(-bh, -bl, bh, bl), vs));
+  x1 = unpack(dot2<DL, CL>(konst(dh, dl), v, konst(-ch, -cl, ch, cl), us));
 }
 
 // ---- complex64 -------------------------------------------------------------

@@ -175,11 +175,11 @@ struct PolDFT {
     else return load_dfc(reinterpret_cast<const double2*>(sm)[pos]);
   }
   __device__ static void store_raw(unsigned char* sm, int pos, const dfc& v) {
-    if constexpr (kOutPairs) reinterpret_cast<float4*>(sm)[pos] = make_float4(v.rh, v.rl, v.ih, v.il);
+    if constexpr (kOutPairs) reinterpret_cast<float4*>(sm)[pos] = make_float4(v.rh, v.ih, v.rl, v.il);
     else reinterpret_cast<double2*>(sm)[pos] = store_dfc(v);
   }
   __device__ static void store_work(unsigned char* sm, int pos, const dfc& v) {
-    reinterpret_cast<float4*>(sm)[pos] = make_float4(v.rh, v.rl, v.ih, v.il);
+    reinterpret_cast<float4*>(sm)[pos] = make_float4(v.rh, v.ih, v.rl, v.il);
   }
   __device__ static dfc cmk(const Cst& c, int k, const dfc& x) {  // matrix entry k (0..3) times x
     return cmul_df(c.h[2 * k], c.l[2 * k], c.h[2 * k + 1], c.l[2 * k + 1], x);
@@ -220,8 +220,8 @@ struct PolDFT {
       y0 = x1;
       y1 = x0;
     } else {  // U2_IMAG_ANTI
-      if (h[3] > 0) y0 = dfc{-x1.ih, -x1.il, x1.rh, x1.rl}; else y0 = dfc{x1.ih, x1.il, -x1.rh, -x1.rl};
-      if (h[5] > 0) y1 = dfc{-x0.ih, -x0.il, x0.rh, x0.rl}; else y1 = dfc{x0.ih, x0.il, -x0.rh, -x0.rl};
+      if (h[3] > 0) y0 = dfc{-x1.ih, x1.rh, -x1.il, x1.rl}; else y0 = dfc{x1.ih, -x1.rh, x1.il, -x1.rl};
+      if (h[5] > 0) y1 = dfc{-x0.ih, x0.rh, -x0.il, x0.rl}; else y1 = dfc{x0.ih, -x0.rh, x0.il, -x0.rl};
     }
     x0 = y0;
     x1 = y1;
@@ -229,11 +229,11 @@ struct PolDFT {
   template <int CLS>
   __device__ static dfc phase(const Cst& c, const dfc& x) {
     if (CLS == PH_GENERAL) return cmk(c, 0, x);
-    if (CLS == PH_NEG) return dfc{-x.rh, -x.rl, -x.ih, -x.il};
-    if (CLS == PH_I) return dfc{-x.ih, -x.il, x.rh, x.rl};
-    return dfc{x.ih, x.il, -x.rh, -x.rl};
+    if (CLS == PH_NEG) return dfc{-x.rh, -x.ih, -x.rl, -x.il};
+    if (CLS == PH_I) return dfc{-x.ih, x.rh, -x.il, x.rl};
+    return dfc{x.ih, -x.rh, x.il, -x.rl};
   }
-  __device__ static dfc times_i(const dfc& x) { return dfc{-x.ih, -x.il, x.rh, x.rl}; }
+  __device__ static dfc times_i(const dfc& x) { return dfc{-x.ih, x.rh, -x.il, x.rl}; }
   __device__ static dfc cmul_idx(const Cst& c, int which, const dfc& x) {
     const bool w = which != 0;
     return cmul_df(w ? c.h[2] : c.h[0], w ? c.l[2] : c.l[0], w ? c.h[3] : c.h[1], w ? c.l[3] : c.l[1], x);
@@ -1002,7 +1002,7 @@ __global__ void __launch_bounds__(512, 1) k_tile_jobs(int n, const TileJobRec* _
       for (int l = threadIdx.x; l < g.K; l += g.T) {
         const int q = swz<E>(l);
         const dfc v = load_dfc(reinterpret_cast<const double2*>(tile)[q]);
-        reinterpret_cast<float4*>(tile)[q] = make_float4(v.rh, v.rl, v.ih, v.il);
+        reinterpret_cast<float4*>(tile)[q] = make_float4(v.rh, v.ih, v.rl, v.il);
       }
     }
     int64_t ob = jr.op_begin;
@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(512, 1) k_job_loop(int n, JobLoopSlot* slots, 
       for (int l = threadIdx.x; l < g.K; l += g.T) {
         const int q = swz<E>(l);
         const dfc v = load_dfc(reinterpret_cast<const double2*>(tile)[q]);
-        reinterpret_cast<float4*>(tile)[q] = make_float4(v.rh, v.rl, v.ih, v.il);
+        reinterpret_cast<float4*>(tile)[q] = make_float4(v.rh, v.ih, v.rl, v.il);
       }
     }
     int64_t ob = jr.op_begin;
