@@ -282,10 +282,9 @@ std::vector<std::complex<double>> parity_table(const TOp& t, int E) {
 struct Shape {
   int rbits, bufs, ctas;
 };
-// Measured on the 30-qubit layered + QFT circuit: double-float keeps 8 registers
-// per thread, two tile buffers and one CTA per SM (16 registers per thread spill
-// at two CTAs and starve latency hiding at one); complex64 holds 16 registers per
-// thread with two buffers and two CTAs per SM.
+// The shape of programs compiled without one (parameter sweeps, tiles of 2^12): 8 registers
+// per thread for double-float, 16 for complex64, two tile buffers. The runtime gives large
+// double-float states another (default_shape).
 Shape shape_for(int prec) {
   if (prec == QG_C128) return Shape{3, 2, 1};
   return Shape{4, 2, 2};
@@ -1112,6 +1111,42 @@ class PassGen {
     o_ << "    }\n";
   }
 
+  // lt = the thread's index bits under layout t (zeros at the register positions). The
+  // lanes' low bits carry one free index bit of each bank class of the swizzle (and bit 0
+  // of an 8-byte amplitude unless it is a register bit: then pairs move), so the accesses
+  // of a layout are free of bank conflicts whatever its register bits; the other thread
+  // bits take the remaining index bits in ascending order. With the index bits in plain
+  // ascending order, two of the three low lane bits often fell into one class (26 qubits,
+  // complex128: 28 % of a pass's shared-memory cycles were conflicts).
+  void thread_map(const TOp& t) {
+    uint32_t rb = 0;
+    for (int q = 0; q < sh_.rbits; ++q) rb |= 1u << t.dbits[q];
+    std::vector<int> order;
+    uint32_t used = rb;
+    auto take = [&](int b) {
+      order.push_back(b);
+      used |= 1u << b;
+    };
+    if (!df_ && !(rb & 1u)) take(0);
+    for (int c = 0; c < 3; ++c)
+      for (int b = c + (df_ ? 0 : 1); b < pd_.k; b += 3)
+        if (!(used & (1u << b))) {
+          take(b);
+          break;
+        }
+    for (int b = 0; b < pd_.k; ++b)
+      if (!(used & (1u << b))) take(b);
+    o_ << "    lt = 0u";
+    for (size_t i = 0; i < order.size();) {
+      size_t j = i + 1;
+      while (j < order.size() && order[j] == order[j - 1] + 1) ++j;
+      const std::string src = "((tid >> " + std::to_string(i) + ") & " + hex32((1u << (j - i)) - 1) + ")";
+      o_ << " | (" << src << " << " << order[i] << ")";
+      i = j;
+    }
+    o_ << ";\n";
+  }
+
   void body() {
     const std::string V = df_ ? "dfc" : "float2";
     const int E = df_ ? 16 : 8;
@@ -1133,12 +1168,7 @@ class PassGen {
           raw = false;
         }
         for (int q = 0; q < sh_.rbits; ++q) rpos_[q] = t.dbits[q];
-        // thread bits: zeros inserted at the register positions (ascending)
-        o_ << "    lt = tid;\n";
-        for (int q = 0; q < sh_.rbits; ++q) {
-          const int b = t.dbits[q];
-          o_ << "    lt = ((lt >> " << b << ") << " << (b + 1) << ") | (lt & " << hex32((1u << b) - 1) << ");\n";
-        }
+        thread_map(t);
         for (int j = 0; j < ns_; ++j) {
           uint32_t lj = 0;
           for (int q = 0; q < sh_.rbits; ++q)
@@ -1689,6 +1719,10 @@ bool pass_kernel_ready(const PassKernels& pk, size_t step) {
 
 double pass_kernels_compile_ms(const PassKernels& pk) { return static_cast<const Compiled&>(pk).compile_ms; }
 
+// Up to 16 waves of CTAs, each with at least four tiles: with one wave, the CTAs of an SM
+// drift apart and the SM ends on a few of them (28 qubits, layers + QFT: double-float
+// 55.3 -> 50.7 ms at (10,3,2,4), complex64 31.9 -> 30.2 ms at (12,4,2,2); 4, 8 and 32 waves
+// measured 51.9, 51.2 and 50.8 ms).
 cudaError_t launch_pass_kernel(const PassKernels& pk, size_t step, int n, const PassDesc& pd, void* state, int prec,
                                cudaStream_t st) {
   const Compiled& c = static_cast<const Compiled&>(pk);
@@ -1696,7 +1730,8 @@ cudaError_t launch_pass_kernel(const PassKernels& pk, size_t step, int n, const 
   const uint64_t ntiles = 1ULL << (n - pd.k);
   const Shape sh = c.sh;
   (void)prec;
-  uint64_t grid = (uint64_t)kSMCount * sh.ctas;
+  const uint64_t wave = (uint64_t)kSMCount * sh.ctas;
+  uint64_t grid = std::max(wave, std::min(16 * wave, ntiles / 4));
   if (grid > ntiles) grid = ntiles;
   unsigned long long nt = ntiles;
   unsigned char* sp = static_cast<unsigned char*>(state);

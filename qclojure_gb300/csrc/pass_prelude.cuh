@@ -39,12 +39,15 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// XOR swizzle of the shared-memory tile (16-byte units, 8 per 128-byte row);
-// 8-byte amplitudes move in 16-byte pairs.
+// XOR swizzle of the shared-memory tile (16-byte units, 8 per 128-byte row; 8-byte
+// amplitudes move in 16-byte pairs). Every index bit above the row's three unit bits is
+// folded onto one of them, so all bits fall into three classes (position mod 3), and any
+// lanes whose three low bits carry one index bit of each class touch eight different
+// units: the generator picks the lanes' bits that way in every layout (thread_map).
 template <int E>
 __device__ __forceinline__ int swz(int l) {
-  if (E == 16) return l ^ ((l >> 3) & 7);
-  return l ^ (((l >> 4) & 7) << 1);
+  if (E == 16) return l ^ (((l >> 3) ^ (l >> 6) ^ (l >> 9) ^ (l >> 12)) & 7);
+  return l ^ ((((l >> 4) ^ (l >> 7) ^ (l >> 10)) & 7) << 1);
 }
 
 // ---------------------------------------------------------------------------

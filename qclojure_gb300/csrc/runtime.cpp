@@ -717,13 +717,32 @@ static bool will_specialise(const Ctx* c, int n, int prec, int arith, int fusion
   if (mode == QG_PASS_KERNELS_OFF) return false;
   return mode == QG_PASS_KERNELS_ALWAYS || n >= c->spec_min_qubits[prec == QG_C64 ? 1 : 0].load();
 }
-// The tuned shape for programs of this kind, if one was chosen (copied into *out).
+// The pass kernels' shape where none was tuned or set. Double-float passes are bound by the
+// FP32 pipe and by the barriers of their layout changes: four CTAs per SM on tiles of 2^10
+// overlap one CTA's shared-memory phase with the others' arithmetic (FP32 pipe 68-73 % busy;
+// 50-57 % with one CTA on 2^12), which pays for the extra passes from 22 qubits on (layers +
+// QFT: 22 qubits 0.70 against 0.85 ms, 24 qubits 2.60 / 3.13, 28 qubits 44.7 / 51.3 ms); at 20
+// qubits and below, where a pass is a wave or less, fewer passes win (20 qubits 0.28 / 0.25).
+// complex64 passes are nearer to HBM and keep 2^12 (28 qubits: 14.0 ms either way).
+static qg_tuning default_shape(int n, int prec) {
+  qg_tuning t;
+  std::memset(&t, 0, sizeof(t));
+  t.tile_bits = std::min(12, n);
+  t.reg_bits = prec == QG_C128 ? 3 : 4;
+  t.buffers = 2;
+  t.ctas_per_sm = prec == QG_C128 ? 1 : 2;
+  if (prec == QG_C128 && n >= 22) {
+    t.tile_bits = 10;
+    t.ctas_per_sm = 4;
+  }
+  return t;
+}
+// The tuned shape for programs of this kind, or the default one (copied into *out).
 static const qg_tuning* tuning_for(Ctx* c, int n, int prec, int arith, int fusion, qg_tuning* out) {
   if (!c || !will_specialise(c, n, prec, arith, fusion)) return nullptr;
   std::lock_guard<std::mutex> lk(c->tune_mu);
   auto it = c->tunings.find({n, prec});
-  if (it == c->tunings.end()) return nullptr;
-  *out = it->second;
+  *out = it == c->tunings.end() ? default_shape(n, prec) : it->second;
   return out;
 }
 
@@ -2618,11 +2637,7 @@ int qg_tuning_get(void* ctx, int32_t n, int32_t precision, qg_tuning* out) {
     *out = it->second;
     return QG_OK;
   }
-  std::memset(out, 0, sizeof(*out));
-  out->tile_bits = std::min(12, (int)n);
-  out->reg_bits = precision == QG_C128 ? 3 : 4;
-  out->buffers = 2;
-  out->ctas_per_sm = precision == QG_C128 ? 1 : 2;
+  *out = default_shape(n, precision);
   return QG_OK;
 }
 
@@ -2694,7 +2709,9 @@ int qg_autotune(void* ctx, int32_t n, int32_t precision, const qg_circuit* calib
   }
   // candidates: the default first (tile bits, register bits, buffers, CTAs per SM)
   std::vector<qg_tuning> cand;
+  cand.push_back(default_shape(n, precision));
   auto add = [&](int k, int r, int b, int ct) {
+    if (k == cand[0].tile_bits && r == cand[0].reg_bits && b == cand[0].buffers && ct == cand[0].ctas_per_sm) return;
     qg_tuning t;
     std::memset(&t, 0, sizeof(t));
     t.tile_bits = k;
