@@ -22,7 +22,6 @@
 #include <cmath>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -36,8 +35,6 @@ constexpr uint32_t kStreamReadout = 0x20000000u;  // + qubit: readout flips
 constexpr uint32_t kStreamKraus = 0x40000000u;    // + site: Kraus operator choice
 constexpr int kMinQubits = 5;                     // tiled passes need 2^5 amplitudes per tile
 constexpr double kNormTolerance = 1e-12;          // normalize-state leaves smaller norms alone
-
-double uniform01(uint64_t x) { return (double)(x >> 11) * 0x1p-53; }
 
 struct Channel {
   bool built = false;
@@ -132,18 +129,18 @@ int build_channel(const qg_gate_noise& e, Channel* ch, std::string* err) {
   return QG_OK;
 }
 
-// apply-quantum-channel's choice (channel.clj:212-231): the first operator whose
-// cumulative probability exceeds the draw, else the last one.
-int choose(const Channel& ch, double u) {
-  const int k = (int)ch.ops.size();
-  if (k <= 1) return 0;
+// apply-quantum-channel's choice (channel.clj:212-231), the first operator whose cumulative
+// probability exceeds the draw, else the last one, on the draw's integer: u = k 2^-53 is below
+// a cumulative probability c exactly when k < ceil(c 2^53).
+NoiseChannel device_channel(const Channel& ch) {
+  NoiseChannel d{};
+  d.count = (int32_t)ch.ops.size();
   double cum = 0.0;
-  for (int i = 0; i < k; ++i) {
-    const double nc = cum + ch.probs[i];
-    if (u < nc || i >= k - 1) return i;
-    cum = nc;
+  for (int i = 0; i + 1 < d.count; ++i) {
+    cum += ch.probs[i];
+    d.below[i] = cum > 0 ? (uint64_t)std::ceil(std::min(cum, 2.0) * 0x1p53) : 0ull;
   }
-  return k - 1;
+  return d;
 }
 
 struct Readout {
@@ -153,54 +150,11 @@ struct Readout {
   std::vector<double> factor;  // [source * n + target], NaN where no factor is given
 };
 
-// calculate-final-bitstring (noise.clj:107-160): qubits in order; a qubit's flip
-// probability is its base probability times the factors from earlier flipped qubits.
-uint64_t apply_readout(uint64_t bits, int n, const Readout& r, uint64_t seed, uint64_t shot) {
-  if (!r.on) return bits;
-  int hist[64];
-  int nh = 0;
-  for (int q = 0; q < n; ++q) {
-    const int b = n - 1 - q;
-    const int bit = (int)((bits >> b) & 1ULL);
-    const double base = bit ? r.p10 : r.p01;
-    double f = 1.0;
-    if (r.corr)
-      for (int h = 0; h < nh; ++h) {
-        const double c = r.factor[(size_t)hist[h] * n + q];
-        if (!std::isnan(c)) f *= c;
-      }
-    const double eff = std::min(1.0, std::max(0.0, base * f));
-    if (uniform01(draw64(seed, shot, kStreamReadout + (uint32_t)q)) < eff) {
-      bits ^= 1ULL << b;
-      hist[nh++] = q;
-    }
-  }
-  return bits;
-}
-
 struct Site {
   int entry;
   int pass;    // tiled pass holding its op
   int64_t at;  // index of its op within the pass
 };
-
-// Run body(begin, end) over [0, count) on the host's cores.
-template <class F>
-void parallel_for(uint64_t count, uint64_t grain, F body) {
-  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const uint64_t parts = std::min<uint64_t>(hw, std::max<uint64_t>(1, count / std::max<uint64_t>(1, grain)));
-  if (parts <= 1) {
-    body(0, count);
-    return;
-  }
-  std::vector<std::thread> th;
-  const uint64_t per = (count + parts - 1) / parts;
-  for (uint64_t t = 0; t < parts; ++t) {
-    const uint64_t b = t * per, e = std::min(count, b + per);
-    if (b < e) th.emplace_back(body, b, e);
-  }
-  for (auto& x : th) x.join();
-}
 
 double ms_between(std::chrono::steady_clock::time_point a) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - a).count();
@@ -330,58 +284,67 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
     const PassDesc& pd = prog.steps[pass_steps[p]].pass;
     encode_kops(precision, arith, prog.tops.data() + pd.op_begin, nops[p], tmpl.data() + rec * (size_t)rec_off[p]);
   }
-  std::vector<std::vector<unsigned char>> variants(sites.size());
-  for (size_t s = 0; s < sites.size(); ++s) {
+  const size_t S = sites.size();
+  std::vector<unsigned char> variants(rec * 4 * S);
+  std::vector<int32_t> site_of((size_t)R, -1), pass_ops((size_t)R), site_chan(S);
+  std::vector<int64_t> pass_off((size_t)R);
+  for (size_t p = 0; p < P; ++p)
+    for (int64_t j = rec_off[p]; j < rec_off[p + 1]; ++j) {
+      pass_off[(size_t)j] = rec_off[p];
+      pass_ops[(size_t)j] = (int32_t)nops[p];
+    }
+  for (size_t s = 0; s < S; ++s) {
     const Channel& ch = chans[sites[s].entry];
     const PassDesc& pd = prog.steps[pass_steps[sites[s].pass]].pass;
     TOp t = prog.tops[(size_t)(pd.op_begin + sites[s].at)];
-    variants[s].resize(rec * ch.applied.size());
     for (size_t v = 0; v < ch.applied.size(); ++v) {
       set_op_matrix(&t, ch.applied[v].data());
-      encode_kops(precision, arith, &t, 1, variants[s].data() + rec * v);
+      encode_kops(precision, arith, &t, 1, variants.data() + rec * (4 * s + v));
     }
+    site_of[(size_t)(rec_off[sites[s].pass] + sites[s].at)] = (int32_t)s;
+    site_chan[s] = sites[s].entry;
   }
+  std::vector<NoiseChannel> dch(chans.size());
+  for (size_t e = 0; e < chans.size(); ++e) dch[e] = device_channel(chans[e]);
 
   // Batches of shots. Shots whose Kraus choices coincide end in the same state, so each
   // batch simulates only its distinct choice vectors and samples every shot from its
-  // vector's state (with the shot's own draw). Batch size: device memory for one state
-  // per shot, host op records for one state per shot.
+  // vector's state (with the shot's own draw). Batch size: device memory for one state and
+  // its op records per shot.
   const int dev = ctx_device_of(ctx);
   cudaSetDevice(dev);
   const size_t state_bytes = (precision == QG_C64 ? 8ull : 16ull) << n_run;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return fail(QG_ERR_DEVICE, "cudaMemGetInfo failed");
   const size_t budget = std::min(free_b / 2, (size_t)64 << 30);
-  const size_t per = state_bytes + rec * (size_t)R + 64;
+  const size_t per = state_bytes + rec * (size_t)R + S + 128;
   if (budget < per) return fail(QG_ERR_OOM, "one trajectory does not fit the device memory budget");
   uint64_t B = std::min<uint64_t>(shots ? shots : 1, 65536);
   B = std::min<uint64_t>(B, std::max<size_t>(1, budget / per));
-  B = std::min<uint64_t>(B, std::max<size_t>(1, ((size_t)1 << 30) / std::max<size_t>(1, rec * (size_t)R)));
-  const size_t S = sites.size();
+  B = std::min<uint64_t>(B, std::max<size_t>(1, ((size_t)4 << 30) / std::max<size_t>(1, rec * (size_t)R)));
 
   cudaStream_t st;
   if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return fail(QG_ERR_DEVICE, "stream");
-  void* slab = nullptr;
-  void** d_ptrs = nullptr;
-  unsigned char* d_kops = nullptr;
-  uint64_t* d_out = nullptr;
-  double* d_norm = nullptr;
-  int32_t* d_state_of = nullptr;
-  unsigned char* h_kops = nullptr;
-  size_t h_cap = 0;
+  // Device memory of the call: small pieces from the stream-ordered pool the states use, large
+  // ones (more than kPooled) allocated and freed, so that the pool does not keep them.
+  constexpr size_t kPooled = (size_t)256 << 20;
+  std::vector<std::pair<void*, bool>> held;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   double device_ms = 0;
   int batches = 0;
   int64_t distinct = 0;
+  auto drop_from = [&](size_t at) {
+    for (; held.size() > at; held.pop_back()) {
+      if (held.back().second) cudaFreeAsync(held.back().first, st);
+      else {
+        cudaStreamSynchronize(st);
+        cudaFree(held.back().first);
+      }
+    }
+  };
   auto cleanup = [&]() {
+    drop_from(0);
     cudaStreamSynchronize(st);
-    if (slab) cudaFree(slab);
-    if (d_ptrs) cudaFree(d_ptrs);
-    if (d_kops) cudaFree(d_kops);
-    if (d_out) cudaFree(d_out);
-    if (d_norm) cudaFree(d_norm);
-    if (d_state_of) cudaFree(d_state_of);
-    if (h_kops) cudaFreeHost(h_kops);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     cudaStreamDestroy(st);
@@ -391,94 +354,148 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
   };
-  bool ok = cuda_check(cudaMalloc(&slab, state_bytes * B), "alloc trajectories") &&
-            cuda_check(cudaMalloc((void**)&d_ptrs, sizeof(void*) * B), "alloc pointers") &&
-            cuda_check(cudaMalloc((void**)&d_kops, rec * (size_t)R * B + 16), "alloc op records") &&
-            cuda_check(cudaMalloc((void**)&d_out, sizeof(uint64_t) * B), "alloc outcomes") &&
-            cuda_check(cudaMalloc((void**)&d_norm, sizeof(double) * B), "alloc norms") &&
-            cuda_check(cudaMalloc((void**)&d_state_of, sizeof(int32_t) * B), "alloc shot states") &&
-            cuda_check(cudaEventCreate(&e0), "event") && cuda_check(cudaEventCreate(&e1), "event");
-  if (ok) {
-    std::vector<void*> ptrs(B);
-    for (uint64_t m = 0; m < B; ++m) ptrs[m] = (unsigned char*)slab + state_bytes * m;
-    ok = cuda_check(cudaMemcpyAsync(d_ptrs, ptrs.data(), sizeof(void*) * B, cudaMemcpyHostToDevice, st), "H2D") &&
-         cuda_check(cudaStreamSynchronize(st), "sync");
-  }
+  auto take = [&](size_t bytes, const char* what, void** p) {
+    bytes = std::max<size_t>(bytes, 16);
+    const bool pooled = bytes <= kPooled;
+    if (!cuda_check(pooled ? cudaMallocAsync(p, bytes, st) : cudaMalloc(p, bytes), what)) return false;
+    held.push_back({*p, pooled});
+    return true;
+  };
+  // one upload for every table of the call: each at a 256-byte boundary
+  std::vector<unsigned char> tables;
+  auto put = [&](const void* src, size_t bytes) {
+    const size_t at = (tables.size() + 255) / 256 * 256;
+    tables.resize(at + std::max<size_t>(bytes, 16));
+    if (bytes) std::memcpy(tables.data() + at, src, bytes);
+    return at;
+  };
+  const size_t o_chan = put(dch.data(), sizeof(NoiseChannel) * dch.size());
+  const size_t o_site_chan = put(site_chan.data(), sizeof(int32_t) * S);
+  const size_t o_tmpl = put(tmpl.data(), tmpl.size()), o_var = put(variants.data(), variants.size());
+  const size_t o_site = put(site_of.data(), sizeof(int32_t) * site_of.size());
+  const size_t o_poff = put(pass_off.data(), sizeof(int64_t) * pass_off.size());
+  const size_t o_pops = put(pass_ops.data(), sizeof(int32_t) * pass_ops.size());
+  const size_t o_fac = put(ro.factor.data(), sizeof(double) * ro.factor.size());
+  unsigned char *d_tab = nullptr, *d_choices = nullptr;
+  struct Hash {
+    uint64_t a, b;
+  };
+  Hash* d_hash = nullptr;
+  uint64_t* d_out = nullptr;
+  int32_t *d_state_of = nullptr, *d_reps = nullptr, *d_differ = nullptr;
+  bool ok = cuda_check(cudaEventCreate(&e0), "event") && cuda_check(cudaEventCreate(&e1), "event") &&
+            take(tables.size(), "alloc tables", (void**)&d_tab) && take(S * B, "alloc choices", (void**)&d_choices) &&
+            take(sizeof(Hash) * B, "alloc hashes", (void**)&d_hash) &&
+            take(sizeof(uint64_t) * B, "alloc outcomes", (void**)&d_out) &&
+            take(sizeof(int32_t) * B, "alloc shot states", (void**)&d_state_of) &&
+            take(sizeof(int32_t) * B, "alloc state shots", (void**)&d_reps) &&
+            take(sizeof(int32_t), "alloc check", (void**)&d_differ) &&
+            cuda_check(cudaMemcpyAsync(d_tab, tables.data(), tables.size(), cudaMemcpyHostToDevice, st), "H2D tables");
+  NoiseRecords nr;
+  nr.tmpl = d_tab + o_tmpl;
+  nr.variants = d_tab + o_var;
+  nr.site_of = reinterpret_cast<const int32_t*>(d_tab + o_site);
+  nr.pass_off = reinterpret_cast<const int64_t*>(d_tab + o_poff);
+  nr.pass_ops = reinterpret_cast<const int32_t*>(d_tab + o_pops);
+  nr.sites = (int)S;
+  nr.pieces = (int)(rec / 16);
+  nr.records = R;
+  const uint64_t N = 1ULL << n;
+  std::vector<Hash> h_hash(B);
   std::vector<uint64_t> h_out(B);
   std::vector<double> h_norm(B);
-  std::vector<int32_t> state_of(B);
-  std::vector<uint8_t> choices(B * std::max<size_t>(S, 1));
-  std::vector<uint64_t> reps;
-  std::unordered_map<std::string, int32_t> seen;
-  std::vector<double> host_state;
+  std::vector<int32_t> state_of(B), reps, slots;
+  std::vector<void*> ptrs;
+  std::vector<uint8_t> h_choices;
+  const size_t fixed = held.size();
   int result = QG_OK;
   for (uint64_t base = 0; ok && base < shots; base += B) {
     const uint64_t nb = std::min<uint64_t>(B, shots - base);
-    // Kraus choices of every shot, and the distinct choice vectors
-    reps.clear();
-    seen.clear();
-    parallel_for(nb, 256, [&](uint64_t b, uint64_t e) {
-      for (uint64_t m = b; m < e; ++m) {
-        uint8_t* cv = choices.data() + m * S;
-        for (size_t s = 0; s < S; ++s) {
-          const Channel& ch = chans[sites[s].entry];
-          cv[s] = (uint8_t)(ch.ops.size() > 1
-                                ? choose(ch, uniform01(draw64(seed, base + m, kStreamKraus + (uint32_t)s)))
-                                : 0);
-        }
-      }
-    });
-    for (uint64_t m = 0; m < nb; ++m) {
-      const uint8_t* cv = choices.data() + m * S;
-      auto it = seen.emplace(std::string((const char*)cv, S), (int32_t)reps.size());
-      if (it.second) reps.push_back(m);
-      state_of[m] = it.first->second;
-    }
-    const uint64_t U = reps.size();
-    distinct += (int64_t)U;
-    const size_t need = rec * (size_t)R * U + 16;
-    if (need > h_cap) {  // pinned staging for the records, grown on demand
-      if (h_kops) cudaFreeHost(h_kops);
-      h_kops = nullptr;
-      h_cap = std::max(need, std::min(rec * (size_t)R * B + 16, h_cap * 2));
-      if (!cuda_check(cudaMallocHost((void**)&h_kops, h_cap), "alloc host records")) {
-        ok = false;
-        break;
-      }
-    }
-    // op records of the distinct states: pass-major, states contiguous within a pass
-    parallel_for(U, 64, [&](uint64_t b, uint64_t e) {
-      for (uint64_t u = b; u < e; ++u) {
-        const uint8_t* cv = choices.data() + reps[u] * S;
-        for (size_t p = 0; p < P; ++p) {
-          unsigned char* dst = h_kops + rec * (size_t)(rec_off[p] * (int64_t)U + (int64_t)u * nops[p]);
-          std::memcpy(dst, tmpl.data() + rec * (size_t)rec_off[p], rec * (size_t)nops[p]);
-        }
-        for (size_t s = 0; s < S; ++s) {
-          const Site& si = sites[s];
-          unsigned char* dst =
-              h_kops + rec * (size_t)(rec_off[si.pass] * (int64_t)U + (int64_t)u * nops[si.pass] + si.at);
-          std::memcpy(dst, variants[s].data() + rec * (size_t)cv[s], rec);
-        }
-      }
-    });
+    drop_from(fixed);
     ok = cuda_check(cudaEventRecord(e0, st), "event") &&
-         cuda_check(cudaMemcpyAsync(d_kops, h_kops, rec * (size_t)R * U, cudaMemcpyHostToDevice, st), "H2D records") &&
-         cuda_check(cudaMemcpyAsync(d_state_of, state_of.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice, st),
-                    "H2D shot states") &&
-         cuda_check(launch_batch_zero(slab, precision, n_run, (int)U, st), "zero states");
+         cuda_check(launch_noise_choices(reinterpret_cast<const NoiseChannel*>(d_tab + o_chan),
+                                         reinterpret_cast<const int32_t*>(d_tab + o_site_chan), (int)S, base, (int)nb,
+                                         seed, kStreamKraus, d_choices, d_hash, st),
+                    "choices") &&
+         cuda_check(cudaMemcpyAsync(h_hash.data(), d_hash, sizeof(Hash) * nb, cudaMemcpyDeviceToHost, st), "D2H") &&
+         cuda_check(cudaStreamSynchronize(st), "sync");
+    if (!ok) break;
+    // distinct choice vectors in order of first appearance (open addressing on the hashes)
+    size_t cap = 64;
+    while (cap < 2 * nb) cap *= 2;
+    slots.assign(cap, -1);
+    reps.clear();
+    for (uint64_t m = 0; m < nb; ++m) {
+      const Hash h = h_hash[m];
+      size_t q = (size_t)(h.a ^ (h.b >> 7)) & (cap - 1);
+      while (slots[q] >= 0) {
+        const Hash& o = h_hash[(size_t)reps[(size_t)slots[q]]];
+        if (o.a == h.a && o.b == h.b) break;
+        q = (q + 1) & (cap - 1);
+      }
+      if (slots[q] < 0) {
+        slots[q] = (int32_t)reps.size();
+        reps.push_back((int32_t)m);
+      }
+      state_of[m] = slots[q];
+    }
+    void *slab = nullptr, *d_kops = nullptr;
+    void** d_ptrs = nullptr;
+    double* d_norm = nullptr;
+    uint64_t U = 0;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+      U = reps.size();
+      drop_from(fixed);
+      int32_t differ = 0;
+      ok = take(state_bytes * U, "alloc trajectories", &slab) &&
+           take(rec * (size_t)R * U, "alloc op records", &d_kops) &&
+           take(sizeof(void*) * U, "alloc pointers", (void**)&d_ptrs) &&
+           take(sizeof(double) * U, "alloc norms", (void**)&d_norm);
+      if (!ok) break;
+      ptrs.resize(U);
+      for (uint64_t m = 0; m < U; ++m) ptrs[m] = (unsigned char*)slab + state_bytes * m;
+      ok = cuda_check(cudaMemcpyAsync(d_ptrs, ptrs.data(), sizeof(void*) * U, cudaMemcpyHostToDevice, st), "H2D") &&
+           cuda_check(cudaMemcpyAsync(d_state_of, state_of.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice, st),
+                      "H2D shot states") &&
+           cuda_check(cudaMemcpyAsync(d_reps, reps.data(), sizeof(int32_t) * U, cudaMemcpyHostToDevice, st),
+                      "H2D state shots") &&
+           cuda_check(cudaMemsetAsync(d_differ, 0, sizeof(int32_t), st), "clear check") &&
+           cuda_check(launch_noise_records(nr, d_choices, d_state_of, (int)nb, d_reps, (int)U, d_kops, d_differ, st),
+                      "op records") &&
+           cuda_check(cudaMemcpyAsync(&differ, d_differ, sizeof(differ), cudaMemcpyDeviceToHost, st), "D2H check") &&
+           cuda_check(cudaStreamSynchronize(st), "sync");
+      if (!ok || !differ || attempt) break;
+      // two choice vectors met in one 128-bit hash: group by the choices themselves
+      h_choices.resize(S * nb);
+      ok = cuda_check(cudaMemcpy(h_choices.data(), d_choices, S * nb, cudaMemcpyDeviceToHost), "D2H choices");
+      if (!ok) break;
+      std::unordered_map<std::string, int32_t> seen;
+      reps.clear();
+      for (uint64_t m = 0; m < nb; ++m) {
+        auto it = seen.emplace(std::string((const char*)h_choices.data() + m * S, S), (int32_t)reps.size());
+        if (it.second) reps.push_back((int32_t)m);
+        state_of[m] = it.first->second;
+      }
+    }
+    distinct += (int64_t)U;
+    ok = ok && cuda_check(launch_batch_zero(slab, precision, n_run, (int)U, st), "zero states");
     for (size_t p = 0; ok && p < P; ++p) {
       PassDesc pd = prog.steps[pass_steps[p]].pass;
       pd.op_begin = 0;
       pd.op_end = nops[p];
       ok = cuda_check(launch_tile_pass(precision, arith, tile_pass_io(prog, pass_steps[p]), n_run, pd, d_ptrs, (int)U,
-                                       d_kops + rec * (size_t)(rec_off[p] * (int64_t)U), nops[p], nullptr, st),
+                                       (unsigned char*)d_kops + rec * (size_t)(rec_off[p] * (int64_t)U), nops[p],
+                                       nullptr, st),
                       "trajectory pass");
     }
     ok = ok && cuda_check(launch_traj_normalise(precision, d_ptrs, (int)U, n_run, d_norm, st), "renormalise") &&
          cuda_check(launch_traj_sample(precision, d_ptrs, d_state_of, (int)nb, n_run, shift, seed, base,
                                        kStreamMeasure, d_out, st),
                     "trajectory sampling") &&
+         (!ro.on || cuda_check(launch_noise_readout(d_out, (int)nb, n, seed, base, kStreamReadout, ro.p01, ro.p10,
+                                                    ro.corr ? reinterpret_cast<const double*>(d_tab + o_fac) : nullptr,
+                                                    st),
+                               "readout noise")) &&
          cuda_check(cudaEventRecord(e1, st), "event") &&
          cuda_check(cudaMemcpyAsync(h_out.data(), d_out, sizeof(uint64_t) * nb, cudaMemcpyDeviceToHost, st), "D2H") &&
          cuda_check(cudaMemcpyAsync(h_norm.data(), d_norm, sizeof(double) * U, cudaMemcpyDeviceToHost, st), "D2H") &&
@@ -497,34 +514,29 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
       }
     }
     if (result != QG_OK) break;
-    parallel_for(nb, 1024, [&](uint64_t b, uint64_t e) {
-      for (uint64_t m = b; m < e; ++m) outcomes[base + m] = apply_readout(h_out[m], n, ro, seed, base + m);
-    });
-    // final states: the first max_trajectories shots, and the last shot
-    const uint64_t N = 1ULL << n, Nr = 1ULL << n_run;
-    for (uint64_t m = 0; m < nb; ++m) {
-      const uint64_t traj = base + m;
-      double* dst_t = (trajectories && traj < (uint64_t)max_trajectories) ? trajectories + 2 * N * traj : nullptr;
-      double* dst_f = (final_state && traj == shots - 1) ? final_state : nullptr;
-      if (!dst_t && !dst_f) continue;
-      host_state.resize(2 * Nr);
-      const unsigned char* src = (const unsigned char*)slab + state_bytes * (size_t)state_of[m];
-      if (precision == QG_C64) {
-        std::vector<float> f(2 * Nr);
-        ok = cuda_check(cudaMemcpy(f.data(), src, state_bytes, cudaMemcpyDeviceToHost), "D2H state");
-        for (uint64_t i = 0; i < 2 * Nr; ++i) host_state[i] = f[i];
-      } else {
-        ok = cuda_check(cudaMemcpy(host_state.data(), src, state_bytes, cudaMemcpyDeviceToHost), "D2H state");
+    std::memcpy(outcomes + base, h_out.data(), sizeof(uint64_t) * nb);
+    // final states: the first max_trajectories shots, and the last shot, collected without
+    // their padding qubits and copied kCollect bytes at a time
+    constexpr uint64_t kCollect = (uint64_t)256 << 20;
+    const uint64_t chunk = std::max<uint64_t>(1, kCollect / (16 * N));
+    auto collect = [&](uint64_t first, uint64_t count, double* dst) {
+      double* d_tr = nullptr;
+      const size_t at = held.size();
+      if (!take(16 * N * std::min(chunk, count), "alloc final states", (void**)&d_tr)) return false;
+      for (uint64_t t = 0; t < count; t += chunk) {
+        const uint64_t c = std::min(chunk, count - t);
+        if (!cuda_check(launch_noise_collect(precision, d_ptrs, d_state_of, (int)(first + t), (int)c, n, shift, d_tr, st),
+                        "final states") ||
+            !cuda_check(cudaMemcpyAsync(dst + 2 * N * t, d_tr, 16 * N * c, cudaMemcpyDeviceToHost, st), "D2H states") ||
+            !cuda_check(cudaStreamSynchronize(st), "sync"))
+          return false;
       }
-      if (!ok) break;
-      for (double* dst : {dst_t, dst_f}) {
-        if (!dst) continue;
-        for (uint64_t i = 0; i < N; ++i) {
-          dst[2 * i] = host_state[2 * (i << shift)];
-          dst[2 * i + 1] = host_state[2 * (i << shift) + 1];
-        }
-      }
-    }
+      drop_from(at);
+      return true;
+    };
+    const uint64_t keep = (uint64_t)max_trajectories;
+    if (trajectories && base < keep) ok = collect(0, std::min(nb, keep - base), trajectories + 2 * N * base);
+    if (ok && final_state && base + nb == shots) ok = collect(nb - 1, 1, final_state);
   }
   cleanup();
   if (!ok) return fail(QG_ERR_DEVICE, err);

@@ -296,6 +296,33 @@ cudaError_t launch_traj_normalise(int precision, void* const* d_states, int nsta
 cudaError_t launch_traj_sample(int precision, void* const* d_states, const int32_t* d_state_of, int nshots, int n,
                                int shift, uint64_t seed, uint64_t traj0, uint32_t stream, uint64_t* d_out,
                                cudaStream_t st);
+// Shots' Kraus choices, op records, readout noise and final states of noisy trajectories
+// (noisy_kernels.cu). A channel of `count` operators chooses the first c with
+// (draw >> 11) < below[c], the integer form of u < cumulative probability; the last one
+// otherwise. launch_noise_records sets *d_differ when a shot's choices are not those of
+// the shot reps[state_of[shot]], and writes the records of `states` states pass-major.
+struct NoiseChannel {
+  int32_t count, pad;
+  uint64_t below[3];
+};
+struct NoiseRecords {
+  const void* tmpl = nullptr;       // records x pieces x 16 bytes
+  const void* variants = nullptr;   // sites x 4 x pieces x 16 bytes
+  const int32_t* site_of = nullptr;
+  const int64_t* pass_off = nullptr;
+  const int32_t* pass_ops = nullptr;
+  int sites = 0, pieces = 0;
+  int64_t records = 0;
+};
+cudaError_t launch_noise_choices(const NoiseChannel* d_chans, const int32_t* d_site_chan, int sites, uint64_t shot0,
+                                 int shots, uint64_t seed, uint32_t stream, uint8_t* d_choices, void* d_hash,
+                                 cudaStream_t st);
+cudaError_t launch_noise_records(const NoiseRecords& r, const uint8_t* d_choices, const int32_t* d_state_of, int shots,
+                                 const int32_t* d_reps, int states, void* d_out, int32_t* d_differ, cudaStream_t st);
+cudaError_t launch_noise_readout(uint64_t* d_outcomes, int shots, int n, uint64_t seed, uint64_t shot0, uint32_t stream,
+                                 double p01, double p10, const double* d_factors, cudaStream_t st);
+cudaError_t launch_noise_collect(int precision, void* const* d_states, const int32_t* d_state_of, int first, int count,
+                                 int n, int shift, double* d_out, cudaStream_t st);
 int diag_max_terms_per_group();
 uint32_t diag_qmask(uint64_t z);  // bit q: parity of q & bits 8..11 of z
 cudaError_t launch_diag_expect(void* const* d_states, int precision, int n, const void* d_diag, const uint64_t* d_z,
