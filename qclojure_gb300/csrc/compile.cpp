@@ -572,6 +572,13 @@ void set_op_matrix(TOp* t, const double m[8]) {
   split_coeffs(t);
 }
 
+void set_op_operator(TOp* t, const double m[8]) {
+  const GOp g = classify(m, t->t, 0);
+  t->kind = g.kind < 0 ? OK_NONE : OK_U2;
+  t->cls = g.kind == OK_U2 ? g.cls : U2_DIAG;  // a phase form is diagonal
+  set_op_matrix(t, m);
+}
+
 namespace {
 
 // Insert OK_LAYOUT ops: consecutive ops whose non-diagonal bits fit in three

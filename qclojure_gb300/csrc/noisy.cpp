@@ -296,9 +296,11 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
   for (size_t s = 0; s < S; ++s) {
     const Channel& ch = chans[sites[s].entry];
     const PassDesc& pd = prog.steps[pass_steps[sites[s].pass]].pass;
-    TOp t = prog.tops[(size_t)(pd.op_begin + sites[s].at)];
     for (size_t v = 0; v < ch.applied.size(); ++v) {
-      set_op_matrix(&t, ch.applied[v].data());
+      // each operator in its own class: with weak noise nearly every choice is the identity,
+      // which costs its dispatch instead of a general 2x2 on every amplitude
+      TOp t = prog.tops[(size_t)(pd.op_begin + sites[s].at)];
+      set_op_operator(&t, ch.applied[v].data());
       encode_kops(precision, arith, &t, 1, variants.data() + rec * (4 * s + v));
     }
     site_of[(size_t)(rec_off[sites[s].pass] + sites[s].at)] = (int32_t)s;

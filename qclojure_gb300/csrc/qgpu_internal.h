@@ -41,7 +41,8 @@ enum OpKind : int32_t {
   OK_PARITY = 4,    // amp *= (parity(idx & mask) ? ph1 : ph0)
   OK_COLLAPSE = 5,  // amp = ((idx & mask) == val) ? amp * scale : 0
   OK_DENSE = 6,     // dense 2^dk x 2^dk block on bits dbits[0..dk) (dbits[0] = least significant)
-  OK_LAYOUT = 7     // tiled executor only: registers hold the local bits dbits[0..3) from here on
+  OK_LAYOUT = 7,    // tiled executor only: registers hold the local bits dbits[0..3) from here on
+  OK_NONE = 8       // tiled executor only: nothing (a noise site whose operator is the identity)
 };
 
 // Matrix classes of OK_U2 (picked on the host from exact zero / unit entries).
@@ -217,6 +218,9 @@ void ctx_report_error(void* ctx, const std::string& msg);
 int ctx_compile_tiled(void* ctx, const qg_circuit* c, int precision, Program* prog, std::string* err);
 // Set the 2x2 matrix of a tiled op (and its float-pair split for the float policies).
 void set_op_matrix(TOp* t, const double m[8]);
+// Makes the uncontrolled OK_U2 op t the operator m: the class that m's exact zero and unit
+// entries allow, or OK_NONE for the identity.
+void set_op_operator(TOp* t, const double m[8]);
 // ---------------------------------------------------------------------------
 // Specialised pass kernels (pass_kernels.cpp): every tiled pass of a program
 // (complex64, or complex128 double-float) compiled by NVRTC into its own

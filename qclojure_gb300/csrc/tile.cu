@@ -316,6 +316,7 @@ enum KCode : int32_t {
   KC_BLOCKADE = 62,
   KC_PARITY = 63,
   KC_COLLAPSE = 64,
+  KC_NONE = 65,    // nothing (a noise site whose operator is the identity)
   KF_COND = 0x100  // the op has control / mask conditions to evaluate
 };
 
@@ -1182,6 +1183,9 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
     k.rmr = t.rmask | (t.rval << 8);
     bool cond = t.tmask != 0 || t.rmask != 0;
     switch (t.kind) {
+      case OK_NONE:
+        k.code = KC_NONE;
+        break;
       case OK_U2:
         k.code = KC_U2 + t.cls * 4 + t.t2;
         k.gmask = k.gval = t.gcmask;
