@@ -113,7 +113,98 @@ inline bool hi_lo_nonzero(const TOp& t, int q) { return t.mf[8 + q] != 0.0f; }
 // blockade masks are data (they differ between members, for instance between
 // QAOA graphs), so the layout must not depend on them: ops keep their order
 // (no sinking, no look-ahead) and the free register bits ignore those masks.
-std::vector<TOp> plan_layouts(const TOp* ops, int nops, int k, int R, bool table = false, bool pair0 = false) {
+//
+// Index permutations. An X (no control, one local control, or tile controls), CNOT or SWAP
+// maps local indices by an affine map over GF(2), i -> M i ^ c. It needs no register bit and
+// no data movement of its own: every layout change already sends each register through
+// shared memory, so the permutations gathered since the last one only change the address a
+// register is read from (or, at the end of the pass, written to). LayoutMap holds that map:
+// column b is the image of local bit b, c0 the constant part, conds the parts that hold on
+// tiles whose index has all bits of a mask.
+struct LayoutMap {
+  uint16_t col[kMaxTileBits];
+  uint16_t c0 = 0;
+  std::vector<std::pair<uint64_t, uint16_t>> conds;
+  LayoutMap() {
+    for (int b = 0; b < kMaxTileBits; ++b) col[b] = (uint16_t)(1u << b);
+  }
+  bool identity() const {
+    for (int b = 0; b < kMaxTileBits; ++b)
+      if (col[b] != (1u << b)) return false;
+    return c0 == 0 && conds.empty();
+  }
+  uint16_t of(uint32_t l) const {  // the linear part
+    uint16_t r = 0;
+    for (int b = 0; b < kMaxTileBits; ++b)
+      if ((l >> b) & 1) r ^= col[b];
+    return r;
+  }
+  // this map after the permutation op (applied first): A -> A o op
+  void compose(const TOp& t) {
+    if (t.kind == OK_SWAP) {
+      std::swap(col[t.t], col[t.t2]);
+    } else if (t.lcmask) {
+      col[__builtin_ctz(t.lcmask)] ^= col[t.t];
+    } else if (t.gcmask) {
+      for (auto it = conds.begin(); it != conds.end(); ++it)
+        if (it->first == t.gcmask) {
+          it->second ^= col[t.t];
+          if (!it->second) conds.erase(it);
+          return;
+        }
+      conds.push_back({t.gcmask, col[t.t]});
+    } else {
+      c0 ^= col[t.t];
+    }
+  }
+  LayoutMap inverse() const {  // M^-1 by elimination; the constants go through it
+    uint32_t rows[kMaxTileBits], inv[kMaxTileBits];
+    for (int r = 0; r < kMaxTileBits; ++r) {
+      rows[r] = 0;
+      inv[r] = 1u << r;
+      for (int b = 0; b < kMaxTileBits; ++b) rows[r] |= (uint32_t)((col[b] >> r) & 1) << b;
+    }
+    for (int p = 0; p < kMaxTileBits; ++p) {
+      int r = p;
+      while (!((rows[r] >> p) & 1)) ++r;  // M is invertible: a product of invertible maps
+      std::swap(rows[r], rows[p]);
+      std::swap(inv[r], inv[p]);
+      for (int q = 0; q < kMaxTileBits; ++q)
+        if (q != p && ((rows[q] >> p) & 1)) {
+          rows[q] ^= rows[p];
+          inv[q] ^= inv[p];
+        }
+    }
+    LayoutMap m;
+    for (int b = 0; b < kMaxTileBits; ++b) {
+      m.col[b] = 0;
+      for (int r = 0; r < kMaxTileBits; ++r) m.col[b] |= (uint16_t)(((inv[r] >> b) & 1) << r);
+    }
+    m.c0 = m.of(c0);
+    for (const auto& c : conds) m.conds.push_back({c.first, m.of(c.second)});
+    return m;
+  }
+};
+
+bool is_permutation(const TOp& t) {
+  if (t.kind == OK_U2 && t.cls == U2_X)
+    return t.lcmask == 0 || (t.gcmask == 0 && (t.lcmask & (t.lcmask - 1)) == 0);
+  return t.kind == OK_SWAP && t.lcmask == 0 && t.gcmask == 0 && !(t.flags & 1);
+}
+
+// How a plan treats permutations: as register ops (their target is a register bit), in
+// layout changes only, or in layout changes unless a group's register bits hold the target
+// already.
+enum PermMode { kPermRegisters, kPermLayouts, kPermBoth };
+
+struct LayoutPlan {
+  std::vector<TOp> ops;          // an OK_LAYOUT's pad1 is its map's index
+  std::vector<LayoutMap> maps;   // where each layout's registers are read from
+  LayoutMap last;                // where the last layout's registers are written to
+  int layouts = 0, moves = 0;    // moves: permutations applied to registers
+};
+
+LayoutPlan plan_layouts_mode(const TOp* ops, int nops, int k, int R, bool table, bool pair0, PermMode mode) {
   auto required = [](const TOp& t) -> uint32_t {
     if (t.kind == OK_U2) return 1u << t.t;
     if (t.kind == OK_SWAP) return (1u << t.t) | (1u << t.t2);
@@ -148,7 +239,8 @@ std::vector<TOp> plan_layouts(const TOp* ops, int nops, int k, int R, bool table
     }
     flush(0, true);
   }
-  std::vector<TOp> out;
+  LayoutPlan plan;
+  std::vector<TOp>& out = plan.ops;
   auto cond_bits = [&](const TOp& t) -> uint32_t {
     if (data_mask(t)) return 0u;
     return t.kind == OK_U2 || t.kind == OK_SWAP ? t.lcmask : t.lmask;
@@ -160,13 +252,39 @@ std::vector<TOp> plan_layouts(const TOp* ops, int nops, int k, int R, bool table
   // shared memory and fewer barriers.
   std::vector<char> taken(in.size(), 0);
   size_t first = 0;
-  while (first < in.size()) {
+  LayoutMap map;  // permutations since the last layout
+  bool pending = false;
+  while (first < in.size() || pending) {
     uint32_t rb = 0, changed = 0, seen = 0;
+    if (mode != kPermRegisters) {
+      // permutations that commute with every op left out before them join the layout change
+      for (size_t j = first; j < in.size(); ++j) {
+        if (taken[j]) continue;
+        const uint32_t req = required(in[j]), tb = req | cond_bits(in[j]);
+        if (is_permutation(in[j]) && (req & seen) == 0 && ((tb & ~req) & changed) == 0) {
+          map.compose(in[j]);
+          pending = true;
+          taken[j] = 1;
+        } else {
+          changed |= req;
+          seen |= tb;
+        }
+      }
+      while (first < in.size() && taken[first]) ++first;
+      if (first == in.size() && plan.layouts > 0) {  // nothing left: the last registers are written through it
+        plan.last = map.inverse();
+        break;
+      }
+      pending = false;
+      changed = seen = 0;
+    }
     std::vector<TOp> grp;
     for (size_t j = first; j < in.size(); ++j) {
       if (taken[j]) continue;
       const uint32_t req = required(in[j]), tb = req | cond_bits(in[j]);
-      const bool commutes = (req & seen) == 0 && ((tb & ~req) & changed) == 0;
+      const bool perm = mode != kPermRegisters && is_permutation(in[j]);
+      const bool commutes = (req & seen) == 0 && ((tb & ~req) & changed) == 0 &&
+                            (!perm || (mode == kPermBoth && (req & ~rb) == 0));
       if (commutes && __builtin_popcount(rb | req) <= R) {
         rb |= req;
         grp.push_back(in[j]);
@@ -201,6 +319,10 @@ std::vector<TOp> plan_layouts(const TOp* ops, int nops, int k, int R, bool table
     std::memset(&lay, 0, sizeof(lay));
     lay.kind = OK_LAYOUT;
     for (int q = 0; q < R; ++q) lay.dbits[q] = pos[q];
+    lay.pad1 = (int)plan.maps.size();
+    plan.maps.push_back(map);
+    map = LayoutMap();
+    ++plan.layouts;
     out.push_back(lay);
     auto rpos = [&](int b) {
       for (int q = 0; q < R; ++q)
@@ -237,10 +359,31 @@ std::vector<TOp> plan_layouts(const TOp* ops, int nops, int k, int R, bool table
       t.rval = reg_part(v);
       t.tmask = m & ~rb;
       t.tval = v & ~rb;
+      if (is_permutation(t)) ++plan.moves;
       out.push_back(t);
     }
   }
-  return out;
+  return plan;
+}
+
+// The cheapest of the three treatments of permutations: a layout change costs each register a
+// store, a barrier and a load, a map a second barrier, a permutation of registers its selects
+// or moves. The weights were measured (layers + QFT, ms; register ops only 50.7 at 28 qubits
+// complex128 and 30.4 at 29 qubits complex64): 10, 3, 1 gives 48.2 and 28.4; 10, 0, 3: 50.6 and
+// 28.9; 10, 6, 3: 48.5 and 28.8; 10, 10, 1: 48.9 and 29.8.
+LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table = false, bool pair0 = false) {
+  LayoutPlan best = plan_layouts_mode(ops, nops, k, R, table, pair0, kPermRegisters);
+  if (table) return best;  // members of a sweep share one plan in circuit order
+  auto cost = [](const LayoutPlan& p) {
+    int mapped = p.last.identity() ? 0 : 1;
+    for (const LayoutMap& m : p.maps) mapped += m.identity() ? 0 : 1;
+    return 10 * p.layouts + 3 * mapped + p.moves;
+  };
+  for (const PermMode m : {kPermBoth, kPermLayouts}) {
+    LayoutPlan p = plan_layouts_mode(ops, nops, k, R, table, pair0, m);
+    if (cost(p) < cost(best)) best = std::move(p);
+  }
+  return best;
 }
 
 // A real or RX-shaped 2x2 whose diagonal is (1, +-1) (a rotation with its
@@ -312,8 +455,8 @@ class PassGen {
     if (!unsupported_) plan_ = plan_layouts(tagged.data(), nops, pd.k, sh_.rbits, table, !df_);
     // pairs handed over by the previous pass may carry unnormalised operations
     if (io & kTileInPairs) carry_ = kRenormEvery / 2 - 1;
-    ops_ = plan_.data();
-    nops_ = (int)plan_.size();
+    ops_ = plan_.ops.data();
+    nops_ = (int)plan_.ops.size();
     ns_ = 1 << sh_.rbits;
     if (ns_ > kMaxRegs) unsupported_ = true;  // the generator's per-register tables hold 16
   }
@@ -369,7 +512,7 @@ class PassGen {
   bool tab_;
   Shape sh_;
   bool unsupported_ = false;
-  std::vector<TOp> plan_;
+  LayoutPlan plan_;
   const TOp* ops_ = nullptr;
   int nops_ = 0;
   int ns_ = 8;  // registers (amplitudes) per thread: at most kMaxRegs
@@ -432,9 +575,55 @@ class PassGen {
   // register p goes to the slot of logical register p ^ xm
   // complex64 with tile bit 0 as register bit 0: registers j, j + 1 (j even) fill one
   // 16-byte slot pair (the swizzle keeps bit 0)
-  bool paired() const { return !df_ && rpos_[0] == 0; }
+  // (and the map the registers are read or written through keeps their halves in place)
+  bool paired(const LayoutMap& m) const {
+    if (df_ || rpos_[0] != 0 || m.col[0] != 1u || (m.c0 & 1u)) return false;
+    for (int b = 1; b < kMaxTileBits; ++b)
+      if (m.col[b] & 1u) return false;
+    for (const auto& c : m.conds)
+      if (c.second & 1u) return false;
+    return true;
+  }
+  // the linear part of a map on the thread's index bits, and its constants on this tile
+  std::string mapped_thread(const LayoutMap& m) const {
+    uint32_t rb = 0, keep = 0;
+    for (int q = 0; q < sh_.rbits; ++q) rb |= 1u << rpos_[q];
+    std::string e;
+    for (int b = 0; b < pd_.k; ++b) {
+      if ((rb >> b) & 1) continue;
+      if (m.col[b] == (1u << b)) keep |= 1u << b;
+      else e += " ^ ((0u - ((lt >> " + std::to_string(b) + ") & 1u)) & " + hex32(m.col[b]) + ")";
+    }
+    if (m.c0) e += " ^ " + hex32(m.c0);
+    for (const auto& c : m.conds)
+      e += " ^ ((base & " + hex64(c.first) + ") == " + hex64(c.first) + " ? " + hex32(c.second) + " : 0u)";
+    return "(lt & " + hex32(keep) + ")" + e;
+  }
+  uint32_t reg_offset(int j) const {  // register j's local index bits under the current layout
+    uint32_t lj = 0;
+    for (int q = 0; q < sh_.rbits; ++q)
+      if ((j >> q) & 1) lj |= 1u << rpos_[q];
+    return lj;
+  }
+  // store through a map that is not the identity (the end of a pass)
+  void store_mapped(const std::string& fn, const LayoutMap& m) {
+    const std::string E = std::to_string(df_ ? 16 : 8);
+    o_ << "    { const int pm = swz<" << E << ">((int)(" << mapped_thread(m) << "))";
+    for (int bb = 0; bb < sh_.rbits; ++bb)
+      if ((pend_ >> bb) & 1)
+        o_ << " ^ swz<" << E << ">((int)(((xm >> " << bb << ") & 1u) * " << hex32(m.col[rpos_[bb]]) << "))";
+    o_ << ";\n";
+    const bool pair = paired(m) && !(pend_ & 1u);
+    for (int j = 0; j < ns_; j += pair ? 2 : 1) {
+      const std::string at = "pm ^ swz<" + E + ">(" + hex32(m.of(reg_offset(j))) + ")";
+      if (pair) o_ << "      F32::st_pair(buf, " << at << ", r" << j << ", r" << j + 1 << ");\n";
+      else o_ << "      " << fn << "(buf, " << at << ", r" << j << ");\n";
+    }
+    o_ << "    }\n    xm = 0u;\n";
+    pend_ = 0;
+  }
   void store_regs(const std::string& fn) {
-    if (paired() && !(pend_ & 1u)) {  // a pending X of register bit 0 would swap the halves
+    if (paired(LayoutMap()) && !(pend_ & 1u)) {  // a pending X of register bit 0 would swap the halves
       std::string xo = "";
       if (pend_) {
         const int E = 8;
@@ -1127,13 +1316,45 @@ class PassGen {
       order.push_back(b);
       used |= 1u << b;
     };
-    if (!df_ && !(rb & 1u)) take(0);
-    for (int c = 0; c < 3; ++c)
-      for (int b = c + (df_ ? 0 : 1); b < pd_.k; b += 3)
-        if (!(used & (1u << b))) {
-          take(b);
-          break;
-        }
+    // bank vector of an index offset: its 16-byte unit in the row (and the half, bit 0 of an
+    // 8-byte amplitude); lanes are conflict-free when the vectors of their bits are independent,
+    // as stored (the bits themselves) and as read (their images under the layout's map)
+    auto bank = [&](uint32_t l) {
+      uint32_t v = 0;
+      for (int b = 0; b < kMaxTileBits; ++b)
+        if ((l >> b) & 1) v ^= df_ ? 1u << (b % 3) : (b == 0 ? 1u : 2u << ((b - 1) % 3));
+      return v;
+    };
+    const LayoutMap& m = plan_.maps[(size_t)t.pad1];
+    const bool low = !df_ && !(rb & 1u);  // bit 0 of 8-byte amplitudes on a lane
+    if (low) take(0);
+    auto independent = [&](const std::vector<uint32_t>& vs) {
+      for (uint32_t pick = 1; pick < (1u << vs.size()); ++pick) {
+        uint32_t x = 0;
+        for (size_t i = 0; i < vs.size(); ++i)
+          if ((pick >> i) & 1) x ^= vs[i];
+        if (!x) return false;
+      }
+      return true;
+    };
+    int lanes[3] = {-1, -1, -1};
+    for (int mapped = 1; mapped >= 0 && lanes[0] < 0; --mapped)
+      for (int a = 0; a < pd_.k && lanes[0] < 0; ++a)
+        for (int b = a + 1; b < pd_.k && lanes[0] < 0; ++b)
+          for (int c = b + 1; c < pd_.k && lanes[0] < 0; ++c) {
+            if (used & ((1u << a) | (1u << b) | (1u << c))) continue;
+            std::vector<uint32_t> st, ld;
+            if (low) st.push_back(bank(1u)), ld.push_back(bank(m.col[0]));
+            for (int x : {a, b, c}) {
+              uint32_t sv = bank(1u << x), lv = bank(m.col[x]);
+              if (!df_ && !low) sv &= ~1u, lv &= ~1u;  // 16-byte pairs: the unit only
+              st.push_back(sv);
+              ld.push_back(lv);
+            }
+            if (independent(st) && (!mapped || independent(ld))) lanes[0] = a, lanes[1] = b, lanes[2] = c;
+          }
+    for (int x : lanes)
+      if (x >= 0) take(x);
     for (int b = 0; b < pd_.k; ++b)
       if (!(used & (1u << b))) take(b);
     o_ << "    lt = 0u";
@@ -1157,12 +1378,15 @@ class PassGen {
     o_ << ";\n    unsigned lt = 0, xm = 0u;\n";
     o_ << "    (void)lt; (void)xm;\n";
     pend_ = 0;
-    bool in_regs = false, raw = true;
+    // a register read through a map comes from a slot that another thread will store to:
+    // those stores wait for every thread's reads
+    bool in_regs = false, raw = true, moved_in = false;
     for (int i = 0; i < nops_; ++i) {
       const TOp& t = ops_[i];
       if (t.kind == OK_LAYOUT) {
         if (in_regs) {
           renorm_for_store();
+          if (moved_in) o_ << "    __syncthreads();\n";
           store_regs(std::string(pol()) + "::st_work");
           o_ << "    __syncthreads();\n";
           raw = false;
@@ -1176,12 +1400,17 @@ class PassGen {
           o_ << "    q" << j << " = swz<" << E << ">((int)(lt | " << hex32(lj) << "));\n";
         }
         const std::string ld = raw ? ld_raw() : std::string(pol()) + "::ld_work";
-        if (paired()) {  // complex64: raw and working forms are the same
-          for (int j = 0; j < ns_; j += 2)
-            o_ << "    F32::ld_pair(buf, q" << j << ", r" << j << ", r" << j + 1 << ");\n";
-        } else {
-          for (int j = 0; j < ns_; ++j) o_ << "    r" << j << " = " << ld << "(buf, q" << j << ");\n";
+        const LayoutMap& m = plan_.maps[(size_t)t.pad1];
+        const bool moved = !m.identity(), pair = paired(m);  // pairs: complex64, one form only
+        if (moved) o_ << "    { const int pm = swz<" << E << ">((int)(" << mapped_thread(m) << "));\n";
+        for (int j = 0; j < ns_; j += pair ? 2 : 1) {
+          const std::string at = moved ? "pm ^ swz<" + std::to_string(E) + ">(" + hex32(m.of(reg_offset(j))) + ")"
+                                       : "q" + std::to_string(j);
+          if (pair) o_ << "    F32::ld_pair(buf, " << at << ", r" << j << ", r" << j + 1 << ");\n";
+          else o_ << "    r" << j << " = " << ld << "(buf, " << at << ");\n";
         }
+        if (moved) o_ << "    }\n";
+        moved_in = moved;
         for (int j = 0; j < ns_; ++j) since_[j] = carry_;
         in_regs = true;
         continue;
@@ -1207,7 +1436,9 @@ class PassGen {
     }
     if (in_regs) {
       if (io_ & kTileOutPairs) renorm_for_store();  // st_doubles normalises on its own
-      store_regs(st_raw());
+      if (moved_in || !plan_.last.identity()) o_ << "    __syncthreads();\n";
+      if (plan_.last.identity()) store_regs(st_raw());
+      else store_mapped(st_raw(), plan_.last);
     } else if (df_ && ((io_ & kTileInPairs) != 0) != ((io_ & kTileOutPairs) != 0)) {
       // no op loaded the tile: convert its storage form in place, each thread its own slots
       o_ << "    for (int l = (int)tid; l < (1 << K_BITS); l += (1 << K_BITS) >> R_BITS) {\n"
@@ -1791,7 +2022,7 @@ void pass_coefficients(const Program& prog, size_t step, int prec, float* out) {
   std::vector<TOp> tagged(ops, ops + nops);
   for (int i = 0; i < nops; ++i) tagged[i].pad1 = i;
   const std::vector<TOp> plan =
-      plan_layouts(tagged.data(), nops, pd.k, shape_of(prog, prec).rbits, true, prec == QG_C64);
+      plan_layouts(tagged.data(), nops, pd.k, shape_of(prog, prec).rbits, true, prec == QG_C64).ops;
   const int ns = 1 << shape_of(prog, prec).rbits;  // registers per thread
   auto put = [&](float* at, std::complex<double> v) {
     if (prec == QG_C128) {
