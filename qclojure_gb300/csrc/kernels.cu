@@ -11,6 +11,7 @@
 // The complex128 path therefore reproduces the CPU restatement bit for bit, and
 // the plain (one pass per gate) and tiled (many gates per pass) executors give
 // identical amplitudes. Dense fused blocks use FMA and are checked to tolerance.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 
@@ -661,29 +662,44 @@ __global__ void __launch_bounds__(256, 3) k_samp_sums(const typename C2<R>::T* _
 // single CTA: exclusive prefix of block sums (bpre[nb] = T) and the FP64 total
 // T 2^-62 + N 2^-63: every quantised probability lost less than one unit of
 // 2^-62 to the floor, so the estimate is within N 2^-63 of sum p (2e-9 at 34
-// qubits, well inside the 1e-8 normalisation tolerance).
+// qubits, well inside the 1e-8 normalisation tolerance). Latency-bound: each thread adds up
+// 16 consecutive sums, one warp-shuffle scan covers 16384 of them (30 qubits, 2^17 sums:
+// 228 us with a 1024-entry scan in shared memory per step).
+constexpr int kScanPer = 16;
 __global__ void __launch_bounds__(1024) k_samp_scan(const unsigned long long* __restrict__ bsum, uint64_t nb,
                                                     uint64_t n_amps, unsigned long long* __restrict__ bpre,
                                                     double* __restrict__ total) {
-  __shared__ unsigned long long sh[1024];
-  __shared__ unsigned long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint64_t base = 0; base < nb; base += 1024) {
-    uint64_t i = base + threadIdx.x;
-    unsigned long long v = i < nb ? bsum[i] : 0ULL;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {  // Hillis-Steele inclusive scan
-      unsigned long long add = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : 0ULL;
-      __syncthreads();
-      sh[threadIdx.x] += add;
-      __syncthreads();
+  __shared__ unsigned long long wsum[2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long carry = 0;
+  int par = 0;
+  for (uint64_t base = 0; base < nb; base += 1024 * kScanPer, par ^= 1) {
+    const uint64_t i0 = base + (uint64_t)threadIdx.x * kScanPer;
+    unsigned long long v[kScanPer], mine = 0;
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+      v[k] = i0 + k < nb ? bsum[i0 + k] : 0ULL;
+      mine += v[k];
     }
-    if (i < nb) bpre[i] = carry + sh[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry += sh[1023];
-    __syncthreads();
+    unsigned long long incl = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) wsum[par][warp] = incl;
+    __syncthreads();  // the other half of wsum is written in the next round: one barrier each
+    unsigned long long all = wsum[par][lane], before = lane < warp ? all : 0ULL;
+    for (int o = 16; o > 0; o >>= 1) {
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    unsigned long long at = carry + before + incl - mine;
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+      if (i0 + k < nb) bpre[i0 + k] = at;
+      at += v[k];
+    }
+    carry += all;
   }
   if (threadIdx.x == 0) {
     total[0] = (double)carry * 0x1p-62 + (double)n_amps * 0x1p-63;
@@ -691,73 +707,93 @@ __global__ void __launch_bounds__(1024) k_samp_scan(const unsigned long long* __
   }
 }
 
-// one warp per shot
+// One warp per shot, `batch` (1..32) shots one after the other with their draws computed
+// side by side. The block is found 32 ways at a time (2^17 blocks: four dependent loads; a
+// binary search made 17), its chunk by a scan of the block's 256 sums, 64 bytes per lane, the
+// amplitude by a scan of the chunk. Bound by the latency of these loads (30 qubits, 10^6
+// shots: 977 us with the binary search and one Philox draw per lane and shot).
 template <typename R>
 __global__ void __launch_bounds__(256) k_samp_resolve(const typename C2<R>::T* __restrict__ s, SampleGeom g,
                                                       const unsigned long long* __restrict__ csum,
                                                       const unsigned long long* __restrict__ bpre, uint64_t shots,
-                                                      uint64_t seed, uint64_t* __restrict__ out) {
+                                                      uint64_t seed, int batch, uint64_t* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t stride = (((uint64_t)gridDim.x * blockDim.x) >> 5) * (uint64_t)batch;
   const unsigned long long T = bpre[g.nb];
-  for (uint64_t shot = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; shot < shots; shot += warps) {
+  const int per = (g.cpb + 31) / 32;
+  for (uint64_t first = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (uint64_t)batch; first < shots;
+       first += stride) {
+    const int cnt = (int)(shots - first < (uint64_t)batch ? shots - first : (uint64_t)batch);
     if (T == 0) {
-      if (lane == 0) out[shot] = 0;
+      if (lane < cnt) out[first + lane] = 0;
       continue;
     }
-    unsigned long long u = __umul64hi(draw64(seed, shot, 0u), T);
-    // block: first b with bpre[b+1] > u
-    uint64_t lo = 0, hi = g.nb - 1;
-    while (lo < hi) {
-      uint64_t mid = (lo + hi) >> 1;
-      if (bpre[mid + 1] > u) hi = mid; else lo = mid + 1;
-    }
-    const uint64_t b = lo;
-    unsigned long long r = u - bpre[b];
-    // chunk within block: cpb <= 256 chunk sums, 8 per lane
-    const int per = (g.cpb + 31) / 32;
-    unsigned long long loc[8];
-    unsigned long long mine = 0;
-    for (int k = 0; k < per; ++k) {
-      int c = lane * per + k;
-      loc[k] = c < g.cpb ? csum[b * g.cpb + c] : 0ULL;
-      mine += loc[k];
-    }
-    unsigned long long incl = mine;
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    unsigned long long excl = incl - mine;
-    unsigned ballot = __ballot_sync(0xffffffffu, incl > r);
-    int owner = ballot ? __ffs(ballot) - 1 : 31;
-    int chunk_in_block = 0;
-    unsigned long long before = 0;
-    if (lane == owner) {
-      unsigned long long c = excl;
-      int kk = 0;
-      for (; kk < per; ++kk) {
-        if (c + loc[kk] > r) break;
-        c += loc[kk];
+    unsigned long long draw = 0, picked = 0;
+    if (lane < cnt) draw = __umul64hi(draw64(seed, first + lane, 0u), T);
+    for (int q = 0; q < cnt; ++q) {
+      const unsigned long long u = __shfl_sync(0xffffffffu, draw, q);
+      // block: first b with bpre[b + 1] > u; bpre[nb] = T > u
+      uint64_t b = 0, len = g.nb;
+      while (len > 1) {
+        const uint64_t step = (len + 31) >> 5, at = (uint64_t)(lane + 1) * step;
+        const unsigned hit = __ballot_sync(0xffffffffu, bpre[b + (at < len ? at : len)] > u);
+        const uint64_t skip = (uint64_t)(__ffs((int)hit) - 1) * step;
+        b += skip;
+        len = len - skip < step ? len - skip : step;
       }
-      if (kk >= per) kk = per - 1;
-      chunk_in_block = lane * per + kk;
-      before = c;
+      const unsigned long long r = u - bpre[b];
+      // chunk within block: cpb <= 256 chunk sums, 8 per lane
+      unsigned long long loc[8];
+      unsigned long long mine = 0;
+      if (g.cpb == 256) {
+        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(csum + b * 256) + lane * 4;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const ulonglong2 x = src[k];
+          loc[2 * k] = x.x;
+          loc[2 * k + 1] = x.y;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int c = lane * per + k;
+          loc[k] = k < per && c < g.cpb ? csum[b * g.cpb + c] : 0ULL;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) mine += loc[k];
+      unsigned long long incl = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const unsigned ballot = __ballot_sync(0xffffffffu, incl > r);
+      const int owner = ballot ? __ffs(ballot) - 1 : 31;
+      // the owner's first chunk whose cumulative sum exceeds r (its last one otherwise)
+      unsigned long long before = incl - mine;
+      int kk = 0;
+#pragma unroll
+      for (int k = 0; k < 7; ++k)
+        if (kk == k && k < per - 1 && before + loc[k] <= r) {
+          before += loc[k];
+          kk = k + 1;
+        }
+      int chunk_in_block = lane * per + kk;
       if (chunk_in_block >= g.cpb) chunk_in_block = g.cpb - 1;
+      chunk_in_block = __shfl_sync(0xffffffffu, chunk_in_block, owner);
+      before = __shfl_sync(0xffffffffu, before, owner);
+      const unsigned long long r2 = r - before;
+      const uint64_t chunk = b * g.cpb + chunk_in_block;
+      unsigned long long qi = lane < g.ch ? quant(p_of<R>(s[chunk * g.ch + lane])) : 0ULL;
+      for (int o = 1; o < 32; o <<= 1) {
+        unsigned long long v = __shfl_up_sync(0xffffffffu, qi, o);
+        if (lane >= o) qi += v;
+      }
+      const unsigned bl = __ballot_sync(0xffffffffu, (lane < g.ch) && qi > r2);
+      const int pick = bl ? __ffs(bl) - 1 : g.ch - 1;
+      if (lane == q) picked = chunk * g.ch + pick;
     }
-    chunk_in_block = __shfl_sync(0xffffffffu, chunk_in_block, owner);
-    before = __shfl_sync(0xffffffffu, before, owner);
-    unsigned long long r2 = r - before;
-    const uint64_t chunk = b * g.cpb + chunk_in_block;
-    unsigned long long q = lane < g.ch ? quant(p_of<R>(s[chunk * g.ch + lane])) : 0ULL;
-    unsigned long long qi = q;
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned long long v = __shfl_up_sync(0xffffffffu, qi, o);
-      if (lane >= o) qi += v;
-    }
-    unsigned bl = __ballot_sync(0xffffffffu, (lane < g.ch) && qi > r2);
-    int pick = bl ? __ffs(bl) - 1 : g.ch - 1;
-    if (lane == 0) out[shot] = chunk * g.ch + pick;
+    if (lane < cnt) out[first + lane] = picked;
   }
 }
 
@@ -1009,13 +1045,15 @@ cudaError_t launch_sample(const void* s, int precision, int n, uint64_t shots, u
   e = cudaGetLastError();
   counted(2);
   if (e != cudaSuccess || shots == 0) return e;
-  uint64_t warps_needed = shots;
-  uint64_t blocks = (warps_needed * 32 + 255) / 256;
-  if (blocks > (uint64_t)kSMs * 16) blocks = (uint64_t)kSMs * 16;
+  const uint64_t most = (uint64_t)kSMs * 16 * 8;  // warps of a full grid
+  const int batch = (int)std::min<uint64_t>(32, (shots + most - 1) / most);
+  const uint64_t warps_needed = (shots + batch - 1) / batch;
+  const uint64_t blocks = std::min<uint64_t>((warps_needed + 7) / 8, (uint64_t)kSMs * 16);
   if (precision == QG_C64)
-    k_samp_resolve<float><<<(unsigned)blocks, 256, 0, st>>>((const float2*)s, g, csum, bpre, shots, seed, d_outcomes);
+    k_samp_resolve<float><<<(unsigned)blocks, 256, 0, st>>>((const float2*)s, g, csum, bpre, shots, seed, batch,
+                                                            d_outcomes);
   else
-    k_samp_resolve<double><<<(unsigned)blocks, 256, 0, st>>>((const double2*)s, g, csum, bpre, shots, seed,
+    k_samp_resolve<double><<<(unsigned)blocks, 256, 0, st>>>((const double2*)s, g, csum, bpre, shots, seed, batch,
                                                              d_outcomes);
   counted();
   return cudaGetLastError();

@@ -542,35 +542,36 @@ static int st_compare(State* a, State* b, double* out, std::string* err) {
   return QG_OK;
 }
 
-static int st_sample(State* s, uint64_t shots, uint64_t seed, std::vector<uint64_t>* outcomes, std::string* err) {
-  size_t scratch = sampler_scratch_bytes(s->n, shots);
-  void* d_scratch = nullptr;
-  uint64_t* d_out = nullptr;
-  double* d_total = nullptr;
-  CK(cudaMallocAsync(&d_scratch, scratch, s->stream), "alloc sampler");
-  CK(cudaMallocAsync((void**)&d_out, sizeof(uint64_t) * std::max<uint64_t>(shots, 1), s->stream), "alloc outcomes");
-  CK(cudaMallocAsync((void**)&d_total, sizeof(double) * 2, s->stream), "alloc total");
-  CK(launch_sample(s->d, s->prec, s->n, shots, seed, d_scratch, d_out, d_total, s->stream), "sample");
+// outcomes: `shots` values on the host, written when the state is normalised. They are copied
+// straight into the caller's buffer (an intermediate vector of 10^6 outcomes cost 0.5 ms of
+// page faults and copies).
+static int st_sample(State* s, uint64_t shots, uint64_t seed, uint64_t* outcomes, std::string* err) {
+  const size_t scratch = (sampler_scratch_bytes(s->n, shots) + 255) / 256 * 256;
+  unsigned char* d = nullptr;  // scratch, total, outcomes
+  CK(cudaMallocAsync((void**)&d, scratch + 256 + sizeof(uint64_t) * shots, s->stream), "alloc sampler");
+  double* d_total = reinterpret_cast<double*>(d + scratch);
+  uint64_t* d_out = reinterpret_cast<uint64_t*>(d + scratch + 256);
   double total = 0;
-  outcomes->resize(shots);
-  CK(cudaMemcpyAsync(&total, d_total, sizeof(double), cudaMemcpyDeviceToHost, s->stream), "D2H total");
-  if (shots) {
-    CK(cudaMemcpyAsync(outcomes->data(), d_out, sizeof(uint64_t) * shots, cudaMemcpyDeviceToHost, s->stream),
-       "D2H outcomes");
-  }
-  CK(cudaStreamSynchronize(s->stream), "sync");
-  cudaFreeAsync(d_scratch, s->stream);
-  cudaFreeAsync(d_out, s->stream);
-  cudaFreeAsync(d_total, s->stream);
+  int rc = QG_OK;
+  cudaError_t e = launch_sample(s->d, s->prec, s->n, shots, seed, d, d_out, d_total, s->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&total, d_total, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   // state.clj:901-903 rejects |sum p - 1| > 1e-8; a complex64 state carries FP32
   // rounding (about 1e-7 per gate), so its check allows 1e-4 instead.
   const double norm_tol = s->prec == QG_C64 ? 1e-4 : 1e-8;
-  if (std::fabs(total - 1.0) > norm_tol) {
+  if (e != cudaSuccess) {
+    rc = cuda_fail(err, e, "sample");
+  } else if (std::fabs(total - 1.0) > norm_tol) {
     *err = "State is not properly normalized (total probability " + std::to_string(total) + ")";
-    outcomes->clear();
-    return QG_ERR_NOT_NORMALIZED;
+    rc = QG_ERR_NOT_NORMALIZED;
+  } else if (shots) {
+    e = cudaMemcpyAsync(outcomes, d_out, sizeof(uint64_t) * shots, cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) rc = cuda_fail(err, e, "D2H outcomes");
   }
-  return QG_OK;
+  cudaFreeAsync(d, s->stream);
+  return rc;
 }
 
 static int st_probs(State* s, double* host, std::string* err) {
@@ -885,7 +886,9 @@ static int job_results(Ctx* c, Job* j, std::unique_ptr<State> st, cudaStream_t s
   const SpecCopy& sp = j->spec;
   const uint64_t N = 1ULL << j->n;
   if (rc == QG_OK && (sp.flags & QG_RES_MEASUREMENTS)) {
-    rc = st_sample(st.get(), sp.shots, j->seed, &j->shots, &err);
+    j->shots.resize(sp.shots);
+    rc = st_sample(st.get(), sp.shots, j->seed, j->shots.data(), &err);
+    if (rc != QG_OK) j->shots.clear();
     if (rc == QG_OK) {
       std::vector<uint64_t> sorted = j->shots;
       std::sort(sorted.begin(), sorted.end());
@@ -2349,10 +2352,7 @@ int qg_state_sample(void* state, uint64_t shots, uint64_t seed, uint64_t* host_o
   State* s = (State*)state;
   cudaSetDevice(s->ctx->device);
   std::string err;
-  std::vector<uint64_t> out;
-  int rc = st_sample(s, shots, seed, &out, &err);
-  if (rc == QG_OK && shots) std::memcpy(host_outcomes, out.data(), sizeof(uint64_t) * shots);
-  return state_err(s, rc, err);
+  return state_err(s, st_sample(s, shots, seed, host_outcomes, &err), err);
 }
 
 // Same kernels and outcomes as qg_state_sample; the scratch is the file-scope array
