@@ -283,6 +283,7 @@ constexpr int kPassKernelMinQubits = 29;
 // while the device works through the queue, so the compile costs the job nothing.
 constexpr int kPrecompileMinQubits = 20;
 constexpr int kPrecompileThreads = 2;
+constexpr std::chrono::milliseconds kPrecompileWait{250};  // queued for at least this long
 
 static std::shared_ptr<const PassKernels> maybe_pass_kernels(const State* s, const Program& prog);
 static std::shared_ptr<const PassKernels> forced_pass_kernels(const State* s, const Program& prog);
@@ -1638,18 +1639,32 @@ static void precompile_loop(Ctx* c) {
       if (c->pre_stop) break;
       // the queued job with the most interpreted work (2^n amplitudes x gates) first: a
       // compile costs all host cores for seconds, and the largest jobs save the most
-      // device time by it (a 28-qubit job hundreds of milliseconds, a 20-qubit job a few)
-      auto best = c->pre_queue.begin();
+      // device time by it (a 28-qubit job hundreds of milliseconds, a 20-qubit job a few).
+      // Only jobs that have waited kPrecompileWait count: a backlog that drains sooner than
+      // that has run them before a compile could finish.
+      const auto now = Clock::now();
+      auto next = now + kPrecompileWait;
       double best_w = -1.0;
-      for (auto it = c->pre_queue.begin(); it != c->pre_queue.end(); ++it) {
-        const double w = std::ldexp((double)(*it)->ops.size(), (*it)->n);
-        if ((*it)->status.load() == QG_JOB_QUEUED && w > best_w) {
-          best_w = w;
-          best = it;
+      for (auto it = c->pre_queue.begin(); it != c->pre_queue.end();) {
+        if ((*it)->status.load() != QG_JOB_QUEUED) {  // started or finished meanwhile
+          it = c->pre_queue.erase(it);
+          continue;
         }
+        const auto due = (*it)->submitted + kPrecompileWait;
+        const double w = std::ldexp((double)(*it)->ops.size(), (*it)->n);
+        if (due > now) {
+          next = std::min(next, due);
+        } else if (w > best_w) {
+          best_w = w;
+          j = *it;
+        }
+        ++it;
       }
-      j = *best;
-      c->pre_queue.erase(best);
+      if (!j) {
+        if (!c->pre_queue.empty()) c->pre_cv.wait_until(lk, next);
+        continue;
+      }
+      c->pre_queue.erase(std::find(c->pre_queue.begin(), c->pre_queue.end(), j));
     }
     if (j->status.load() != QG_JOB_QUEUED) continue;
     NvtxRange nvtx("qg precompile");
