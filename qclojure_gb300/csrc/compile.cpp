@@ -390,10 +390,22 @@ void factor_global_phases(std::vector<GOp>* gops, std::vector<int>* measure_at, 
           then_x = true;
         }
         g = classify(n, g.t, 0);
+      } else if (rotations && (g.cls == U2_IMAG_ANTI || g.cls == U2_ANTIDIAG)) {
+        // [[0, a], [b, 0]] = X diag(b, a): a phase and an X (a Y gate needs no register bit then)
+        const cd a(m[2], m[3]), b(m[4], m[5]);
+        if (b != cd(0.0, 0.0)) {
+          const cd r = a / b;
+          const int t = g.t;
+          f = b;
+          g = make_phase(1ULL << t, r.real(), r.imag());
+          if (g.kind >= 0) out.push_back(g);
+          g = xgate(t);
+        }
       }
     }
+    const int target = g.t;
     if (g.kind >= 0) out.push_back(g);
-    if (then_x) out.push_back(xgate(g.t));
+    if (then_x) out.push_back(xgate(target));
     if (f != cd(1.0, 0.0)) absorb(f);
   }
   if (measured_before[gops->size()]) emit_scale();
@@ -468,8 +480,8 @@ TOp localize(const GOp& g, const int* lpos /* abs bit -> local or -1 */, int n) 
   auto split = [&](uint64_t mask, uint32_t* lm, uint64_t* gm) {
     *lm = 0;
     *gm = 0;
-    for (int b = 0; b < n; ++b) {
-      if (!(mask & (1ULL << b))) continue;
+    for (uint64_t rest = n >= 64 ? mask : mask & ((1ULL << n) - 1); rest; rest &= rest - 1) {
+      const int b = __builtin_ctzll(rest);
       if (lpos[b] >= 0) *lm |= 1u << lpos[b];
       else *gm |= 1ULL << b;
     }
@@ -581,6 +593,288 @@ void set_op_operator(TOp* t, const double m[8]) {
 
 namespace {
 
+}  // namespace
+
+// Register planning: every thread holds 2^R amplitudes
+// whose local indices differ in R "register bits". Consecutive ops whose
+// non-diagonal bits fit in R bits share one layout; the remaining register bits
+// go to the local bits the group's conditions use most, so those conditions
+// select registers at compile time. (The interpreter plans the same way with
+// R = 3; there R is a property of the kernel shape.)
+// table = true (kernels shared by the states of a sweep group): parity and
+// blockade masks are data (they differ between members, for instance between
+// QAOA graphs), so the layout must not depend on them: ops keep their order
+// (no sinking, no look-ahead) and the free register bits ignore those masks.
+namespace {
+
+bool is_permutation(const TOp& t) {
+  if (t.kind == OK_U2 && t.cls == U2_X)
+    return t.lcmask == 0 || (t.gcmask == 0 && (t.lcmask & (t.lcmask - 1)) == 0);
+  return t.kind == OK_SWAP && t.lcmask == 0 && t.gcmask == 0 && !(t.flags & 1);
+}
+
+// One op as the planner sees it: the bits it changes (they must be register bits), all bits it
+// touches, and the masks a free register bit helps with.
+struct PlanOp {
+  const TOp* op;
+  uint32_t req, all, cond;
+  bool perm;
+};
+
+LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool table, bool pair0, PermMode mode,
+                             bool emit) {
+  LayoutPlan plan;
+  std::vector<TOp>& out = plan.ops;
+  if (emit) out.reserve(in.size() * 2 + 1);
+  // Groups are formed with look-ahead: an op joins the current layout when its
+  // non-diagonal bits fit the register bits and it commutes with every op left
+  // out before it (no shared bit that either changes; tile bits are only ever
+  // diagonal, so local bits decide). Fewer layouts mean fewer trips through
+  // shared memory and fewer barriers.
+  std::vector<char> taken(in.size(), 0);
+  std::vector<int> grp;
+  size_t first = 0;
+  LayoutMap map;  // permutations since the last layout
+  bool pending = false;
+  while (first < in.size() || pending) {
+    uint32_t rb = 0, changed = 0, seen = 0;
+    if (mode != kPermRegisters) {
+      // permutations that commute with every op left out before them join the layout change
+      for (size_t j = first; j < in.size(); ++j) {
+        if (taken[j]) continue;
+        const PlanOp& q = in[j];
+        if (q.perm && (q.req & seen) == 0 && ((q.all & ~q.req) & changed) == 0) {
+          map.compose(*q.op);
+          pending = true;
+          taken[j] = 1;
+        } else {
+          changed |= q.req;
+          seen |= q.all;
+        }
+      }
+      while (first < in.size() && taken[first]) ++first;
+      if (first == in.size() && plan.layouts > 0) {  // nothing left: the last registers are written through it
+        plan.last = map.inverse();
+        break;
+      }
+      pending = false;
+      changed = seen = 0;
+    }
+    grp.clear();
+    for (size_t j = first; j < in.size(); ++j) {
+      if (taken[j]) continue;
+      const PlanOp& q = in[j];
+      const bool commutes = (q.req & seen) == 0 && ((q.all & ~q.req) & changed) == 0 &&
+                            (!q.perm || mode == kPermRegisters || (mode == kPermBoth && (q.req & ~rb) == 0));
+      if (commutes && __builtin_popcount(rb | q.req) <= R) {
+        rb |= q.req;
+        grp.push_back((int)j);
+        taken[j] = 1;
+        if (q.perm) ++plan.moves;
+      } else {
+        if (table) break;
+        changed |= q.req;
+        seen |= q.all;
+      }
+    }
+    while (first < in.size() && taken[first]) ++first;
+    ++plan.layouts;
+    plan.maps.push_back(map);
+    map = LayoutMap();
+    if (!emit) continue;
+    int uses[32] = {0};
+    for (int j : grp)
+      for (int b = 0; b < k; ++b)
+        if (in[(size_t)j].cond & (1u << b)) ++uses[b];
+    while (__builtin_popcount(rb) < R) {
+      int best = -1;
+      for (int b = k - 1; b >= 0; --b)
+        if (!(rb & (1u << b)) && (best < 0 || uses[b] > uses[best])) best = b;
+      // pair0 (complex64): a free register slot that no condition asks for takes tile
+      // bit 0, so registers j and j + 1 share one 16-byte slot pair in shared memory and
+      // a layout change moves them with one access
+      if (pair0 && uses[best] == 0 && !(rb & 1u)) best = 0;
+      rb |= 1u << best;
+    }
+    int pos[5], np = 0;
+    for (int b = 0; b < k && np < R; ++b)
+      if (rb & (1u << b)) pos[np++] = b;
+    TOp lay;
+    std::memset(&lay, 0, sizeof(lay));
+    lay.kind = OK_LAYOUT;
+    for (int q = 0; q < R; ++q) lay.dbits[q] = pos[q];
+    lay.pad1 = plan.layouts - 1;
+    out.push_back(lay);
+    auto rpos = [&](int b) {
+      for (int q = 0; q < R; ++q)
+        if (pos[q] == b) return q;
+      return -1;
+    };
+    auto reg_part = [&](uint32_t m) {
+      uint32_t r = 0;
+      for (int q = 0; q < R; ++q)
+        if (m & (1u << pos[q])) r |= 1u << q;
+      return r;
+    };
+    for (int j : grp) {
+      out.push_back(*in[(size_t)j].op);
+      TOp& t = out.back();
+      uint32_t m = 0, v = 0;
+      if (t.kind == OK_U2) {
+        t.t2 = rpos(t.t);
+        m = v = t.lcmask;
+      } else if (t.kind == OK_SWAP) {
+        const int a = rpos(t.t), b = rpos(t.t2);
+        t.dbits[0] = a < b ? a : b;
+        t.dbits[1] = a < b ? b : a;
+        m = v = t.lcmask;
+      } else if (t.kind == OK_PHASE) {
+        m = v = t.lmask;
+      } else if (t.kind == OK_COLLAPSE) {
+        m = t.lmask;
+        v = t.lval;
+      } else {  // BLOCKADE, PARITY: the mask selects the bits to count
+        m = t.lmask;
+        v = 0;
+      }
+      t.rmask = reg_part(m);
+      t.rval = reg_part(v);
+      t.tmask = m & ~rb;
+      t.tval = v & ~rb;
+    }
+  }
+  return plan;
+}
+
+}  // namespace
+
+// The cheapest of the three treatments of permutations: a layout change costs each register a
+// store, a barrier and a load, a map a second barrier, a permutation of registers its selects
+// or moves. The weights were measured (layers + QFT, ms; register ops only 50.7 at 28 qubits
+// complex128 and 30.4 at 29 qubits complex64): 10, 3, 1 gives 48.2 and 28.4; 10, 0, 3: 50.6 and
+// 28.9; 10, 6, 3: 48.5 and 28.8; 10, 10, 1: 48.9 and 29.8.
+LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool pair0, int move_cost) {
+  auto describe = [&](const TOp& t) {
+    PlanOp p{&t, 0, 0, 0, false};
+    if (t.kind == OK_U2) p.req = 1u << t.t;
+    if (t.kind == OK_SWAP) p.req = (1u << t.t) | (1u << t.t2);
+    if (!(table && (t.kind == OK_PARITY || t.kind == OK_BLOCKADE)))
+      p.cond = t.kind == OK_U2 || t.kind == OK_SWAP ? t.lcmask : t.lmask;
+    p.all = p.req | p.cond;
+    p.perm = is_permutation(t);
+    return p;
+  };
+  // Phase gates sink to the latest point they can reach: a phase commutes with
+  // every gate that does not change one of its bits, so it waits until a gate
+  // targets one of them (or the pass ends). Phases then arrive in runs, which the
+  // generator applies through shared per-mask factors (phase_run).
+  std::vector<PlanOp> in, waiting;
+  in.reserve((size_t)nops);
+  bool perms = false;
+  auto flush = [&](uint32_t bits, bool all) {
+    size_t kept = 0;
+    for (const PlanOp& p : waiting) {
+      if (all || (p.op->lmask & bits)) in.push_back(p);
+      else waiting[kept++] = p;
+    }
+    waiting.resize(kept);
+  };
+  for (int i = 0; i < nops; ++i) {
+    const TOp& t = ops[i];
+    if (t.kind == OK_LAYOUT) continue;
+    const PlanOp p = describe(t);
+    if (t.kind == OK_PHASE && !table) {
+      waiting.push_back(p);
+      continue;
+    }
+    const bool diagonal_other = t.kind == OK_BLOCKADE || t.kind == OK_PARITY || t.kind == OK_COLLAPSE;
+    flush(p.req, diagonal_other || t.kind == OK_DENSE);
+    in.push_back(p);
+    perms = perms || p.perm;
+  }
+  flush(0, true);
+  PermMode mode = kPermRegisters;  // members of a sweep share one plan in circuit order
+  if (!table && perms) {
+    int least = -1;
+    for (const PermMode m : {kPermRegisters, kPermBoth, kPermLayouts}) {
+      const LayoutPlan p = plan_layouts_mode(in, k, R, table, pair0, m, false);
+      int mapped = p.last.identity() ? 0 : 1;
+      for (const LayoutMap& x : p.maps) mapped += x.identity() ? 0 : 1;
+      const int cost = 10 * p.layouts + 3 * mapped + move_cost * p.moves;
+      if (least < 0 || cost < least) {
+        least = cost;
+        mode = m;
+      }
+    }
+  }
+  return plan_layouts_mode(in, k, R, table, pair0, mode, true);
+}
+
+namespace {
+
+// The interpreter's records of a planned pass: layouts with the map their registers are read
+// through, the tile-conditioned parts of a map before it, and a map at the end before the
+// registers are written back. A permutation of registers costs the interpreter a dispatch and
+// selects on sixteen values, about as much as a layout change.
+void plan_interpreted(const std::vector<TOp>& ops, int k, std::vector<TOp>* records) {
+  LayoutPlan plan = plan_layouts(ops.data(), (int)ops.size(), k, 3, false, false, 7);
+  auto blank = [&](int32_t kind) -> TOp& {
+    records->emplace_back();
+    TOp& t = records->back();
+    std::memset(&t, 0, sizeof(t));
+    t.kind = kind;
+    return t;
+  };
+  auto put_conds = [&](const LayoutMap& m) {
+    for (const auto& c : m.conds) {
+      TOp& x = blank(OK_MAPX);
+      x.gmask = c.first;
+      x.mc0 = c.second;
+    }
+  };
+  auto put_map = [&](TOp* lay, const LayoutMap& m) {
+    lay->mapped = m.identity() ? 0 : 1;
+    lay->mc0 = m.c0;
+    for (int b = 0; b < kMaxTileBits; ++b) lay->mcol[b] = m.col[b];
+  };
+  const TOp* last = nullptr;
+  for (size_t i = 0; i < plan.ops.size();) {
+    TOp& t = plan.ops[i];
+    if (t.kind == OK_LAYOUT) {
+      const LayoutMap& m = plan.maps[(size_t)t.pad1];
+      t.pad1 = 0;
+      for (int s = 0; s < 8; ++s)
+        t.lj[s] = ((uint32_t)(s & 1) << t.dbits[0]) | ((uint32_t)((s >> 1) & 1) << t.dbits[1]) |
+                  ((uint32_t)((s >> 2) & 1) << t.dbits[2]);
+      put_conds(m);
+      put_map(&t, m);
+      last = &t;
+    }
+    // runs of two or more phases (planning sinks them together): a header, then the phases by
+    // register mask. A single phase is cheaper as an op of its own (noisy circuits, where an
+    // operator follows every gate: 4.7 against 5.8 ms of passes).
+    size_t j = i;
+    while (j < plan.ops.size() && plan.ops[j].kind == OK_PHASE) ++j;
+    if (j <= i + 1) {
+      records->push_back(t);
+      ++i;
+      continue;
+    }
+    blank(OK_PHASES).dk = (int)(j - i);
+    for (uint32_t m = 0; m < 8; ++m)
+      for (size_t q = i; q < j; ++q)
+        if ((plan.ops[q].rmask & 7u) == m) records->push_back(plan.ops[q]);
+    i = j;
+  }
+  if (last && !plan.last.identity()) {
+    put_conds(plan.last);
+    TOp lay = *last;
+    lay.kind = OK_REMAP;
+    put_map(&lay, plan.last);
+    records->push_back(lay);
+  }
+}
+
 // Insert OK_LAYOUT ops: consecutive ops whose non-diagonal bits fit in three
 // register bits form a group; the register positions are written into the ops.
 void plan_register_groups(std::vector<TOp>& ops, int k) {
@@ -675,6 +969,7 @@ int schedule(int n, int precision, int fusion, int fuse_k, const std::vector<GOp
   prog->n = n;
   prog->steps.clear();
   prog->tops.clear();
+  prog->raw.clear();
   prog->dense.clear();
   prog->dense_tc.clear();
   prog->hbm_passes = 0;
@@ -801,6 +1096,9 @@ int schedule(int n, int precision, int fusion, int fuse_k, const std::vector<GOp
   // measurement. Overtaking changes the order of roundings, so the exact policy
   // (bit-identical to the reference's gate order) forms passes strictly in order.
   std::vector<char> done(ops.size(), 0);
+  const bool keep_raw = precision == QG_C64 || prog->arith == QG_ARITH_DOUBLE_FLOAT;  // passes that get kernels
+  prog->tops.reserve(2 * ops.size() + 16);
+  if (keep_raw) prog->raw.reserve(ops.size());
   const uint64_t all_bits = n >= 64 ? ~0ULL : ((1ULL << n) - 1);
   size_t oi = 0;
   mi = 0;
@@ -834,7 +1132,7 @@ int schedule(int n, int precision, int fusion, int fuse_k, const std::vector<GOp
       // ops before the next measurement only
       while (limit > begin && orig_index[limit - 1] >= (size_t)measure_at[mi]) --limit;
     }
-    // at most half the kernel-parameter op records: every gate may need a layout op before it
+    // at most half the kernel's op records: every gate may need a layout op before it
     const size_t max_ops = (size_t)max_ops_per_tile_pass() / 2;
     // Ops left out so far: bits they change (non-diagonal targets) and bits they
     // read or phase. A later op commutes past them when its own non-diagonal
@@ -871,12 +1169,27 @@ int schedule(int n, int precision, int fusion, int fuse_k, const std::vector<GOp
     for (int b = 0; b < 64; ++b) lpos[b] = -1;
     for (int j = 0; j < s.pass.k; ++j) lpos[s.pass.lbits[j]] = j;
     std::vector<TOp> pass_ops;
-    for (size_t j : members) pass_ops.push_back(localize(ops[j], lpos, n));
-    plan_register_groups(pass_ops, s.pass.k);
+    pass_ops.reserve(members.size());
+    bool dense = false;
+    for (size_t j : members) {
+      pass_ops.push_back(localize(ops[j], lpos, n));
+      split_coeffs(&pass_ops.back());
+      dense = dense || pass_ops.back().kind == OK_DENSE;
+    }
+    if (keep_raw) {
+      s.raw_begin = (int64_t)prog->raw.size();
+      prog->raw.insert(prog->raw.end(), pass_ops.begin(), pass_ops.end());
+      s.raw_end = (int64_t)prog->raw.size();
+    }
+    // The exact policy keeps the circuit's order of roundings and sweeps one pass structure
+    // for all members; the others gather commuting ops under fewer layouts and move X, CNOT
+    // and SWAP into the layout changes.
     s.pass.op_begin = (int64_t)prog->tops.size();
-    for (TOp& t : pass_ops) {
-      split_coeffs(&t);
-      prog->tops.push_back(t);
+    if (reorder && !dense) {
+      plan_interpreted(pass_ops, s.pass.k, &prog->tops);
+    } else {
+      plan_register_groups(pass_ops, s.pass.k);
+      prog->tops.insert(prog->tops.end(), pass_ops.begin(), pass_ops.end());
     }
     s.pass.op_end = (int64_t)prog->tops.size();
     prog->steps.push_back(s);

@@ -10,9 +10,8 @@
 // The draws here depend only on (seed, shot, site), never on the state, so every
 // trajectory is the same program with different Kraus matrices: the circuit with one
 // QG_OP_KRAUS per noise site is compiled once into tiled passes, and a batch of
-// trajectories runs as one launch per pass over all its states, each state reading its
-// own op records (the template's records with the chosen operators patched in); shots
-// with equal choices share one state. The
+// trajectories runs as one launch per pass over all its states, which share the op records and
+// look the chosen operators up at the noise sites; shots with equal choices share one state. The
 // renormalisations are deferred to the end of the shot (every operator is linear, so
 // the final direction is the same) and done by the kernel that also samples the shot.
 // States of fewer than 5 qubits run padded with idle low qubits, which stay |0>.
@@ -286,13 +285,7 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
   }
   const size_t S = sites.size();
   std::vector<unsigned char> variants(rec * 4 * S);
-  std::vector<int32_t> site_of((size_t)R, -1), pass_ops((size_t)R), site_chan(S);
-  std::vector<int64_t> pass_off((size_t)R);
-  for (size_t p = 0; p < P; ++p)
-    for (int64_t j = rec_off[p]; j < rec_off[p + 1]; ++j) {
-      pass_off[(size_t)j] = rec_off[p];
-      pass_ops[(size_t)j] = (int32_t)nops[p];
-    }
+  std::vector<int32_t> site_chan(S);
   for (size_t s = 0; s < S; ++s) {
     const Channel& ch = chans[sites[s].entry];
     const PassDesc& pd = prog.steps[pass_steps[sites[s].pass]].pass;
@@ -303,7 +296,7 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
       set_op_operator(&t, ch.applied[v].data());
       encode_kops(precision, arith, &t, 1, variants.data() + rec * (4 * s + v));
     }
-    site_of[(size_t)(rec_off[sites[s].pass] + sites[s].at)] = (int32_t)s;
+    encode_site(tmpl.data() + rec * (size_t)(rec_off[sites[s].pass] + sites[s].at), (int)s);
     site_chan[s] = sites[s].entry;
   }
   std::vector<NoiseChannel> dch(chans.size());
@@ -311,19 +304,17 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
 
   // Batches of shots. Shots whose Kraus choices coincide end in the same state, so each
   // batch simulates only its distinct choice vectors and samples every shot from its
-  // vector's state (with the shot's own draw). Batch size: device memory for one state and
-  // its op records per shot.
+  // vector's state (with the shot's own draw). Batch size: device memory for one state per shot.
   const int dev = ctx_device_of(ctx);
   cudaSetDevice(dev);
   const size_t state_bytes = (precision == QG_C64 ? 8ull : 16ull) << n_run;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return fail(QG_ERR_DEVICE, "cudaMemGetInfo failed");
   const size_t budget = std::min(free_b / 2, (size_t)64 << 30);
-  const size_t per = state_bytes + rec * (size_t)R + S + 128;
+  const size_t per = state_bytes + S + 128;
   if (budget < per) return fail(QG_ERR_OOM, "one trajectory does not fit the device memory budget");
   uint64_t B = std::min<uint64_t>(shots ? shots : 1, 65536);
   B = std::min<uint64_t>(B, std::max<size_t>(1, budget / per));
-  B = std::min<uint64_t>(B, std::max<size_t>(1, ((size_t)4 << 30) / std::max<size_t>(1, rec * (size_t)R)));
 
   cudaStream_t st;
   if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return fail(QG_ERR_DEVICE, "stream");
@@ -374,9 +365,6 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
   const size_t o_chan = put(dch.data(), sizeof(NoiseChannel) * dch.size());
   const size_t o_site_chan = put(site_chan.data(), sizeof(int32_t) * S);
   const size_t o_tmpl = put(tmpl.data(), tmpl.size()), o_var = put(variants.data(), variants.size());
-  const size_t o_site = put(site_of.data(), sizeof(int32_t) * site_of.size());
-  const size_t o_poff = put(pass_off.data(), sizeof(int64_t) * pass_off.size());
-  const size_t o_pops = put(pass_ops.data(), sizeof(int32_t) * pass_ops.size());
   const size_t o_fac = put(ro.factor.data(), sizeof(double) * ro.factor.size());
   unsigned char *d_tab = nullptr, *d_choices = nullptr;
   struct Hash {
@@ -393,15 +381,7 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
             take(sizeof(int32_t) * B, "alloc state shots", (void**)&d_reps) &&
             take(sizeof(int32_t), "alloc check", (void**)&d_differ) &&
             cuda_check(cudaMemcpyAsync(d_tab, tables.data(), tables.size(), cudaMemcpyHostToDevice, st), "H2D tables");
-  NoiseRecords nr;
-  nr.tmpl = d_tab + o_tmpl;
-  nr.variants = d_tab + o_var;
-  nr.site_of = reinterpret_cast<const int32_t*>(d_tab + o_site);
-  nr.pass_off = reinterpret_cast<const int64_t*>(d_tab + o_poff);
-  nr.pass_ops = reinterpret_cast<const int32_t*>(d_tab + o_pops);
-  nr.sites = (int)S;
-  nr.pieces = (int)(rec / 16);
-  nr.records = R;
+  const NoiseSites ns{d_choices, d_reps, d_tab + o_var, (int)S};
   const uint64_t N = 1ULL << n;
   std::vector<Hash> h_hash(B);
   std::vector<uint64_t> h_out(B);
@@ -441,7 +421,7 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
       }
       state_of[m] = slots[q];
     }
-    void *slab = nullptr, *d_kops = nullptr;
+    void* slab = nullptr;
     void** d_ptrs = nullptr;
     double* d_norm = nullptr;
     uint64_t U = 0;
@@ -450,7 +430,6 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
       drop_from(fixed);
       int32_t differ = 0;
       ok = take(state_bytes * U, "alloc trajectories", &slab) &&
-           take(rec * (size_t)R * U, "alloc op records", &d_kops) &&
            take(sizeof(void*) * U, "alloc pointers", (void**)&d_ptrs) &&
            take(sizeof(double) * U, "alloc norms", (void**)&d_norm);
       if (!ok) break;
@@ -462,8 +441,7 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
            cuda_check(cudaMemcpyAsync(d_reps, reps.data(), sizeof(int32_t) * U, cudaMemcpyHostToDevice, st),
                       "H2D state shots") &&
            cuda_check(cudaMemsetAsync(d_differ, 0, sizeof(int32_t), st), "clear check") &&
-           cuda_check(launch_noise_records(nr, d_choices, d_state_of, (int)nb, d_reps, (int)U, d_kops, d_differ, st),
-                      "op records") &&
+           cuda_check(launch_noise_verify(d_choices, (int)S, d_state_of, (int)nb, d_reps, d_differ, st), "check") &&
            cuda_check(cudaMemcpyAsync(&differ, d_differ, sizeof(differ), cudaMemcpyDeviceToHost, st), "D2H check") &&
            cuda_check(cudaStreamSynchronize(st), "sync");
       if (!ok || !differ || attempt) break;
@@ -486,8 +464,7 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
       pd.op_begin = 0;
       pd.op_end = nops[p];
       ok = cuda_check(launch_tile_pass(precision, arith, tile_pass_io(prog, pass_steps[p]), n_run, pd, d_ptrs, (int)U,
-                                       (unsigned char*)d_kops + rec * (size_t)(rec_off[p] * (int64_t)U), nops[p],
-                                       nullptr, st),
+                                       d_tab + o_tmpl + rec * (size_t)rec_off[p], 0, nullptr, st, &ns),
                       "trajectory pass");
     }
     ok = ok && cuda_check(launch_traj_normalise(precision, d_ptrs, (int)U, n_run, d_norm, st), "renormalise") &&

@@ -1,12 +1,12 @@
-// Kernels of the noisy trajectories (noisy.cpp): the draws of every shot, the op records of
-// the distinct trajectories, readout noise and the collected final states.
+// Kernels of the noisy trajectories (noisy.cpp): the draws of every shot, readout noise and
+// the collected final states.
 //
 // The host did this work before: 20,000 shots of the 300-gate recipe at 10 qubits (0.1 % / 1 %
 // depolarizing, about 8,000 distinct states) drew 6 million Kraus choices on the host cores,
 // wrote 440 MB of op records into pinned memory allocated for the call and copied them over,
 // about 40 of 58 ms. Here a shot's choices cost one Philox draw per site on the device, shots
 // are grouped by a 128-bit sum of hashes that is checked against the choices themselves, and
-// the records are expanded in HBM from the template (one write of each record's 96 bytes).
+// the tile interpreter looks each state's operators up by its choices (NoiseSites).
 #include <algorithm>
 
 #include "qgpu_internal.h"
@@ -67,30 +67,6 @@ __global__ void __launch_bounds__(256) k_noise_verify(const uint8_t* __restrict_
   if (bad) *differ = 1;
 }
 
-// One thread per 16 bytes of a record: pass-major, the records of a state side by side within
-// a pass. Record j of the template belongs to pass pass_of[j]; site_of[j] is its noise site
-// (-1: the template's record).
-__global__ void __launch_bounds__(256) k_noise_records(const uint4* __restrict__ tmpl, const uint4* __restrict__ variants,
-                                                       const int32_t* __restrict__ site_of,
-                                                       const int64_t* __restrict__ pass_off,  // per record: its pass's first record
-                                                       const int32_t* __restrict__ pass_ops,  // per record: records of its pass
-                                                       const uint8_t* __restrict__ choices, int sites,
-                                                       const int32_t* __restrict__ reps, int states, int64_t records,
-                                                       int pieces, uint4* __restrict__ out) {
-  const int64_t row = records * pieces;
-  for (int64_t i = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < row; i += (int64_t)gridDim.y * blockDim.x) {
-    const int64_t j = i / pieces;
-    const int piece = (int)(i - j * pieces), s = site_of[j];
-    const int64_t off = pass_off[j], ops = pass_ops[j];
-    for (int u = (int)blockIdx.x; u < states; u += (int)gridDim.x) {
-      uint4 v;
-      if (s < 0) v = tmpl[i];
-      else v = variants[((int64_t)s * 4 + choices[(size_t)reps[u] * sites + s]) * pieces + piece];
-      out[(off * states + (int64_t)u * ops + (j - off)) * pieces + piece] = v;
-    }
-  }
-}
-
 // One thread per shot: readout noise qubit by qubit (noise.clj:107-160); factors[source * n +
 // target], NaN where none is given (null: no correlations).
 __global__ void __launch_bounds__(256) k_noise_readout(uint64_t* __restrict__ outcomes, int shots, int n, uint64_t seed,
@@ -141,19 +117,11 @@ cudaError_t launch_noise_choices(const NoiseChannel* d_chans, const int32_t* d_s
   return cudaGetLastError();
 }
 
-cudaError_t launch_noise_records(const NoiseRecords& r, const uint8_t* d_choices, const int32_t* d_state_of, int shots,
-                                 const int32_t* d_reps, int states, void* d_out, int32_t* d_differ, cudaStream_t st) {
-  if (r.sites > 0)
-    k_noise_verify<<<(unsigned)(shots + 7) / 8, 256, 0, st>>>(d_choices, r.sites, shots, d_state_of, d_reps, d_differ);
-  const int64_t row = r.records * r.pieces;
-  if (row > 0) {
-    const unsigned gy = (unsigned)std::min<int64_t>((row + 255) / 256, 65535);
-    const unsigned gx = (unsigned)std::min<int64_t>(states, std::max<int64_t>(1, 152 * 16 / gy));
-    k_noise_records<<<dim3(gx, gy), 256, 0, st>>>((const uint4*)r.tmpl, (const uint4*)r.variants, r.site_of, r.pass_off,
-                                                  r.pass_ops, d_choices, r.sites, d_reps, states, r.records, r.pieces,
-                                                  (uint4*)d_out);
-  }
-  count_launch(2);
+cudaError_t launch_noise_verify(const uint8_t* d_choices, int sites, const int32_t* d_state_of, int shots,
+                                const int32_t* d_reps, int32_t* d_differ, cudaStream_t st) {
+  if (sites < 1) return cudaSuccess;
+  k_noise_verify<<<(unsigned)(shots + 7) / 8, 256, 0, st>>>(d_choices, sites, shots, d_state_of, d_reps, d_differ);
+  count_launch(1);
   return cudaGetLastError();
 }
 

@@ -103,289 +103,6 @@ inline bool hi_lo_nonzero(const TOp& t, int q) { return t.mf[8 + q] != 0.0f; }
 // ---------------------------------------------------------------------------
 // Source generation for one pass
 // ---------------------------------------------------------------------------
-// Register planning for the generated kernels: every thread holds 2^R amplitudes
-// whose local indices differ in R "register bits". Consecutive ops whose
-// non-diagonal bits fit in R bits share one layout; the remaining register bits
-// go to the local bits the group's conditions use most, so those conditions
-// select registers at compile time. (The interpreter plans the same way with
-// R = 3 in compile.cpp; here R is a property of the kernel shape.)
-// table = true (kernels shared by the states of a sweep group): parity and
-// blockade masks are data (they differ between members, for instance between
-// QAOA graphs), so the layout must not depend on them: ops keep their order
-// (no sinking, no look-ahead) and the free register bits ignore those masks.
-//
-// Index permutations. An X (no control, one local control, or tile controls), CNOT or SWAP
-// maps local indices by an affine map over GF(2), i -> M i ^ c. It needs no register bit and
-// no data movement of its own: every layout change already sends each register through
-// shared memory, so the permutations gathered since the last one only change the address a
-// register is read from (or, at the end of the pass, written to). LayoutMap holds that map:
-// column b is the image of local bit b, c0 the constant part, conds the parts that hold on
-// tiles whose index has all bits of a mask.
-struct LayoutMap {
-  uint16_t col[kMaxTileBits];
-  uint16_t c0 = 0;
-  std::vector<std::pair<uint64_t, uint16_t>> conds;
-  LayoutMap() {
-    for (int b = 0; b < kMaxTileBits; ++b) col[b] = (uint16_t)(1u << b);
-  }
-  bool identity() const {
-    for (int b = 0; b < kMaxTileBits; ++b)
-      if (col[b] != (1u << b)) return false;
-    return c0 == 0 && conds.empty();
-  }
-  uint16_t of(uint32_t l) const {  // the linear part
-    uint16_t r = 0;
-    for (int b = 0; b < kMaxTileBits; ++b)
-      if ((l >> b) & 1) r ^= col[b];
-    return r;
-  }
-  // this map after the permutation op (applied first): A -> A o op
-  void compose(const TOp& t) {
-    if (t.kind == OK_SWAP) {
-      std::swap(col[t.t], col[t.t2]);
-    } else if (t.lcmask) {
-      col[__builtin_ctz(t.lcmask)] ^= col[t.t];
-    } else if (t.gcmask) {
-      for (auto it = conds.begin(); it != conds.end(); ++it)
-        if (it->first == t.gcmask) {
-          it->second ^= col[t.t];
-          if (!it->second) conds.erase(it);
-          return;
-        }
-      conds.push_back({t.gcmask, col[t.t]});
-    } else {
-      c0 ^= col[t.t];
-    }
-  }
-  LayoutMap inverse() const {  // M^-1 by elimination; the constants go through it
-    uint32_t rows[kMaxTileBits], inv[kMaxTileBits];
-    for (int r = 0; r < kMaxTileBits; ++r) {
-      rows[r] = 0;
-      inv[r] = 1u << r;
-      for (int b = 0; b < kMaxTileBits; ++b) rows[r] |= (uint32_t)((col[b] >> r) & 1) << b;
-    }
-    for (int p = 0; p < kMaxTileBits; ++p) {
-      int r = p;
-      while (!((rows[r] >> p) & 1)) ++r;  // M is invertible: a product of invertible maps
-      std::swap(rows[r], rows[p]);
-      std::swap(inv[r], inv[p]);
-      for (int q = 0; q < kMaxTileBits; ++q)
-        if (q != p && ((rows[q] >> p) & 1)) {
-          rows[q] ^= rows[p];
-          inv[q] ^= inv[p];
-        }
-    }
-    LayoutMap m;
-    for (int b = 0; b < kMaxTileBits; ++b) {
-      m.col[b] = 0;
-      for (int r = 0; r < kMaxTileBits; ++r) m.col[b] |= (uint16_t)(((inv[r] >> b) & 1) << r);
-    }
-    m.c0 = m.of(c0);
-    for (const auto& c : conds) m.conds.push_back({c.first, m.of(c.second)});
-    return m;
-  }
-};
-
-bool is_permutation(const TOp& t) {
-  if (t.kind == OK_U2 && t.cls == U2_X)
-    return t.lcmask == 0 || (t.gcmask == 0 && (t.lcmask & (t.lcmask - 1)) == 0);
-  return t.kind == OK_SWAP && t.lcmask == 0 && t.gcmask == 0 && !(t.flags & 1);
-}
-
-// How a plan treats permutations: as register ops (their target is a register bit), in
-// layout changes only, or in layout changes unless a group's register bits hold the target
-// already.
-enum PermMode { kPermRegisters, kPermLayouts, kPermBoth };
-
-struct LayoutPlan {
-  std::vector<TOp> ops;          // an OK_LAYOUT's pad1 is its map's index
-  std::vector<LayoutMap> maps;   // where each layout's registers are read from
-  LayoutMap last;                // where the last layout's registers are written to
-  int layouts = 0, moves = 0;    // moves: permutations applied to registers
-};
-
-LayoutPlan plan_layouts_mode(const TOp* ops, int nops, int k, int R, bool table, bool pair0, PermMode mode) {
-  auto required = [](const TOp& t) -> uint32_t {
-    if (t.kind == OK_U2) return 1u << t.t;
-    if (t.kind == OK_SWAP) return (1u << t.t) | (1u << t.t2);
-    return 0u;
-  };
-  auto data_mask = [&](const TOp& t) { return table && (t.kind == OK_PARITY || t.kind == OK_BLOCKADE); };
-  // Phase gates sink to the latest point they can reach: a phase commutes with
-  // every gate that does not change one of its bits, so it waits until a gate
-  // targets one of them (or the pass ends). Phases then arrive in runs, which the
-  // generator applies through shared per-mask factors (phase_run).
-  std::vector<TOp> in;
-  {
-    std::vector<TOp> pending;
-    auto flush = [&](uint32_t bits, bool all) {
-      std::vector<TOp> keep;
-      for (const TOp& p : pending) {
-        if (all || (p.lmask & bits)) in.push_back(p);
-        else keep.push_back(p);
-      }
-      pending.swap(keep);
-    };
-    for (int i = 0; i < nops; ++i) {
-      const TOp& t = ops[i];
-      if (t.kind == OK_LAYOUT) continue;
-      if (t.kind == OK_PHASE && !table) {
-        pending.push_back(t);
-        continue;
-      }
-      const bool diagonal_other = t.kind == OK_BLOCKADE || t.kind == OK_PARITY || t.kind == OK_COLLAPSE;
-      flush(required(t), diagonal_other || t.kind == OK_DENSE);
-      in.push_back(t);
-    }
-    flush(0, true);
-  }
-  LayoutPlan plan;
-  std::vector<TOp>& out = plan.ops;
-  auto cond_bits = [&](const TOp& t) -> uint32_t {
-    if (data_mask(t)) return 0u;
-    return t.kind == OK_U2 || t.kind == OK_SWAP ? t.lcmask : t.lmask;
-  };
-  // Groups are formed with look-ahead: an op joins the current layout when its
-  // non-diagonal bits fit the register bits and it commutes with every op left
-  // out before it (no shared bit that either changes; tile bits are only ever
-  // diagonal, so local bits decide). Fewer layouts mean fewer trips through
-  // shared memory and fewer barriers.
-  std::vector<char> taken(in.size(), 0);
-  size_t first = 0;
-  LayoutMap map;  // permutations since the last layout
-  bool pending = false;
-  while (first < in.size() || pending) {
-    uint32_t rb = 0, changed = 0, seen = 0;
-    if (mode != kPermRegisters) {
-      // permutations that commute with every op left out before them join the layout change
-      for (size_t j = first; j < in.size(); ++j) {
-        if (taken[j]) continue;
-        const uint32_t req = required(in[j]), tb = req | cond_bits(in[j]);
-        if (is_permutation(in[j]) && (req & seen) == 0 && ((tb & ~req) & changed) == 0) {
-          map.compose(in[j]);
-          pending = true;
-          taken[j] = 1;
-        } else {
-          changed |= req;
-          seen |= tb;
-        }
-      }
-      while (first < in.size() && taken[first]) ++first;
-      if (first == in.size() && plan.layouts > 0) {  // nothing left: the last registers are written through it
-        plan.last = map.inverse();
-        break;
-      }
-      pending = false;
-      changed = seen = 0;
-    }
-    std::vector<TOp> grp;
-    for (size_t j = first; j < in.size(); ++j) {
-      if (taken[j]) continue;
-      const uint32_t req = required(in[j]), tb = req | cond_bits(in[j]);
-      const bool perm = mode != kPermRegisters && is_permutation(in[j]);
-      const bool commutes = (req & seen) == 0 && ((tb & ~req) & changed) == 0 &&
-                            (!perm || (mode == kPermBoth && (req & ~rb) == 0));
-      if (commutes && __builtin_popcount(rb | req) <= R) {
-        rb |= req;
-        grp.push_back(in[j]);
-        taken[j] = 1;
-      } else {
-        if (table) break;
-        changed |= req;
-        seen |= tb;
-      }
-    }
-    while (first < in.size() && taken[first]) ++first;
-    int uses[32] = {0};
-    for (const TOp& t : grp) {
-      const uint32_t cm = cond_bits(t);
-      for (int b = 0; b < k; ++b)
-        if (cm & (1u << b)) ++uses[b];
-    }
-    while (__builtin_popcount(rb) < R) {
-      int best = -1;
-      for (int b = k - 1; b >= 0; --b)
-        if (!(rb & (1u << b)) && (best < 0 || uses[b] > uses[best])) best = b;
-      // pair0 (complex64): a free register slot that no condition asks for takes tile
-      // bit 0, so registers j and j + 1 share one 16-byte slot pair in shared memory and
-      // a layout change moves them with one access
-      if (pair0 && uses[best] == 0 && !(rb & 1u)) best = 0;
-      rb |= 1u << best;
-    }
-    int pos[5], np = 0;
-    for (int b = 0; b < k && np < R; ++b)
-      if (rb & (1u << b)) pos[np++] = b;
-    TOp lay;
-    std::memset(&lay, 0, sizeof(lay));
-    lay.kind = OK_LAYOUT;
-    for (int q = 0; q < R; ++q) lay.dbits[q] = pos[q];
-    lay.pad1 = (int)plan.maps.size();
-    plan.maps.push_back(map);
-    map = LayoutMap();
-    ++plan.layouts;
-    out.push_back(lay);
-    auto rpos = [&](int b) {
-      for (int q = 0; q < R; ++q)
-        if (pos[q] == b) return q;
-      return -1;
-    };
-    auto reg_part = [&](uint32_t m) {
-      uint32_t r = 0;
-      for (int q = 0; q < R; ++q)
-        if (m & (1u << pos[q])) r |= 1u << q;
-      return r;
-    };
-    for (const TOp& t0 : grp) {
-      TOp t = t0;
-      uint32_t m = 0, v = 0;
-      if (t.kind == OK_U2) {
-        t.t2 = rpos(t.t);
-        m = v = t.lcmask;
-      } else if (t.kind == OK_SWAP) {
-        const int a = rpos(t.t), b = rpos(t.t2);
-        t.dbits[0] = a < b ? a : b;
-        t.dbits[1] = a < b ? b : a;
-        m = v = t.lcmask;
-      } else if (t.kind == OK_PHASE) {
-        m = v = t.lmask;
-      } else if (t.kind == OK_COLLAPSE) {
-        m = t.lmask;
-        v = t.lval;
-      } else {  // BLOCKADE, PARITY: the mask selects the bits to count
-        m = t.lmask;
-        v = 0;
-      }
-      t.rmask = reg_part(m);
-      t.rval = reg_part(v);
-      t.tmask = m & ~rb;
-      t.tval = v & ~rb;
-      if (is_permutation(t)) ++plan.moves;
-      out.push_back(t);
-    }
-  }
-  return plan;
-}
-
-// The cheapest of the three treatments of permutations: a layout change costs each register a
-// store, a barrier and a load, a map a second barrier, a permutation of registers its selects
-// or moves. The weights were measured (layers + QFT, ms; register ops only 50.7 at 28 qubits
-// complex128 and 30.4 at 29 qubits complex64): 10, 3, 1 gives 48.2 and 28.4; 10, 0, 3: 50.6 and
-// 28.9; 10, 6, 3: 48.5 and 28.8; 10, 10, 1: 48.9 and 29.8.
-LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table = false, bool pair0 = false) {
-  LayoutPlan best = plan_layouts_mode(ops, nops, k, R, table, pair0, kPermRegisters);
-  if (table) return best;  // members of a sweep share one plan in circuit order
-  auto cost = [](const LayoutPlan& p) {
-    int mapped = p.last.identity() ? 0 : 1;
-    for (const LayoutMap& m : p.maps) mapped += m.identity() ? 0 : 1;
-    return 10 * p.layouts + 3 * mapped + p.moves;
-  };
-  for (const PermMode m : {kPermBoth, kPermLayouts}) {
-    LayoutPlan p = plan_layouts_mode(ops, nops, k, R, table, pair0, m);
-    if (cost(p) < cost(best)) best = std::move(p);
-  }
-  return best;
-}
-
 // A real or RX-shaped 2x2 whose diagonal is (1, +-1) (a rotation with its
 // diagonal factored out): 1 = [[1, b], [c, 1]], 2 = [[1, b], [c, -1]], else 0.
 int unit_diagonal(const TOp& t) {
@@ -452,7 +169,7 @@ class PassGen {
       if (ops[i].kind == OK_DENSE) unsupported_ = true;
       if (table && (ops[i].kind == OK_BLOCKADE || ops[i].kind == OK_COLLAPSE)) unsupported_ = true;
     }
-    if (!unsupported_) plan_ = plan_layouts(tagged.data(), nops, pd.k, sh_.rbits, table, !df_);
+    if (!unsupported_) plan_ = plan_layouts(tagged.data(), nops, pd.k, sh_.rbits, table, !df_, 1);
     // pairs handed over by the previous pass may carry unnormalised operations
     if (io & kTileInPairs) carry_ = kRenormEvery / 2 - 1;
     ops_ = plan_.ops.data();
@@ -1582,8 +1299,9 @@ bool generate_units(const Program& prog, int prec, std::vector<Unit>* units, std
     const Shape sh = shape_of(prog, prec);
     // a tile of at least 2^10 amplitudes, a warp or more of threads
     if (st.kind != Step::TILE_PASS || st.pass.k < 10 || st.pass.k - sh.rbits < 5) continue;
-    const TOp* ops = prog.tops.data() + st.pass.op_begin;
-    const int nops = (int)(st.pass.op_end - st.pass.op_begin);
+    // sweeps read their coefficient rows in the order of the interpreter's records
+    const TOp* ops = table ? prog.tops.data() + st.pass.op_begin : prog.raw.data() + st.raw_begin;
+    const int nops = (int)(table ? st.pass.op_end - st.pass.op_begin : st.raw_end - st.raw_begin);
     std::ostringstream o;
     PassGen g(o, st.pass, ops, nops, prec, tile_pass_io(prog, i), table, sh);
     if (!g.supported()) continue;
@@ -1601,7 +1319,7 @@ bool generate_units(const Program& prog, int prec, std::vector<Unit>* units, std
   // one unit per host thread; passes dealt largest first to the smallest unit (the
   // compile time of a pass grows faster than its source, so big passes go alone)
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t nunits = std::min<size_t>(pieces.size(), std::min(hw, 32u));
+  const size_t nunits = std::min<size_t>(pieces.size(), 2 * std::min(hw, 32u));
   units->assign(nunits, Unit());
   std::vector<size_t> load(nunits, 0), order(pieces.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
@@ -1862,7 +1580,7 @@ std::shared_ptr<const PassKernels> level_kernels_for(const std::vector<const Pro
   }
   // units: levels dealt largest first, one unit per host thread
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t nunits = std::min<size_t>(pieces.size(), std::min(hw, 32u));
+  const size_t nunits = std::min<size_t>(pieces.size(), 2 * std::min(hw, 32u));
   std::vector<Unit> units(nunits);
   std::vector<size_t> load(nunits, 0), order(pieces.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
@@ -2022,7 +1740,7 @@ void pass_coefficients(const Program& prog, size_t step, int prec, float* out) {
   std::vector<TOp> tagged(ops, ops + nops);
   for (int i = 0; i < nops; ++i) tagged[i].pad1 = i;
   const std::vector<TOp> plan =
-      plan_layouts(tagged.data(), nops, pd.k, shape_of(prog, prec).rbits, true, prec == QG_C64).ops;
+      plan_layouts(tagged.data(), nops, pd.k, shape_of(prog, prec).rbits, true, prec == QG_C64, 1).ops;
   const int ns = 1 << shape_of(prog, prec).rbits;  // registers per thread
   auto put = [&](float* at, std::complex<double> v) {
     if (prec == QG_C128) {

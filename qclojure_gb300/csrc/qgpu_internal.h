@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -42,7 +43,10 @@ enum OpKind : int32_t {
   OK_COLLAPSE = 5,  // amp = ((idx & mask) == val) ? amp * scale : 0
   OK_DENSE = 6,     // dense 2^dk x 2^dk block on bits dbits[0..dk) (dbits[0] = least significant)
   OK_LAYOUT = 7,    // tiled executor only: registers hold the local bits dbits[0..3) from here on
-  OK_NONE = 8       // tiled executor only: nothing (a noise site whose operator is the identity)
+  OK_NONE = 8,      // tiled executor only: nothing (a noise site whose operator is the identity)
+  OK_MAPX = 9,      // tiled executor only: a tile-conditioned part of the next layout's map
+  OK_REMAP = 10,    // tiled executor only: the registers are written back through a map
+  OK_PHASES = 11    // tiled executor only: the next dk phases form one run, by register mask
 };
 
 // Matrix classes of OK_U2 (picked on the host from exact zero / unit entries).
@@ -108,6 +112,12 @@ struct TOp {
   // thread bits (tmask/tval), so each thread tests one word per op.
   uint32_t rmask, rval, tmask, tval;
   uint32_t lj[8];    // OK_LAYOUT: local offset of register slot j
+  // OK_LAYOUT, OK_REMAP: the map registers are read or written through (LayoutMap's columns
+  // and constant; mapped = 0: the identity). OK_MAPX: mc0 joins the next one's constant on
+  // tiles whose index has all bits of gmask.
+  uint16_t mcol[13];
+  uint16_t mc0;
+  int32_t mapped;
 };
 
 constexpr int kMaxTileBits = 13;     // 2^13 amplitudes per tile at most
@@ -125,18 +135,112 @@ struct PassDesc {
   int64_t op_begin, op_end;  // range in the TOp array
 };
 
+// ---------------------------------------------------------------------------
+// Register layouts of a pass (compile.cpp).
+//
+// Index permutations. An X (no control, one local control, or tile controls), CNOT or SWAP
+// maps local indices by an affine map over GF(2), i -> M i ^ c. It needs no register bit and
+// no data movement of its own: every layout change already sends each register through
+// shared memory, so the permutations gathered since the last one only change the address a
+// register is read from (or, at the end of the pass, written to). LayoutMap holds that map:
+// column b is the image of local bit b, c0 the constant part, conds the parts that hold on
+// tiles whose index has all bits of a mask.
+struct LayoutMap {
+  uint16_t col[kMaxTileBits];
+  uint16_t c0 = 0;
+  std::vector<std::pair<uint64_t, uint16_t>> conds;
+  LayoutMap() {
+    for (int b = 0; b < kMaxTileBits; ++b) col[b] = (uint16_t)(1u << b);
+  }
+  bool identity() const {
+    for (int b = 0; b < kMaxTileBits; ++b)
+      if (col[b] != (1u << b)) return false;
+    return c0 == 0 && conds.empty();
+  }
+  uint16_t of(uint32_t l) const {  // the linear part
+    uint16_t r = 0;
+    for (int b = 0; b < kMaxTileBits; ++b)
+      if ((l >> b) & 1) r ^= col[b];
+    return r;
+  }
+  // this map after the permutation op (applied first): A -> A o op
+  void compose(const TOp& t) {
+    if (t.kind == OK_SWAP) {
+      std::swap(col[t.t], col[t.t2]);
+    } else if (t.lcmask) {
+      col[__builtin_ctz(t.lcmask)] ^= col[t.t];
+    } else if (t.gcmask) {
+      for (auto it = conds.begin(); it != conds.end(); ++it)
+        if (it->first == t.gcmask) {
+          it->second ^= col[t.t];
+          if (!it->second) conds.erase(it);
+          return;
+        }
+      conds.push_back({t.gcmask, col[t.t]});
+    } else {
+      c0 ^= col[t.t];
+    }
+  }
+  LayoutMap inverse() const {  // M^-1 by elimination; the constants go through it
+    uint32_t rows[kMaxTileBits], inv[kMaxTileBits];
+    for (int r = 0; r < kMaxTileBits; ++r) {
+      rows[r] = 0;
+      inv[r] = 1u << r;
+      for (int b = 0; b < kMaxTileBits; ++b) rows[r] |= (uint32_t)((col[b] >> r) & 1) << b;
+    }
+    for (int p = 0; p < kMaxTileBits; ++p) {
+      int r = p;
+      while (!((rows[r] >> p) & 1)) ++r;  // M is invertible: a product of invertible maps
+      std::swap(rows[r], rows[p]);
+      std::swap(inv[r], inv[p]);
+      for (int q = 0; q < kMaxTileBits; ++q)
+        if (q != p && ((rows[q] >> p) & 1)) {
+          rows[q] ^= rows[p];
+          inv[q] ^= inv[p];
+        }
+    }
+    LayoutMap m;
+    for (int b = 0; b < kMaxTileBits; ++b) {
+      m.col[b] = 0;
+      for (int r = 0; r < kMaxTileBits; ++r) m.col[b] |= (uint16_t)(((inv[r] >> b) & 1) << r);
+    }
+    m.c0 = m.of(c0);
+    for (const auto& c : conds) m.conds.push_back({c.first, m.of(c.second)});
+    return m;
+  }
+};
+
+// How a plan treats permutations: as register ops (their target is a register bit), in
+// layout changes only, or in layout changes unless a group's register bits hold the target
+// already.
+enum PermMode { kPermRegisters, kPermLayouts, kPermBoth };
+
+struct LayoutPlan {
+  std::vector<TOp> ops;          // an OK_LAYOUT's pad1 is its map's index
+  std::vector<LayoutMap> maps;   // where each layout's registers are read from
+  LayoutMap last;                // where the last layout's registers are written to
+  int layouts = 0, moves = 0;    // moves: permutations applied to registers
+};
+
+// Plans a pass's ops (k local bits, R register bits). table: members of a sweep share the plan,
+// so it keeps circuit order and ignores parity masks; pair0: complex64 kernels pair registers on
+// tile bit 0; move_cost: of a permutation of registers, against 10 for a layout change.
+LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool pair0, int move_cost);
+
 // A compiled step sequence.
 struct Step {
   enum Kind { PLAIN_OP, TILE_PASS, MEASURE } kind;
   GOp op;                  // PLAIN_OP
   PassDesc pass;           // TILE_PASS
+  int64_t raw_begin = 0, raw_end = 0;  // TILE_PASS: its ops in Program::raw
   std::vector<int> mqubits;// MEASURE (qubit indices, outcome bit i <-> mqubits[i])
 };
 
 struct Program {
   int n = 0;
   std::vector<Step> steps;
-  std::vector<TOp> tops;             // all tile ops, referenced by PassDesc ranges
+  std::vector<TOp> tops;             // all tile ops, planned for the interpreter; PassDesc ranges
+  std::vector<TOp> raw;              // the passes' ops before planning (the pass kernels plan their own)
   std::vector<double> dense;         // dense block matrices (re, im interleaved)
   std::vector<float> dense_tc;       // tensor-core blocks: TF32 hi / lo operands (dense_tc_prepare)
   int hbm_passes = 0;
@@ -176,9 +280,20 @@ cudaError_t launch_plain_op(void* s, int precision, int n, const GOp& op, cudaSt
 // (re.hi, re.lo, im.hi, im.lo) written by the previous pass, bit 1 = leave it as
 // float pairs for the next pass; without the bit the state is IEEE doubles.
 constexpr int kTileInPairs = 1, kTileOutPairs = 2;
+// Noisy trajectories: the records of a pass are shared by all states; a record made by
+// encode_site stands for the operator that the state's shot drew at the site
+// (choices[shot_of[state] * sites + site], of variants' four records per site).
+struct NoiseSites {
+  const uint8_t* choices = nullptr;
+  const int32_t* shot_of = nullptr;
+  const void* variants = nullptr;
+  int sites = 0;
+};
+void encode_site(void* record, int site);
 cudaError_t launch_tile_pass(int precision, int arithmetic, int io, int n, const PassDesc& pd,
                              void* const* d_states, int nstates, const void* d_kops, int64_t ops_stride,
-                             const double* d_dense, cudaStream_t st);
+                             const double* d_dense, cudaStream_t st,
+                             const NoiseSites* sites = nullptr);
 // io bits for step i of a program: consecutive double-float tiled passes hand the
 // state over as float pairs; the first converts from doubles, the last back.
 int tile_pass_io(const Program& prog, size_t step);
@@ -300,29 +415,20 @@ cudaError_t launch_traj_normalise(int precision, void* const* d_states, int nsta
 cudaError_t launch_traj_sample(int precision, void* const* d_states, const int32_t* d_state_of, int nshots, int n,
                                int shift, uint64_t seed, uint64_t traj0, uint32_t stream, uint64_t* d_out,
                                cudaStream_t st);
-// Shots' Kraus choices, op records, readout noise and final states of noisy trajectories
+// Shots' Kraus choices, readout noise and final states of noisy trajectories
 // (noisy_kernels.cu). A channel of `count` operators chooses the first c with
 // (draw >> 11) < below[c], the integer form of u < cumulative probability; the last one
-// otherwise. launch_noise_records sets *d_differ when a shot's choices are not those of
-// the shot reps[state_of[shot]], and writes the records of `states` states pass-major.
+// otherwise. launch_noise_verify sets *d_differ when a shot's choices are not those of
+// the shot reps[state_of[shot]].
 struct NoiseChannel {
   int32_t count, pad;
   uint64_t below[3];
 };
-struct NoiseRecords {
-  const void* tmpl = nullptr;       // records x pieces x 16 bytes
-  const void* variants = nullptr;   // sites x 4 x pieces x 16 bytes
-  const int32_t* site_of = nullptr;
-  const int64_t* pass_off = nullptr;
-  const int32_t* pass_ops = nullptr;
-  int sites = 0, pieces = 0;
-  int64_t records = 0;
-};
 cudaError_t launch_noise_choices(const NoiseChannel* d_chans, const int32_t* d_site_chan, int sites, uint64_t shot0,
                                  int shots, uint64_t seed, uint32_t stream, uint8_t* d_choices, void* d_hash,
                                  cudaStream_t st);
-cudaError_t launch_noise_records(const NoiseRecords& r, const uint8_t* d_choices, const int32_t* d_state_of, int shots,
-                                 const int32_t* d_reps, int states, void* d_out, int32_t* d_differ, cudaStream_t st);
+cudaError_t launch_noise_verify(const uint8_t* d_choices, int sites, const int32_t* d_state_of, int shots,
+                                const int32_t* d_reps, int32_t* d_differ, cudaStream_t st);
 cudaError_t launch_noise_readout(uint64_t* d_outcomes, int shots, int n, uint64_t seed, uint64_t shot0, uint32_t stream,
                                  double p01, double p10, const double* d_factors, cudaStream_t st);
 cudaError_t launch_noise_collect(int precision, void* const* d_states, const int32_t* d_state_of, int first, int count,

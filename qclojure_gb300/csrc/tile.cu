@@ -45,6 +45,8 @@ __device__ __forceinline__ float mulD(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float addD(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float subD(float a, float b) { return __fsub_rn(a, b); }
 
+struct KOp;
+
 // ---------------------------------------------------------------------------
 // exact policies (FP64 / FP32), register type = double2 / float2
 // ---------------------------------------------------------------------------
@@ -134,6 +136,13 @@ struct PolExact {
     return r;
   }
   __device__ static V times_i(V x) { V r; r.x = -x.y; r.y = x.x; return r; }
+  __device__ static V minus(V x) { V r; r.x = -x.x; r.y = -x.y; return r; }
+  __device__ static V one() { V r; r.x = 1; r.y = 0; return r; }
+  __device__ static V factor(const KOp& op, V f);  // the phase of a record times f
+  __device__ static V mul(V f, V x) { return cm(f.x, f.y, x); }
+  // phases of one run are multiplied together before they meet the amplitudes (not in FP64,
+  // which keeps the reference's order of roundings)
+  static constexpr bool kPhaseRuns = kFMA;
   // entry 0 or 1 of a phase pair (selected without indexing the constant array)
   __device__ static V cmul_idx(const Cst& c, int which, V x) {
     return which ? cm(c.m[2], c.m[3], x) : cm(c.m[0], c.m[1], x);
@@ -233,6 +242,11 @@ struct PolDFT {
     if (CLS == PH_I) return dfc{-x.ih, x.rh, -x.il, x.rl};
     return dfc{x.ih, -x.rh, x.il, -x.rl};
   }
+  static constexpr bool kPhaseRuns = true;
+  __device__ static dfc minus(const dfc& x) { return dfc{-x.rh, -x.ih, -x.rl, -x.il}; }
+  __device__ static dfc one() { return dfc{1.f, 0.f, 0.f, 0.f}; }
+  __device__ static dfc factor(const KOp& op, const dfc& f);
+  __device__ static dfc mul(const dfc& f, const dfc& x) { return cmul_df(f.rh, f.rl, f.ih, f.il, x); }
   __device__ static dfc times_i(const dfc& x) { return dfc{-x.ih, x.rh, -x.il, x.rl}; }
   __device__ static dfc cmul_idx(const Cst& c, int which, const dfc& x) {
     const bool w = which != 0;
@@ -307,8 +321,14 @@ struct CopyPlan {
 // Compact op records passed by value in kernel-parameter (constant-bank) space:
 // every thread reads the same record, so the loads are uniform and cheap.
 // ---------------------------------------------------------------------------
-enum KCode : int32_t {
-  KC_LAYOUT = 0,   // tmask/tval/rmr = register bits rb0/rb1/rb2, c[0..8) = lj (bit patterns)
+enum KCode : int32_t {  // below 16: everything but gates on registers
+  KC_LAYOUT = 0,   // tmask/tval/rmr = register bits rb0/rb1/rb2, c[0..8) = lj (bit patterns);
+                   // with KF_MAP, as 16-bit halves from c[8]: the map's images of the thread's
+                   // bits 0..9, of the three register bits, and its constant
+  KC_MAPX = 2,     // tmask joins the next map's constant where (base & gmask) == gmask
+  KC_REMAP = 3,    // registers are written back through the map (fields as KC_LAYOUT)
+  KC_SITE = 4,     // noise site tval: the operator that the state drew (BatchArgs::sites)
+  KC_PHASES = 5,   // the next tmask records are phases, by register mask (phase_run)
   KC_DENSE = 1,    // tmask = dk, tval = doff, rmr = dbits (4 bits each)
   KC_U2 = 16,      // + cls * 4 + register position
   KC_PHASE = 128,  // + phase class * 8 + register mask (the registers whose bits must all be 1)
@@ -317,7 +337,8 @@ enum KCode : int32_t {
   KC_PARITY = 63,
   KC_COLLAPSE = 64,
   KC_NONE = 65,    // nothing (a noise site whose operator is the identity)
-  KF_COND = 0x100  // the op has control / mask conditions to evaluate
+  KF_COND = 0x100, // the op has control / mask conditions to evaluate
+  KF_MAP = 0x200   // the layout reads its registers through a map
 };
 
 struct __align__(16) KOp {
@@ -554,21 +575,155 @@ __device__ void dense_df(unsigned char* buf, const KOp& op, const double* dense,
   QG_PHASE_CR(CLS, 0) QG_PHASE_CR(CLS, 1) QG_PHASE_CR(CLS, 2) QG_PHASE_CR(CLS, 3) \
   QG_PHASE_CR(CLS, 4) QG_PHASE_CR(CLS, 5) QG_PHASE_CR(CLS, 6) QG_PHASE_CR(CLS, 7)
 
+// The operators of a noisy trajectory's sites: its choices and every site's four operators.
+struct SiteView {
+  const uint8_t* choices;
+  const KOp* variants;
+};
+
+template <typename R, typename V>
+__device__ __forceinline__ V PolExact<R, V>::factor(const KOp& op, V f) {
+  if constexpr (kFMA) return cm((R)op.c[0], (R)op.c[1], f);
+  else return f;
+}
+template <int IO, bool DENSE>
+__device__ __forceinline__ dfc PolDFT<IO, DENSE>::factor(const KOp& op, const dfc& f) {
+  return cmul_df(op.c[0], op.c[8], op.c[1], op.c[9], f);
+}
+
+// A run of `cnt` phases, sorted by the register bits they ask for. Per register mask m, the
+// phases whose tile and thread bits hold are multiplied into one factor (powers of i are
+// counted), and the registers that include m take it: one product per phase and thread, where
+// the phases one by one took a dispatch and a product per register each (a controlled phase:
+// four of eight registers of both tiles). Two tiles at a time where r1 is given.
+template <class P, bool TWO>
+__device__ __forceinline__ void phase_run(typename P::Reg (&r0)[kRegs], typename P::Reg (&r1)[kRegs],
+                                          const KOp* __restrict__ ph, int cnt, uint64_t base0, uint64_t base1,
+                                          uint32_t lt) {
+  using Reg = typename P::Reg;
+  auto turn = [](Reg x, int pw) {
+    if (pw & 1) x = P::times_i(x);
+    if (pw & 2) x = P::minus(x);
+    return x;
+  };
+  int i = 0;
+#pragma unroll
+  for (int m = 0; m < kRegs; ++m) {
+    if (i >= cnt || (ph[i].code & 7) != m) continue;
+    Reg f0 = P::one(), f1 = P::one();
+    int pw0 = 0, pw1 = 0;
+    bool general = false, hit0 = false, hit1 = false;
+    do {
+      const KOp& p = ph[i];
+      const int cls = (p.code >> 3) & 3;
+      const bool tl = (lt & p.tmask) == p.tmask;
+      const bool c0 = tl && (base0 & p.gmask) == p.gmask, c1 = TWO && tl && (base1 & p.gmask) == p.gmask;
+      if (cls == PH_GENERAL) {
+        general = true;
+        const Reg g0 = P::factor(p, f0);
+        if (c0) f0 = g0;
+        hit0 = hit0 || c0;
+        if (TWO) {
+          const Reg g1 = P::factor(p, f1);
+          if (c1) f1 = g1;
+          hit1 = hit1 || c1;
+        }
+      } else {
+        const int q = cls == PH_NEG ? 2 : cls == PH_I ? 1 : 3;
+        pw0 += c0 ? q : 0;
+        if (TWO) pw1 += c1 ? q : 0;
+      }
+      ++i;
+    } while (i < cnt && (ph[i].code & 7) == m);
+    if (general) {
+      f0 = turn(f0, pw0);
+      if (hit0 || (pw0 & 3)) {
+#pragma unroll
+        for (int j = 0; j < kRegs; ++j)
+          if ((j & m) == m) r0[j] = P::mul(f0, r0[j]);
+      }
+      if (TWO) {
+        f1 = turn(f1, pw1);
+        if (hit1 || (pw1 & 3)) {
+#pragma unroll
+          for (int j = 0; j < kRegs; ++j)
+            if ((j & m) == m) r1[j] = P::mul(f1, r1[j]);
+        }
+      }
+    } else {
+      if (pw0 & 3) {
+#pragma unroll
+        for (int j = 0; j < kRegs; ++j)
+          if ((j & m) == m) r0[j] = turn(r0[j], pw0);
+      }
+      if (TWO && (pw1 & 3)) {
+#pragma unroll
+        for (int j = 0; j < kRegs; ++j)
+          if ((j & m) == m) r1[j] = turn(r1[j], pw1);
+      }
+    }
+  }
+}
+
+// A layout's map on this thread: the image of its index bits and the constant; the images of
+// the register bits go to e[0..3).
+__device__ __forceinline__ uint32_t map_of_thread(const KOp& op, uint32_t (&e)[3]) {
+  const uint32_t* h = reinterpret_cast<const uint32_t*>(op.c + 8);
+  auto half = [&](int i) { return (h[i >> 1] >> (16 * (i & 1))) & 0xFFFFu; };
+  uint32_t m = half(13);
+#pragma unroll
+  for (int i = 0; i < 10; ++i) m ^= (0u - ((threadIdx.x >> i) & 1u)) & half(i);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) e[q] = half(10 + q);
+  return m;
+}
+__device__ __forceinline__ uint32_t map_slot(uint32_t m, const uint32_t (&e)[3], int j) {
+  return m ^ ((j & 1) ? e[0] : 0u) ^ ((j & 2) ? e[1] : 0u) ^ ((j & 4) ? e[2] : 0u);
+}
+
 // Apply the pass's ops to the tile in buf. Returns with the tile in raw format.
 template <class P>
 __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int nops, const double* __restrict__ dense,
-                        uint64_t base, const TileGeo& g) {
+                        uint64_t base, const TileGeo& g, const SiteView& sv) {
   using Reg = typename P::Reg;
   constexpr int E = P::kElem;
   Reg r[kRegs];
   int pos[kRegs];  // swizzled shared-memory slot of register j in the current layout
-  uint32_t lt = 0;
-  bool in_regs = false, raw = true;
+  uint32_t lt = 0, mapx = 0;
+  // moved: registers were read from other threads' slots, so the next stores wait for all reads
+  bool in_regs = false, raw = true, moved = false;
   for (int o = 0; o < nops; ++o) {
-    const KOp& op = sops[o];  // shared memory: a broadcast read
-    const int code = op.code;
-    if (code == KC_LAYOUT) {
+    const KOp* rec = sops + o;  // shared memory: a broadcast read
+    int code = rec->code;
+    if ((code & 0xFF) < 16) {
+    const KOp& op = *rec;
+    if (code == KC_SITE) {
+      rec = sv.variants + ((size_t)op.tval * 4 + __ldg(sv.choices + op.tval));
+      code = rec->code;
+      if (code == KC_NONE) continue;
+    } else {
+    if (code == KC_MAPX) {
+      if ((base & op.gmask) == op.gmask) mapx ^= op.tmask;
+      continue;
+    }
+    if constexpr (P::kPhaseRuns) {
+      if (code == KC_PHASES) {
+        phase_run<P, false>(r, r, sops + o + 1, (int)op.tmask, base, 0, lt);
+        o += (int)op.tmask;
+        continue;
+      }
+    }
+    if (code == KC_REMAP) {
+      uint32_t e[3];
+      const uint32_t m = map_of_thread(op, e) ^ mapx;
+#pragma unroll
+      for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>((int)map_slot(m, e, j));
+      moved = true;  // the slots are other threads' whatever the layout read
+      continue;
+    }
+    if ((code & 0xFF) == KC_LAYOUT) {
       if (in_regs) {
+        if (moved) __syncthreads();
 #pragma unroll
         for (int j = 0; j < kRegs; ++j) P::store_work(buf, pos[j], r[j]);
         raw = false;
@@ -581,12 +736,19 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
       for (int q = 0; q < 3; ++q) lt = ((lt >> rb[q]) << (rb[q] + 1)) | (lt & ((1u << rb[q]) - 1));
 #pragma unroll
       for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>(lt | __float_as_uint(op.c[j]));
+      moved = (code & KF_MAP) != 0;
+      uint32_t m = 0, e[3] = {0, 0, 0};
+      if (moved) {
+        m = map_of_thread(op, e) ^ mapx;
+        mapx = 0;
+      }
+      auto from = [&](int j) { return moved ? swz<E>((int)map_slot(m, e, j)) : pos[j]; };
       if (raw) {
 #pragma unroll
-        for (int j = 0; j < kRegs; ++j) r[j] = P::load_raw(buf, pos[j]);
+        for (int j = 0; j < kRegs; ++j) r[j] = P::load_raw(buf, from(j));
       } else {
 #pragma unroll
-        for (int j = 0; j < kRegs; ++j) r[j] = P::load_work(buf, pos[j]);
+        for (int j = 0; j < kRegs; ++j) r[j] = P::load_work(buf, from(j));
       }
       in_regs = true;
       continue;
@@ -609,6 +771,10 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
       }
       continue;
     }
+    continue;
+    }
+    }
+    const KOp& op = *rec;
     bool tc = true;
     uint32_t cr = 0;
     if (code & KF_COND) {
@@ -660,6 +826,7 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
     }
   }
   if (in_regs) {
+    if (moved) __syncthreads();
 #pragma unroll
     for (int j = 0; j < kRegs; ++j) P::store_raw(buf, pos[j], r[j]);
   } else if (!raw) {
@@ -718,19 +885,48 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
 
 template <class P>
 __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __restrict__ sops, int nops,
-                         const double* __restrict__ dense, uint64_t base0, uint64_t base1, const TileGeo& g) {
+                         const double* __restrict__ dense, uint64_t base0, uint64_t base1, const TileGeo& g,
+                         const SiteView& sv) {
   static_assert(!P::kDF && !P::kInPairs && !P::kOutPairs, "two-tile interpretation: one storage format");
   using Reg = typename P::Reg;
   constexpr int E = P::kElem;
   Reg r0[kRegs], r1[kRegs];
   int pos[kRegs];  // swizzled shared-memory slot of register j in the current layout (both tiles)
-  uint32_t lt = 0;
-  bool in_regs = false;
+  uint32_t lt = 0, mapx0 = 0, mapx1 = 0;
+  int apart = 0;  // the slots of tile 1 against tile 0's (a map's tile-conditioned parts)
+  bool in_regs = false, moved = false;
   for (int o = 0; o < nops; ++o) {
-    const KOp& op = sops[o];
-    const int code = op.code;
-    if (code == KC_LAYOUT) {
+    const KOp* rec = sops + o;
+    int code = rec->code;
+    if ((code & 0xFF) < 16) {
+    const KOp& op = *rec;
+    if (code == KC_SITE) {
+      rec = sv.variants + ((size_t)op.tval * 4 + __ldg(sv.choices + op.tval));
+      code = rec->code;
+      if (code == KC_NONE) continue;
+    } else {
+    if (code == KC_MAPX) {
+      if ((base0 & op.gmask) == op.gmask) mapx0 ^= op.tmask;
+      if ((base1 & op.gmask) == op.gmask) mapx1 ^= op.tmask;
+      continue;
+    }
+    if (code == KC_PHASES) {
+      phase_run<P, true>(r0, r1, sops + o + 1, (int)op.tmask, base0, base1, lt);
+      o += (int)op.tmask;
+      continue;
+    }
+    if (code == KC_REMAP) {
+      uint32_t e[3];
+      const uint32_t m = map_of_thread(op, e) ^ mapx0;
+#pragma unroll
+      for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>((int)map_slot(m, e, j));
+      apart = swz<E>((int)(mapx0 ^ mapx1));
+      moved = true;
+      continue;
+    }
+    if ((code & 0xFF) == KC_LAYOUT) {
       if (in_regs) {
+        if (moved) __syncthreads();
 #pragma unroll
         for (int j = 0; j < kRegs; ++j) {
           P::store_work(buf0, pos[j], r0[j]);
@@ -744,10 +940,24 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
       for (int q = 0; q < 3; ++q) lt = ((lt >> rb[q]) << (rb[q] + 1)) | (lt & ((1u << rb[q]) - 1));
 #pragma unroll
       for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>(lt | __float_as_uint(op.c[j]));
+      moved = (code & KF_MAP) != 0;
+      if (moved) {
+        uint32_t e[3];
+        const uint32_t m = map_of_thread(op, e) ^ mapx0;
+        const int d = swz<E>((int)(mapx0 ^ mapx1));
+        mapx0 = mapx1 = 0;
 #pragma unroll
-      for (int j = 0; j < kRegs; ++j) {
-        r0[j] = P::load_work(buf0, pos[j]);
-        r1[j] = P::load_work(buf1, pos[j]);
+        for (int j = 0; j < kRegs; ++j) {
+          const int at = swz<E>((int)map_slot(m, e, j));
+          r0[j] = P::load_work(buf0, at);
+          r1[j] = P::load_work(buf1, at ^ d);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kRegs; ++j) {
+          r0[j] = P::load_work(buf0, pos[j]);
+          r1[j] = P::load_work(buf1, pos[j]);
+        }
       }
       in_regs = true;
       continue;
@@ -768,6 +978,10 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
       }
       continue;
     }
+    continue;
+    }
+    }
+    const KOp& op = *rec;
     bool tc0 = true, tc1 = true;
     uint32_t cr = 0;
     if (code & KF_COND) {
@@ -834,10 +1048,11 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
     }
   }
   if (in_regs) {
+    if (moved) __syncthreads();
 #pragma unroll
     for (int j = 0; j < kRegs; ++j) {
       P::store_raw(buf0, pos[j], r0[j]);
-      P::store_raw(buf1, pos[j], r1[j]);
+      P::store_raw(buf1, pos[j] ^ apart, r1[j]);
     }
   }
   __syncthreads();
@@ -855,6 +1070,7 @@ struct BatchArgs {
   const KOp* kops;               // op records of state 0
   int64_t ops_stride;            // records between consecutive states' lists (0: one shared list)
   int nstates;
+  NoiseSites sites;              // noisy trajectories: the shared list holds KC_SITE records
 };
 
 template <class P>
@@ -894,6 +1110,11 @@ __global__ void __launch_bounds__(512, 1) k_tile2(const PassDesc pd, const Batch
     const uint64_t t0 = w - (uint64_t)si * ntiles;
     const uint64_t t1 = (ntiles - t0 < w1 - w) ? ntiles : t0 + (w1 - w);
     unsigned char* state = ba.states[si];
+    SiteView sv{nullptr, nullptr};
+    if (ba.sites.sites > 0) {
+      sv.choices = ba.sites.choices + (size_t)ba.sites.shot_of[si] * (size_t)ba.sites.sites;
+      sv.variants = reinterpret_cast<const KOp*>(ba.sites.variants);
+    }
     if (staged < 0 || (si != staged && ba.ops_stride != 0)) {
       __syncthreads();  // previous segment's readers of sops are done
       const uint4* src = reinterpret_cast<const uint4*>(ba.kops + (int64_t)si * ba.ops_stride);
@@ -929,11 +1150,11 @@ __global__ void __launch_bounds__(512, 1) k_tile2(const PassDesc pd, const Batch
           }
           __syncthreads();
           if (cnt == 2) {
-            run_ops2<P>(buf(2 * slot), buf(2 * slot + 1), sops, nops, dense, b0, b1, g);
+            run_ops2<P>(buf(2 * slot), buf(2 * slot + 1), sops, nops, dense, b0, b1, g, sv);
             cp.store(buf(2 * slot), state + b0 * E);
             cp.store(buf(2 * slot + 1), state + b1 * E);
           } else {
-            run_ops<P>(buf(2 * slot), sops, nops, dense, b0, g);
+            run_ops<P>(buf(2 * slot), sops, nops, dense, b0, g, sv);
             cp.store(buf(2 * slot), state + b0 * E);
           }
           __syncthreads();  // these buffers are refilled by the pair after next
@@ -959,7 +1180,7 @@ __global__ void __launch_bounds__(512, 1) k_tile2(const PassDesc pd, const Batch
         cp_wait<0>();
       }
       __syncthreads();
-      run_ops<P>(cur, sops, nops, dense, base, g);
+      run_ops<P>(cur, sops, nops, dense, base, g, sv);
       cp.store(cur, state + base * E);
       __syncthreads();  // the buffer is refilled two tiles later
       base = nbase;
@@ -1015,7 +1236,7 @@ __global__ void __launch_bounds__(512, 1) k_tile_jobs(int n, const TileJobRec* _
       const int words = nops * (int)(sizeof(KOp) / 16);
       for (int q = threadIdx.x; q < words; q += g.T) dst[q] = src[q];
       __syncthreads();
-      run_ops<P>(tile, sops, nops, nullptr, 0, g);  // ends with a barrier
+      run_ops<P>(tile, sops, nops, nullptr, 0, g, SiteView{nullptr, nullptr});  // ends with a barrier
       ob += nops;
     }
     if constexpr (P::kOutPairs) {  // float pairs -> IEEE doubles
@@ -1129,7 +1350,7 @@ __global__ void __launch_bounds__(512, 1) k_job_loop(int n, JobLoopSlot* slots, 
       const int words = nops * (int)(sizeof(KOp) / 16);
       for (int q = threadIdx.x; q < words; q += g.T) dst[q] = src[q];
       __syncthreads();
-      run_ops<P>(tile, sops, nops, nullptr, 0, g);  // ends with a barrier
+      run_ops<P>(tile, sops, nops, nullptr, 0, g, SiteView{nullptr, nullptr});  // ends with a barrier
       ob += nops;
     }
     if constexpr (P::kOutPairs) {  // float pairs -> IEEE doubles
@@ -1158,12 +1379,27 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
   for (int64_t o = 0; o < nops; ++o) {
     const TOp& t = ops[o];
     KOp& k = out[o];
-    if (t.kind == OK_LAYOUT) {
-      k.code = KC_LAYOUT;
+    if (t.kind == OK_MAPX) {
+      k.code = KC_MAPX;
+      k.gmask = t.gmask;
+      k.tmask = t.mc0;
+      continue;
+    }
+    if (t.kind == OK_LAYOUT || t.kind == OK_REMAP) {
+      k.code = t.kind == OK_REMAP ? KC_REMAP : t.mapped ? KC_LAYOUT | KF_MAP : KC_LAYOUT;
       k.tmask = t.dbits[0];
       k.tval = t.dbits[1];
       k.rmr = t.dbits[2];
       for (int j = 0; j < 8; ++j) std::memcpy(&k.c[j], &t.lj[j], 4);
+      if (t.mapped) {
+        uint16_t h[16] = {0};
+        int i = 0;
+        for (int b = 0; b < kMaxTileBits && i < 10; ++b)  // thread bits: the others, ascending
+          if (b != t.dbits[0] && b != t.dbits[1] && b != t.dbits[2]) h[i++] = t.mcol[b];
+        for (int q = 0; q < 3; ++q) h[10 + q] = t.mcol[t.dbits[q]];
+        h[13] = t.mc0;
+        std::memcpy(&k.c[8], h, sizeof(h));
+      }
       continue;
     }
     if (t.kind == OK_DENSE) {
@@ -1186,6 +1422,10 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
       case OK_NONE:
         k.code = KC_NONE;
         break;
+      case OK_PHASES:
+        k.code = KC_PHASES;
+        k.tmask = (uint32_t)t.dk;
+        continue;
       case OK_U2:
         k.code = KC_U2 + t.cls * 4 + t.t2;
         k.gmask = k.gval = t.gcmask;
@@ -1279,6 +1519,13 @@ void encode_kops(int precision, int arithmetic, const TOp* tops, int64_t count, 
   else build_kops<PolD>(k, tops, count);
 }
 
+void encode_site(void* record, int site) {
+  KOp* k = reinterpret_cast<KOp*>(record);
+  std::memset(k, 0, sizeof(KOp));
+  k->code = KC_SITE;
+  k->tval = (uint32_t)site;
+}
+
 template <class P>
 cudaError_t launch_jobs_t(int n, const TileJobRec* d_jobs, int njobs, const KOp* d_kops, const int32_t* d_pass_nops,
                           cudaStream_t st) {
@@ -1330,13 +1577,14 @@ cudaError_t launch_tile_jobs(int precision, int arithmetic, int n, const TileJob
 
 cudaError_t launch_tile_pass(int precision, int arithmetic, int io, int n, const PassDesc& pd,
                              void* const* d_states, int nstates, const void* d_kops, int64_t ops_stride,
-                             const double* d_dense, cudaStream_t st) {
+                             const double* d_dense, cudaStream_t st, const NoiseSites* sites) {
   if (pd.k < 3 || pd.k > kMaxTileBits) return cudaErrorInvalidValue;
   BatchArgs ba;
   ba.states = reinterpret_cast<unsigned char* const*>(d_states);
   ba.kops = reinterpret_cast<const KOp*>(d_kops) + pd.op_begin;
   ba.ops_stride = ops_stride;
   ba.nstates = nstates;
+  ba.sites = sites ? *sites : NoiseSites{};
   if (precision == QG_C64) return launch_t<PolF>(n, pd, ba, d_dense, st);
   if (arithmetic == QG_ARITH_DOUBLE_FLOAT) {
     switch (io & 3) {
