@@ -1382,7 +1382,9 @@ std::string pass_structure_key(const Program& prog, bool table) {
   // the program's passes as bytes (descriptors, hand-over form, op records), which
   // determine the generated source; with a coefficient table the entries' values
   // are left out and only the value-dependent code choices are kept (the
-  // Hadamard shape of a real 2x2, the signs of an imaginary antidiagonal)
+  // Hadamard shape of a real 2x2, the signs of an imaginary antidiagonal; the sign
+  // of a rotation's sine is a value: parameter-shift points on both sides of zero
+  // share their kernels)
   std::string key = std::to_string(prog.arith) + (table ? ":table:" : ":lit:");
   for (size_t i = 0; i < prog.steps.size(); ++i) {
     const Step& st = prog.steps[i];
@@ -1399,8 +1401,9 @@ std::string pass_structure_key(const Program& prog, bool table) {
         // layout-relative fields do not matter; parity masks are data
         if (t.kind == OK_LAYOUT) continue;
         const double* m = t.m;
+        const bool anti = t.kind == OK_U2 && t.cls == U2_IMAG_ANTI;
         const char shape[5] = {(char)(t.cls == U2_REAL && m[0] == m[2] && m[0] == m[4] && m[6] == -m[0]),
-                               (char)(m[3] > 0), (char)(m[5] > 0),
+                               (char)(anti && m[3] > 0), (char)(anti && m[5] > 0),
                                (char)(prev && same_parity_phases(*prev, prog.tops[o])),
                                (char)(unit_diagonal(t))};
         prev = &prog.tops[o];
