@@ -189,23 +189,18 @@ __global__ void __launch_bounds__(256) k_swap(typename C2<R>::T* __restrict__ s,
   }
 }
 
-// kind: 0 blockade (popcount==1 -> ph), 1 parity (ph0/ph1), 2 collapse (match -> scale, else 0)
+// kind: 0 blockade (popcount==1 -> ph), 1 parity (ph0/ph1)
 template <int KIND, typename R>
 __global__ void __launch_bounds__(256) k_diag_all(typename C2<R>::T* __restrict__ s, uint64_t N, uint64_t mask,
-                                                  uint64_t val, Mat<R> m) {
+                                                  Mat<R> m) {
   using V = typename C2<R>::T;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (uint64_t)gridDim.x * blockDim.x) {
     V x = s[i];
     if (KIND == 0) {
       if (__popcll(i & mask) == 1) s[i] = cmul(m.m[0], m.m[1], x);
-    } else if (KIND == 1) {
+    } else {
       if (__popcll(i & mask) & 1) s[i] = cmul(m.m[2], m.m[3], x);
       else s[i] = cmul(m.m[0], m.m[1], x);
-    } else {
-      V r;
-      if ((i & mask) == val) { r.x = mul_(x.x, m.m[0]); r.y = mul_(x.y, m.m[0]); }
-      else { r.x = 0; r.y = 0; }
-      s[i] = r;
     }
   }
 }
@@ -250,13 +245,10 @@ cudaError_t plain_op_t(void* sv, int n, const GOp& op, cudaStream_t st) {
       k_swap<R><<<grid_for(work, T), T, 0, st>>>(s, work, (1ULL << op.t) | (1ULL << op.t2), f, op.flags & 1);
     } break;
     case OK_BLOCKADE:
-      k_diag_all<0, R><<<grid_for(N, T), T, 0, st>>>(s, N, op.mask, 0, to_mat<R>(op.m));
+      k_diag_all<0, R><<<grid_for(N, T), T, 0, st>>>(s, N, op.mask, to_mat<R>(op.m));
       break;
     case OK_PARITY:
-      k_diag_all<1, R><<<grid_for(N, T), T, 0, st>>>(s, N, op.mask, 0, to_mat<R>(op.m));
-      break;
-    case OK_COLLAPSE:
-      k_diag_all<2, R><<<grid_for(N, T), T, 0, st>>>(s, N, op.mask, op.val, to_mat<R>(op.m));
+      k_diag_all<1, R><<<grid_for(N, T), T, 0, st>>>(s, N, op.mask, to_mat<R>(op.m));
       break;
     default:
       return cudaErrorInvalidValue;
@@ -315,6 +307,9 @@ __device__ __forceinline__ double p_of(typename C2<R>::T a) {
     return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
   }
 }
+
+// floor(p 2^62) on the integer pipes (quant.cuh): the FP64 product and conversion's value
+__device__ __forceinline__ unsigned long long quant(double p) { return qg_quant62(p); }
 
 template <typename R>
 __global__ void __launch_bounds__(256) k_probs(const typename C2<R>::T* __restrict__ s, uint64_t N,
@@ -406,26 +401,49 @@ __global__ void __launch_bounds__(256) k_compare(const typename C2<R>::T* __rest
   }
 }
 
-// Marginal over fixed-bit outcomes: blockIdx.y = outcome over the unique measured bits.
+// Measurement of m distinct qubits without a trip to the host: k_marginal sums every outcome's
+// probability (compensated FP64) and quantised probability (integers), k_measure_pick draws
+// the outcome and k_collapse projects on it. Bound by the FP64 pipe: three instructions per
+// probability, a tree over 16 of them before each TwoSum (20 qubits, three measured: 56 us with
+// a TwoSum per amplitude and an FP64 quantisation), and by launches: the host used to wait for
+// the partial sums of every measurement (about 70 us each).
+struct MeasuredBits {
+  int m;
+  int pos[16];   // the measured bits, ascending
+  int rank[16];  // outcome bit of each
+};
+__device__ __forceinline__ uint64_t spread(uint64_t j, const MeasuredBits& f, uint32_t o) {
+#pragma unroll 1
+  for (int i = 0; i < f.m; ++i) {
+    const int b = f.pos[i];
+    const uint64_t lo = j & ((1ULL << b) - 1);
+    j = ((j >> b) << (b + 1)) | ((uint64_t)((o >> f.rank[i]) & 1u) << b) | lo;
+  }
+  return j;
+}
+
 template <typename R>
-__global__ void __launch_bounds__(256) k_marginal(const typename C2<R>::T* __restrict__ s, uint64_t work, Fixed f0,
-                                                  int m, const int* __restrict__ bits, double* d_pm,
-                                                  unsigned long long* d_qm) {
-  const int o = blockIdx.y;
-  Fixed f = f0;
-  uint64_t set = 0;
-  for (int k = 0; k < m; ++k)
-    if ((o >> k) & 1) set |= 1ULL << bits[k];
-  f.setmask = set;
+__global__ void __launch_bounds__(256) k_marginal(const typename C2<R>::T* __restrict__ s, uint64_t work,
+                                                  const MeasuredBits f, double* __restrict__ d_pm,
+                                                  unsigned long long* __restrict__ d_qm) {
+  const uint32_t o = blockIdx.y;
   DD acc{0, 0};
   unsigned long long qs = 0;
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < work; j += (uint64_t)gridDim.x * blockDim.x) {
-    double p = p_of<R>(s[expand(j, f)]);
-    two_sum_acc(acc, p);
-    double v = p * 4611686018427387904.0;
-    qs += (v > 0) ? (unsigned long long)v : 0ULL;
+  for (uint64_t t = (uint64_t)blockIdx.x * 4096; t < work; t += (uint64_t)gridDim.x * 4096) {
+    double v[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const uint64_t j = t + threadIdx.x + (uint64_t)r * 256;
+      v[r] = j < work ? p_of<R>(s[spread(j, f, o)]) : 0.0;
+      qs += quant(v[r]);
+    }
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+      for (int r = 0; r < w; ++r) v[r] = __dadd_rn(v[r], v[r + w]);
+    two_sum_acc(acc, v[0]);
   }
-  const int slot = o * gridDim.x + blockIdx.x;
+  const int slot = (int)(o * gridDim.x + blockIdx.x);
   block_reduce_store<256>(acc, d_pm, slot);
   __shared__ unsigned long long qred[8];
   for (int off = 16; off > 0; off >>= 1) qs += __shfl_down_sync(0xffffffffu, qs, off);
@@ -435,6 +453,91 @@ __global__ void __launch_bounds__(256) k_marginal(const typename C2<R>::T* __res
     unsigned long long t = 0;
     for (int w = 0; w < 8; ++w) t += qred[w];
     d_qm[slot] = t;
+  }
+}
+
+// One CTA. A warp folds each outcome's partials; the first warp then takes the first outcome
+// whose cumulative quantised probability exceeds floor(draw T / 2^64) (the last one when T is
+// 0), each lane over its share of the outcomes.
+__global__ void __launch_bounds__(1024) k_measure_pick(const double* __restrict__ pm,
+                                                       const unsigned long long* __restrict__ qm, int nbx,
+                                                       const MeasuredBits f, uint64_t draw, double* __restrict__ P,
+                                                       unsigned long long* __restrict__ Q, MeasurePick* out) {
+  const int nout = 1 << f.m, lane = threadIdx.x & 31;
+  for (int o = threadIdx.x >> 5; o < nout; o += 32) {
+    DD a{0, 0};
+    unsigned long long q = 0;
+    for (int b = lane; b < nbx; b += 32) {
+      const int slot = o * nbx + b;
+      two_sum_acc(a, pm[2 * slot]);
+      a.c = __dadd_rn(a.c, pm[2 * slot + 1]);
+      q += qm[slot];
+    }
+    for (int d = 16; d > 0; d >>= 1) {
+      DD w;
+      w.s = __shfl_down_sync(0xffffffffu, a.s, d);
+      w.c = __shfl_down_sync(0xffffffffu, a.c, d);
+      a = dd_add(a, w);
+      q += __shfl_down_sync(0xffffffffu, q, d);
+    }
+    if (lane == 0) {
+      P[o] = __dadd_rn(a.s, a.c);
+      Q[o] = q;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int per = (nout + 31) / 32, first = lane * per, last = min(nout, first + per);
+  unsigned long long mine = 0;
+  for (int o = first; o < last; ++o) mine += Q[o];
+  unsigned long long incl = mine;
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  const unsigned long long T = __shfl_sync(0xffffffffu, incl, 31), u = __umul64hi(draw, T);
+  const unsigned ballot = __ballot_sync(0xffffffffu, incl > u);
+  const int owner = T > 0 ? __ffs((int)ballot) - 1 : 31;
+  if (lane != owner) return;
+  int sel = nout - 1;
+  if (T > 0) {
+    unsigned long long c = incl - mine;
+    for (int o = first; o < last; ++o) {
+      c += Q[o];
+      if (c > u) {
+        sel = o;
+        break;
+      }
+    }
+  }
+  out->outcome = (uint64_t)sel;
+  out->probability = P[sel];
+  out->scale = P[sel] > 0 ? __ddiv_rn(1.0, __dsqrt_rn(P[sel])) : 1.0;
+  uint64_t mask = 0, val = 0;
+  for (int i = 0; i < f.m; ++i) {
+    mask |= 1ULL << f.pos[i];
+    if ((sel >> f.rank[i]) & 1) val |= 1ULL << f.pos[i];
+  }
+  out->mask = mask;
+  out->val = val;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) k_collapse(typename C2<R>::T* __restrict__ s, uint64_t N,
+                                                  const MeasurePick* __restrict__ pick) {
+  using V = typename C2<R>::T;
+  const uint64_t mask = pick->mask, val = pick->val;
+  const R scale = (R)pick->scale;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (uint64_t)gridDim.x * blockDim.x) {
+    V r;
+    r.x = 0;
+    r.y = 0;
+    if ((i & mask) == val) {
+      const V x = s[i];
+      r.x = mul_(x.x, scale);
+      r.y = mul_(x.y, scale);
+    }
+    s[i] = r;
   }
 }
 
@@ -503,9 +606,6 @@ SampleGeom sample_geom(int n) {
   g.nb = nch / g.cpb;
   return g;
 }
-
-// floor(p 2^62) on the integer pipes (quant.cuh): the FP64 product and conversion's value
-__device__ __forceinline__ unsigned long long quant(double p) { return qg_quant62(p); }
 
 // one CTA (256 threads = 8 warps) per sample block. Only integer sums are formed here:
 // the FP64 total of the normalisation check is derived from them (k_samp_scan). A
@@ -990,18 +1090,41 @@ cudaError_t launch_compare(const void* a, int precision, const void* b, int n, d
   return cudaGetLastError();
 }
 
-cudaError_t launch_marginal_host(const void* s, int precision, int n, const int* h_bits, const int* d_bits, int m,
-                                 int nbx, double* d_pm, unsigned long long* d_qm, cudaStream_t st) {
-  uint64_t zero = 0;
-  for (int k = 0; k < m; ++k) zero |= 1ULL << h_bits[k];
-  Fixed f = make_fixed(zero, 0);
-  uint64_t work = (1ULL << n) >> m;
-  dim3 grid(nbx, 1u << m);
-  if (precision == QG_C64)
-    k_marginal<float><<<grid, 256, 0, st>>>((const float2*)s, work, f, m, d_bits, d_pm, d_qm);
-  else
-    k_marginal<double><<<grid, 256, 0, st>>>((const double2*)s, work, f, m, d_bits, d_pm, d_qm);
-  counted();
+// scratch: measure_scratch_bytes(m); *pick is device memory
+static int measure_chunks(int n, int m) {
+  const uint64_t work = (1ULL << n) >> m;
+  return (int)std::max<uint64_t>(1, std::min<uint64_t>((work + 4095) / 4096, 1024u >> m));
+}
+size_t measure_scratch_bytes(int n, int m) {
+  const size_t slots = (size_t)measure_chunks(n, m) << m;
+  return slots * (2 * sizeof(double) + sizeof(unsigned long long)) +
+         ((size_t)1 << m) * (sizeof(double) + sizeof(unsigned long long));
+}
+cudaError_t launch_measure(void* s, int precision, int n, const int* bits, int m, uint64_t draw, void* d_scratch,
+                           MeasurePick* d_pick, cudaStream_t st) {
+  MeasuredBits f;
+  f.m = m;
+  int at = 0;
+  for (int b = 0; b < n; ++b)
+    for (int k = 0; k < m; ++k)
+      if (bits[k] == b) {
+        f.pos[at] = b;
+        f.rank[at++] = k;
+      }
+  const uint64_t N = 1ULL << n, work = N >> m;
+  const int nbx = measure_chunks(n, m);
+  const size_t slots = (size_t)nbx << m;
+  double* pm = reinterpret_cast<double*>(d_scratch);
+  unsigned long long* qm = reinterpret_cast<unsigned long long*>(pm + 2 * slots);
+  double* P = reinterpret_cast<double*>(qm + slots);
+  unsigned long long* Q = reinterpret_cast<unsigned long long*>(P + ((size_t)1 << m));
+  const dim3 grid((unsigned)nbx, 1u << m);
+  if (precision == QG_C64) k_marginal<float><<<grid, 256, 0, st>>>((const float2*)s, work, f, pm, qm);
+  else k_marginal<double><<<grid, 256, 0, st>>>((const double2*)s, work, f, pm, qm);
+  k_measure_pick<<<1, 1024, 0, st>>>(pm, qm, nbx, f, draw, P, Q, d_pick);
+  if (precision == QG_C64) k_collapse<float><<<grid_for(N, 256), 256, 0, st>>>((float2*)s, N, d_pick);
+  else k_collapse<double><<<grid_for(N, 256), 256, 0, st>>>((double2*)s, N, d_pick);
+  counted(3);
   return cudaGetLastError();
 }
 

@@ -471,9 +471,16 @@ cudaError_t launch_inner(const void* a, const void* b, int precision, int n, dou
 // a: complex64 or complex128, b: complex128; partials 6 x nblocks double-doubles, maxima nblocks
 cudaError_t launch_compare(const void* a, int precision, const void* b, int n, double* d_part, double* d_max,
                            int nblocks, cudaStream_t st);
-// Marginal probabilities over measured bits: per outcome FP64 (sum, comp) and u64 quantised totals.
-cudaError_t launch_marginal_host(const void* s, int precision, int n, const int* h_bits, const int* d_bits, int m,
-                                 int nbx, double* d_pm, unsigned long long* d_qm, cudaStream_t st);
+// Measures bits[0..m) (distinct, m <= 15; outcome bit k <-> bits[k]): draws the outcome from
+// `draw` (the first whose cumulative quantised probability exceeds floor(draw T / 2^64)),
+// projects the state on it and renormalises, all on the stream; *d_pick tells what was drawn.
+struct MeasurePick {
+  uint64_t outcome, mask, val;
+  double probability, scale;
+};
+size_t measure_scratch_bytes(int n, int m);
+cudaError_t launch_measure(void* s, int precision, int n, const int* bits, int m, uint64_t draw, void* d_scratch,
+                           MeasurePick* d_pick, cudaStream_t st);
 cudaError_t launch_gather(const void* s, int precision, const uint64_t* d_idx, int64_t count, double* d_out,
                           cudaStream_t st);
 cudaError_t launch_density(const void* s, int precision, int n, double* d_rho, cudaStream_t st);

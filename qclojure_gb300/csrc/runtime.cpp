@@ -160,113 +160,39 @@ struct ExecStats {
 
 static int do_measure(State* s, const std::vector<int>& qubits, uint64_t seed, uint64_t draw_index,
                       uint64_t* outcome_out, double* prob_out, std::string* err) {
-  const int n = s->n;
-  const int m_orig = (int)qubits.size();
-  // unique bits in order of first appearance
-  std::vector<int> ubits;
-  std::vector<int> orig_to_u(m_orig);
-  for (int k = 0; k < m_orig; ++k) {
-    int b = n - 1 - qubits[k];
-    auto it = std::find(ubits.begin(), ubits.end(), b);
-    if (it == ubits.end()) {
-      orig_to_u[k] = (int)ubits.size();
-      ubits.push_back(b);
-    } else {
-      orig_to_u[k] = (int)(it - ubits.begin());
-    }
+  // Distinct bits in order of their last appearance: outcomes (bit k <-> qubits[k]) that agree
+  // on repeated qubits then have the same order as the outcomes of the distinct bits.
+  std::vector<int> bits;
+  for (size_t k = 0; k < qubits.size(); ++k) {
+    const int b = s->n - 1 - qubits[k];
+    bits.erase(std::remove(bits.begin(), bits.end(), b), bits.end());
+    bits.push_back(b);
   }
-  const int m = (int)ubits.size();
+  const int m = (int)bits.size();
   if (m > 15) {
     *err = "measurement of more than 15 distinct qubits is not supported";
     return QG_ERR_UNSUPPORTED;
   }
-  const int nout = 1 << m;
-  int nbx = std::max(1, 1024 / nout);
-  uint64_t work = (1ULL << n) >> m;
-  if ((uint64_t)nbx * 256 > work) nbx = (int)std::max<uint64_t>(1, (work + 255) / 256);
-  int* d_bits = nullptr;
-  double* d_pm = nullptr;
-  unsigned long long* d_qm = nullptr;
-  CK(cudaMallocAsync((void**)&d_bits, sizeof(int) * 16, s->stream), "alloc");
-  CK(cudaMallocAsync((void**)&d_pm, sizeof(double) * 2 * nout * nbx, s->stream), "alloc");
-  CK(cudaMallocAsync((void**)&d_qm, sizeof(unsigned long long) * nout * nbx, s->stream), "alloc");
-  CK(cudaMemcpyAsync(d_bits, ubits.data(), sizeof(int) * m, cudaMemcpyHostToDevice, s->stream), "H2D bits");
-  CK(launch_marginal_host(s->d, s->prec, n, ubits.data(), d_bits, m, nbx, d_pm, d_qm, s->stream), "marginal");
-  std::vector<double> hpm(2 * (size_t)nout * nbx);
-  std::vector<unsigned long long> hqm((size_t)nout * nbx);
-  CK(cudaMemcpyAsync(hpm.data(), d_pm, sizeof(double) * hpm.size(), cudaMemcpyDeviceToHost, s->stream), "D2H");
-  CK(cudaMemcpyAsync(hqm.data(), d_qm, sizeof(unsigned long long) * hqm.size(), cudaMemcpyDeviceToHost, s->stream),
-     "D2H");
-  CK(cudaStreamSynchronize(s->stream), "sync");
-  cudaFreeAsync(d_bits, s->stream);
-  cudaFreeAsync(d_pm, s->stream);
-  cudaFreeAsync(d_qm, s->stream);
-  std::vector<double> Pu(nout);
-  std::vector<uint64_t> Qu(nout);
-  for (int o = 0; o < nout; ++o) {
-    double hi = 0, lo = 0;
-    uint64_t q = 0;
-    for (int b = 0; b < nbx; ++b) {
-      size_t slot = (size_t)o * nbx + b;
-      double x = hpm[2 * slot];
-      double t = hi + x, bp = t - hi;
-      lo += (hi - (t - bp)) + (x - bp);
-      hi = t;
-      lo += hpm[2 * slot + 1];
-      q += hqm[slot];
-    }
-    Pu[o] = hi + lo;
-    Qu[o] = q;
+  const size_t scratch = (measure_scratch_bytes(s->n, m) + 255) / 256 * 256;
+  unsigned char* d = nullptr;
+  CK(cudaMallocAsync((void**)&d, scratch + sizeof(MeasurePick), s->stream), "alloc");
+  MeasurePick* d_pick = reinterpret_cast<MeasurePick*>(d + scratch);
+  MeasurePick pick{};
+  cudaError_t e = launch_measure(s->d, s->prec, s->n, bits.data(), m, draw64(seed, draw_index, 1u), d, d_pick, s->stream);
+  const bool wanted = outcome_out || prob_out;
+  if (e == cudaSuccess && wanted) {
+    e = cudaMemcpyAsync(&pick, d_pick, sizeof(pick), cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   }
-  // outcomes in the reference's index order (bit k <-> qubits[k])
-  const uint64_t norig = 1ULL << m_orig;
-  auto to_u = [&](uint64_t o, bool* ok) {
-    uint64_t u = 0;
-    uint64_t seen = 0, val = 0;
-    for (int k = 0; k < m_orig; ++k) {
-      int ui = orig_to_u[k];
-      uint64_t bit = (o >> k) & 1;
-      if (seen & (1ULL << ui)) {
-        if (((val >> ui) & 1) != bit) { *ok = false; return (uint64_t)0; }
-      } else {
-        seen |= 1ULL << ui;
-        val |= bit << ui;
-      }
-    }
-    u = val;
-    *ok = true;
-    return u;
-  };
-  uint64_t T = 0;
-  for (int o = 0; o < nout; ++o) T += Qu[o];
-  uint64_t sel = norig - 1;
-  if (T > 0) {
-    unsigned __int128 prod = (unsigned __int128)draw64(seed, draw_index, 1u) * T;
-    uint64_t u = (uint64_t)(prod >> 64), c = 0;
-    for (uint64_t o = 0; o < norig; ++o) {
-      bool ok;
-      uint64_t ui = to_u(o, &ok);
-      if (!ok) continue;
-      c += Qu[ui];
-      if (c > u) { sel = o; break; }
-    }
+  cudaFreeAsync(d, s->stream);
+  if (e != cudaSuccess) return cuda_fail(err, e, "measurement");
+  if (outcome_out) {
+    uint64_t o = 0;
+    for (size_t k = 0; k < qubits.size(); ++k)
+      if ((pick.val >> (s->n - 1 - qubits[k])) & 1) o |= 1ULL << k;
+    *outcome_out = o;
   }
-  bool ok;
-  uint64_t usel = to_u(sel, &ok);
-  double ps = ok ? Pu[usel] : 0.0;
-  double nf = ps > 0 ? 1.0 / std::sqrt(ps) : 1.0;
-  GOp g;
-  std::memset(&g, 0, sizeof(g));
-  g.kind = OK_COLLAPSE;
-  for (int k = 0; k < m; ++k) {
-    g.mask |= 1ULL << ubits[k];
-    if (ok && ((usel >> k) & 1)) g.val |= 1ULL << ubits[k];
-  }
-  if (!ok) g.val = ~0ULL;  // impossible outcome: everything collapses to zero (never chosen with T > 0)
-  g.m[0] = nf;
-  CK(launch_plain_op(s->d, s->prec, n, g, s->stream), "collapse");
-  if (outcome_out) *outcome_out = sel;
-  if (prob_out) *prob_out = ps;
+  if (prob_out) *prob_out = pick.probability;
   return QG_OK;
 }
 
