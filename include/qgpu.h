@@ -327,7 +327,7 @@ int qg_state_sample(void* state, uint64_t shots, uint64_t seed, uint64_t* host_o
    for callers that cannot allocate while sampling, such as a host runtime that has
    handed every free byte of HBM to its own pool, or a loop that must not take the
    allocator's locks and possible synchronisation on each call. Its scratch is one fixed
-   array per device inside this library (about 4.3 MB), which limits the state to
+   array per device inside this library (about 4.5 MB), which limits the state to
    24 qubits; larger states return QG_ERR_INVALID_ARG. device_outcomes is caller-owned
    device memory of the state's device holding at least `shots` values; the call
    returns after the outcomes are written (it synchronises the state's stream).

@@ -586,8 +586,8 @@ __global__ void k_c64_to_c128(const float2* __restrict__ a, double2* __restrict_
 // chunk (32 amplitudes) and block (256 chunks) sums are exact integers, so the
 // cumulative distribution does not depend on launch shape. A shot draws
 // u = floor(r64 * T / 2^64) from Philox and takes the first i whose cumulative
-// sum exceeds u: block by binary search of the block prefix, chunk by a warp
-// scan of the block's chunk sums, amplitude by a warp scan inside the chunk.
+// sum exceeds u: block by a search of the block prefix, then one of 16 groups of 16
+// chunks, the chunk and the amplitude, each by a scan over lanes.
 // ---------------------------------------------------------------------------
 struct SampleGeom {
   uint64_t N;
@@ -607,135 +607,157 @@ SampleGeom sample_geom(int n) {
   return g;
 }
 
+// floor((re^2 + im^2) 2^62) of a complex64 amplitude, for parts below 2^-10, with eight
+// instructions on the integer pipe (qg_quant62_sq_fast takes 29: it aligns both squares by
+// variable shifts). With x' = |x| 2^41 and X = floor(x'), x'^2 = X^2 + (x' - X)(x' + X). X is a
+// conversion, the squares are two wide multiply-adds, and the second term is zero from 2^-18
+// on (x' is whole there); below, it comes from FP32 in units of z = x' 2^-23 cut off at 1,
+// where zt = floor(z 2^23) 2^-23 is an addition of 1 that rounds to zero. z - zt is exact;
+// z + zt, the product and the sum of both parts round to zero, so that
+//   Sf = X^2 + Y^2 + floor(D) <= p 2^82 < Sf + 9 (per part 2 + 1, the sum 2, the floor 1),
+// and Sf >> 20 is the value unless its fraction and the rounding of the FP64 sum (at most
+// (Sf >> 52) + 4 units, see qg_quant62_fix) reach the next whole number. `worst` is the
+// largest of fraction + (Sf >> 52) and `part` the largest magnitude (NaN stays NaN):
+// the value holds when worst <= kWorstOk and part < 2^-10.
+constexpr uint32_t kWorstOk = (1u << 20) - 16u;
+__device__ __forceinline__ uint64_t quant62_wide(float re, float im, uint32_t& worst, float& part) {
+  using u64 = unsigned long long;
+  auto pk = [](float a, float b) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+  };
+  asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(part) : "f"(re), "f"(im));
+  const uint32_t X = __float2uint_rz(fabsf(re) * 0x1p41f), Y = __float2uint_rz(fabsf(im) * 0x1p41f);
+  const u64 z = pk(__saturatef(fabsf(re) * 0x1p18f), __saturatef(fabsf(im) * 0x1p18f));
+  u64 zp, zt, f, g, d;
+  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(zp) : "l"(z), "l"(pk(1.f, 1.f)));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(zt) : "l"(zp), "l"(pk(-1.f, -1.f)));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(f) : "l"(zp), "l"(pk(-0x1p46f, -0x1p46f)), "l"(pk(0x1p46f, 0x1p46f)));  // -zt 2^46
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(f) : "l"(z), "l"(pk(0x1p46f, 0x1p46f)));
+  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(g) : "l"(z), "l"(zt));
+  asm("mul.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f), "l"(g));
+  float d0, d1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d0), "=f"(d1) : "l"(d));
+  const uint64_t s = (uint64_t)X * X + ((uint64_t)Y * Y + __float2uint_rz(__fadd_rz(d0, d1)));
+  worst = max(worst, ((uint32_t)s & 0xFFFFFu) + (uint32_t)(s >> 52));
+  return s >> 20;
+}
+
 // one CTA (256 threads = 8 warps) per sample block. Only integer sums are formed here:
 // the FP64 total of the normalisation check is derived from them (k_samp_scan). A
 // compensated FP64 reduction per chunk ran on the FP64 pipe (about 1/58 of the FP32
 // rate on this part) and bound the whole sampler by it.
-// Full blocks (256 chunks of 32 amplitudes: states of 13 qubits and more, 16-byte aligned,
-// as every state the runtime allocates): warp w takes the block's chunks 32w .. 32w + 31
-// and reads them with 16-byte loads, eight per lane in flight (one amplitude per lane and
-// load for complex128, two for complex64). Integer sums are associative: every chunk sum
-// equals the lane-per-amplitude form's. The quantised probabilities come from the
-// fixed-point fast path (qg_quant62_sq_fast, no FP64 instruction) wherever its guard
-// allows, and from the FP64 expression (one vote per group of eight loads) where it
-// fails; both give the same integers. Parts of 2^-10 or more fail it, and since the
-// probabilities sum to one, at most 2^20 amplitudes of a state have them. complex128
-// votes on the group's largest part first and sends such groups to the FP64 expression
-// whole; for complex64 that check cost more than it saved (28 qubits: 530 against
-// 585 us per launch, even for a GHZ state). Three CTAs per SM: 80 registers (ptxas
+// Full blocks (256 chunks of 32 amplitudes: states of 13 qubits and more; every state the
+// runtime allocates is aligned to 16 bytes and more): warp w takes the block's chunks 32w ..
+// 32w + 31, four lanes to a chunk, with 16-byte loads, eight per lane in flight (one
+// amplitude per lane and load for complex128, two for complex64). A lane adds up what it
+// holds of a chunk before it exchanges anything: three exchanges per 32 chunks. (With a
+// load spread over one or two whole chunks they were 15 for complex64 and 36 for complex128,
+// of 8 instructions each.) Integer sums are associative: every chunk sum equals the
+// lane-per-amplitude form's. The quantised probabilities come from fixed-point forms without
+// an FP64 instruction (quant62_wide for complex64, qg_quant62_sq_fast for complex128), and,
+// one vote per group of loads, from the FP64 expression where their guards fail; all give the
+// same integers. Parts of 2^-10 or more fail, and since the probabilities sum to one, at most
+// 2^20 amplitudes of a state have them. complex128 votes on the group's largest part first
+// and sends such groups to the FP64 expression whole. Three CTAs per SM: 80 registers (ptxas
 // otherwise picks 64 for complex128 and spills).
+// complex64, 30 qubits: 1547 us, 82 % of the copy rate (1855 us bound by the integer pipe
+// when the squares were aligned by variable shifts, 1994 us with 15 exchanges).
 template <typename R>
 __global__ void __launch_bounds__(256, 3) k_samp_sums(const typename C2<R>::T* __restrict__ s, SampleGeom g,
                                                    unsigned long long* __restrict__ csum,
+                                                   unsigned long long* __restrict__ gsum,
                                                    unsigned long long* __restrict__ bsum) {
   using T = typename C2<R>::T;
   constexpr int A = 16 / (int)sizeof(T);  // amplitudes per 16-byte load
-  constexpr int CL = 32 / A;              // lanes per chunk
-  constexpr int LOADS = 32 / A;           // loads per lane for the warp's 32 chunks
-  constexpr int U = 8;                    // loads in flight per lane
+  constexpr int L = 4;                    // lanes per chunk
+  constexpr int CPR = 32 / L;             // chunks per round of the warp
+  constexpr int LOADS = 32 / (A * L);     // loads per lane and chunk
+  constexpr int U = A == 2 ? 8 : 4;       // loads in flight per lane (8 spill for complex128)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ unsigned long long wq[8];
   for (uint64_t b = blockIdx.x; b < g.nb; b += gridDim.x) {
     unsigned long long bq = 0;
-    if (g.ch == 32 && g.cpb == 256 && (reinterpret_cast<uintptr_t>(s) & 15u) == 0) {
+    if (g.cpb == 256) {
       const uint64_t c0 = b * 256 + (uint64_t)warp * 32;  // the warp's first chunk
-      const uint4* src = reinterpret_cast<const uint4*>(s + c0 * 32);
-      if constexpr (A == 2) {
-        // complex64: load u gives lane L amplitudes 64u + 2L, +1 (chunk 2u + L / 16), so
-        // each half-warp holds one partial per chunk of its parity; recursive halving
-        // (each step a lane sends the half of its partials it does not keep) leaves lane
-        // l of half h the sum of chunk 2l + h after 15 exchanges for all 32 chunks
-        unsigned long long w[LOADS];
+      const uint4* src = reinterpret_cast<const uint4*>(s + (c0 + (uint64_t)(lane / L)) * 32) + lane % L;
+      uint64_t w[L];  // round k: chunk CPR k + lane / L
 #pragma unroll
-        for (int i0 = 0; i0 < LOADS; i0 += U) {
-          uint4 v[U];
+      for (int k = 0; k < L; ++k) w[k] = 0;
 #pragma unroll
-          for (int u = 0; u < U; ++u) v[u] = __ldg(src + (i0 + u) * 32 + lane);
-          unsigned slow = 0;
+      for (int i0 = 0; i0 < L * LOADS; i0 += U) {
+        uint4 v[U];
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            uint64_t q0, q1;
-            const bool f0 = qg_quant62_sq_fast(__uint_as_float(v[u].x), __uint_as_float(v[u].y), &q0);
-            const bool f1 = qg_quant62_sq_fast(__uint_as_float(v[u].z), __uint_as_float(v[u].w), &q1);
-            w[i0 + u] = q0 + q1;
-            slow |= (unsigned)!(f0 && f1) << u;
-          }
-          if (__any_sync(0xffffffffu, slow)) {  // the FP64 expression
+        for (int u = 0; u < U; ++u)
+          v[u] = __ldg(src + (i0 + u) / LOADS * (CPR * 32 / A) + (i0 + u) % LOADS * L);
+        uint64_t q[U];
+        unsigned slow = 0;
+        if constexpr (A == 2) {
+          uint32_t worst = 0;
+          float part = 0.f;
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (slow & (1u << u)) {
-                const float2 x0 = make_float2(__uint_as_float(v[u].x), __uint_as_float(v[u].y));
-                const float2 x1 = make_float2(__uint_as_float(v[u].z), __uint_as_float(v[u].w));
-                w[i0 + u] = quant(p_of<R>(x0)) + quant(p_of<R>(x1));
-              }
-          }
-        }
-#pragma unroll
-        for (int o = 8, K = LOADS; o >= 1; o >>= 1, K >>= 1) {
-          const bool up = (lane & o) != 0;
-#pragma unroll
-          for (int i = 0; i < K / 2; ++i) {
-            const unsigned long long send = up ? w[i] : w[i + K / 2];
-            const unsigned long long keep = up ? w[i + K / 2] : w[i];
-            w[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-          }
-        }
-        csum[c0 + 2 * (uint64_t)(lane & 15) + (uint64_t)(lane >> 4)] = w[0];
-        bq = w[0];
-      } else {
-#pragma unroll
-        for (int i0 = 0; i0 < LOADS; i0 += U) {
-          uint4 v[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) v[u] = __ldg(src + (i0 + u) * 32 + lane);
-          uint64_t qs[U];
+          for (int u = 0; u < U; ++u)
+            q[u] = quant62_wide(__uint_as_float(v[u].x), __uint_as_float(v[u].y), worst, part) +
+                   quant62_wide(__uint_as_float(v[u].z), __uint_as_float(v[u].w), worst, part);
+          if (!(worst <= kWorstOk && part < 0x1p-10f)) slow = (1u << U) - 1;
+        } else {
           bool big = false;
 #pragma unroll
           for (int u = 0; u < U; ++u)  // high words: sign, exponent, top of the significand
             big |= max(v[u].y & 0x7FFFFFFFu, v[u].w & 0x7FFFFFFFu) >= (1013u << 20);
-          unsigned slow = (1u << U) - 1;
+          slow = (1u << U) - 1;
           if (!__any_sync(0xffffffffu, big)) {
             slow = 0;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
               const bool f = qg_quant62_sq_fast(__hiloint2double((int)v[u].y, (int)v[u].x),
-                                                __hiloint2double((int)v[u].w, (int)v[u].z), &qs[u]);
+                                                __hiloint2double((int)v[u].w, (int)v[u].z), &q[u]);
               slow |= (unsigned)!f << u;
             }
           }
-          if (__any_sync(0xffffffffu, slow)) {  // the FP64 expression
+        }
+        if (__any_sync(0xffffffffu, slow)) {  // the FP64 expression
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (slow & (1u << u)) {
+          for (int u = 0; u < U; ++u)
+            if (slow & (1u << u)) {
+              if constexpr (A == 2) {
+                const float2 x0 = make_float2(__uint_as_float(v[u].x), __uint_as_float(v[u].y));
+                const float2 x1 = make_float2(__uint_as_float(v[u].z), __uint_as_float(v[u].w));
+                uint64_t q0, q1;
+                if (!qg_quant62_sq_fast(x0.x, x0.y, &q0)) q0 = quant(p_of<R>(x0));
+                if (!qg_quant62_sq_fast(x1.x, x1.y, &q1)) q1 = quant(p_of<R>(x1));
+                q[u] = q0 + q1;
+              } else {
                 const double2 x = make_double2(__hiloint2double((int)v[u].y, (int)v[u].x),
                                                __hiloint2double((int)v[u].w, (int)v[u].z));
-                qs[u] = quant(p_of<R>(x));
+                q[u] = quant(p_of<R>(x));
               }
-          }
-          // load u holds chunk i0 + u across the warp: recursive halving over lane bits 4,
-          // 3, 2 (7 exchanges) leaves lane l a partial of chunk i0 + ((l >> 2) & 7), and two
-          // butterfly steps over bits 1, 0 complete it (5 exchanges per chunk before)
-#pragma unroll
-          for (int o = 16, K = U; o >= 4; o >>= 1, K >>= 1) {
-            const bool up = (lane & o) != 0;
-#pragma unroll
-            for (int i = 0; i < K / 2; ++i) {
-              const uint64_t send = up ? qs[i] : qs[i + K / 2];
-              const uint64_t keep = up ? qs[i + K / 2] : qs[i];
-              qs[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
-          }
-          unsigned long long q = qs[0];
-          q += __shfl_xor_sync(0xffffffffu, q, 2);
-          q += __shfl_xor_sync(0xffffffffu, q, 1);
-          if ((lane & 3) == 0) {
-            csum[c0 + (uint64_t)(i0 + ((lane >> 2) & 7))] = q;
-            bq += q;
-          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[(i0 + u) / LOADS] += q[u];
+      }
+      // recursive halving (each step a lane sends the half of its partials it does not
+      // keep): lane l ends with the sum of chunk CPR (l % L) + l / L
+#pragma unroll
+      for (int o = L / 2, K = L; o >= 1; o >>= 1, K >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < K / 2; ++i) {
+          const uint64_t send = up ? w[i] : w[i + K / 2];
+          const uint64_t keep = up ? w[i + K / 2] : w[i];
+          w[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
       }
+      csum[c0 + (uint64_t)(CPR * (lane % L) + lane / L)] = w[0];
+      bq = w[0];
+      // the sums of 16 chunks: the lanes of one value of bit 1
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) bq += __shfl_xor_sync(0xffffffffu, bq, o);
+      for (int o : {1, 4, 8, 16}) bq += __shfl_xor_sync(0xffffffffu, bq, o);
+      if ((lane & 29) == 0) gsum[c0 / 16 + (uint64_t)(lane >> 1)] = bq;
+      bq += __shfl_xor_sync(0xffffffffu, bq, 2);
     } else {
       for (int c = warp; c < g.cpb; c += 8) {
         uint64_t chunk = b * g.cpb + c;
@@ -759,140 +781,230 @@ __global__ void __launch_bounds__(256, 3) k_samp_sums(const typename C2<R>::T* _
   }
 }
 
-// single CTA: exclusive prefix of block sums (bpre[nb] = T) and the FP64 total
+// Exclusive prefix of block sums (bpre[nb] = T) and the FP64 total
 // T 2^-62 + N 2^-63: every quantised probability lost less than one unit of
 // 2^-62 to the floor, so the estimate is within N 2^-63 of sum p (2e-9 at 34
-// qubits, well inside the 1e-8 normalisation tolerance). Latency-bound: each thread adds up
-// 16 consecutive sums, one warp-shuffle scan covers 16384 of them (30 qubits, 2^17 sums:
-// 228 us with a 1024-entry scan in shared memory per step).
-constexpr int kScanPer = 16;
-__global__ void __launch_bounds__(1024) k_samp_scan(const unsigned long long* __restrict__ bsum, uint64_t nb,
+// qubits, well inside the 1e-8 normalisation tolerance). Latency-bound: a CTA takes 8192 sums,
+// eight rows of 1024, through warp shuffles; with more than that (27 qubits and up) each CTA
+// leaves its total in place of its first sum and k_samp_scan_add adds up those before it
+// (30 qubits, 2^17 sums: 11 us; one CTA in 16 steps 93 us, 138 us with 16 consecutive sums
+// per thread, whose loads and stores touch a line per lane, 228 us with a 1024-entry scan in
+// shared memory per step).
+constexpr int kScanRows = 8;
+constexpr uint64_t kScanStep = 1024 * kScanRows;
+__device__ __forceinline__ void scan_end(unsigned long long T, uint64_t n_amps, uint64_t nb,
+                                         unsigned long long* bpre, double* total) {
+  total[0] = (double)T * 0x1p-62 + (double)n_amps * 0x1p-63;
+  bpre[nb] = T;
+}
+__global__ void __launch_bounds__(1024) k_samp_scan(unsigned long long* __restrict__ bsum, uint64_t nb,
                                                     uint64_t n_amps, unsigned long long* __restrict__ bpre,
                                                     double* __restrict__ total) {
-  __shared__ unsigned long long wsum[2][32];
+  __shared__ unsigned long long wsum[kScanRows][32], wpre[kScanRows][32], rows[kScanRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long carry = 0;
-  int par = 0;
-  for (uint64_t base = 0; base < nb; base += 1024 * kScanPer, par ^= 1) {
-    const uint64_t i0 = base + (uint64_t)threadIdx.x * kScanPer;
-    unsigned long long v[kScanPer], mine = 0;
+  const uint64_t base = blockIdx.x * kScanStep + threadIdx.x;
+  unsigned long long v[kScanRows], incl[kScanRows], carry = 0;
 #pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-      v[k] = i0 + k < nb ? bsum[i0 + k] : 0ULL;
-      mine += v[k];
+  for (int k = 0; k < kScanRows; ++k) {
+    const uint64_t i = base + (uint64_t)k * 1024;
+    incl[k] = v[k] = i < nb ? bsum[i] : 0ULL;
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+    for (int k = 0; k < kScanRows; ++k) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, incl[k], o);
+      if (lane >= o) incl[k] += up;
+    }
+  if (lane == 31)
+#pragma unroll
+    for (int k = 0; k < kScanRows; ++k) wsum[k][warp] = incl[k];
+  __syncthreads();
+  if (warp < kScanRows) {  // warp w scans the warp sums of row w
+    const unsigned long long x = wsum[warp][lane];
+    unsigned long long s = x;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += up;
+    }
+    wpre[warp][lane] = s - x;
+    if (lane == 31) rows[warp] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kScanRows; ++k) {
+    const uint64_t i = base + (uint64_t)k * 1024;
+    if (i < nb) bpre[i] = carry + wpre[k][warp] + incl[k] - v[k];
+    carry += rows[k];
+  }
+  if (threadIdx.x == 0) {
+    if (gridDim.x == 1) scan_end(carry, n_amps, nb, bpre, total);
+    else bsum[base] = carry;
+  }
+}
+// CTA c adds the totals of the CTAs before it (nb = gridDim.x * kScanStep, 256 CTAs at most)
+__global__ void __launch_bounds__(1024) k_samp_scan_add(const unsigned long long* __restrict__ bsum, uint64_t nb,
+                                                        uint64_t n_amps, unsigned long long* __restrict__ bpre,
+                                                        double* __restrict__ total) {
+  __shared__ unsigned long long part[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long before = threadIdx.x < blockIdx.x ? bsum[(uint64_t)threadIdx.x * kScanStep] : 0ULL;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (lane == 0) part[warp] = before;
+  __syncthreads();
+  before = part[lane];
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  const uint64_t base = blockIdx.x * kScanStep + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kScanRows; ++k) bpre[base + (uint64_t)k * 1024] += before;
+  if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1)
+    scan_end(before + bsum[(uint64_t)blockIdx.x * kScanStep], n_amps, nb, bpre, total);
+}
+
+// States below 13 qubits (one block of at most 128 chunks): one warp per shot, up to four
+// consecutive chunk sums per lane.
+template <typename R>
+__global__ void __launch_bounds__(256) k_samp_resolve_small(const typename C2<R>::T* __restrict__ s, SampleGeom g,
+                                                            const unsigned long long* __restrict__ csum,
+                                                            const unsigned long long* __restrict__ bpre,
+                                                            uint64_t shots, uint64_t seed,
+                                                            uint64_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t stride = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const unsigned long long T = bpre[g.nb];
+  const int per = (g.cpb + 31) / 32;
+  for (uint64_t k = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < shots; k += stride) {
+    if (T == 0) {
+      if (lane == 0) out[k] = 0;
+      continue;
+    }
+    const unsigned long long r = __umul64hi(draw64(seed, k, 0u), T);
+    unsigned long long loc[4], mine = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      loc[c] = c < per && lane * per + c < g.cpb ? csum[lane * per + c] : 0ULL;
+      mine += loc[c];
     }
     unsigned long long incl = mine;
     for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += up;
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
     }
-    if (lane == 31) wsum[par][warp] = incl;
-    __syncthreads();  // the other half of wsum is written in the next round: one barrier each
-    unsigned long long all = wsum[par][lane], before = lane < warp ? all : 0ULL;
-    for (int o = 16; o > 0; o >>= 1) {
-      before += __shfl_xor_sync(0xffffffffu, before, o);
-      all += __shfl_xor_sync(0xffffffffu, all, o);
-    }
-    unsigned long long at = carry + before + incl - mine;
+    // the owner's first chunk whose cumulative sum exceeds r (the last one where sums of infinite
+    // amplitudes wrapped)
+    const int owner = __ffs((int)(__ballot_sync(0xffffffffu, incl > r) | 0x80000000u)) - 1;
+    unsigned long long before = incl - mine;
+    int chunk = lane * per;
 #pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-      if (i0 + k < nb) bpre[i0 + k] = at;
-      at += v[k];
+    for (int c = 0; c < 3; ++c)
+      if (chunk == lane * per + c && c < per - 1 && before + loc[c] <= r) {
+        before += loc[c];
+        ++chunk;
+      }
+    chunk = __shfl_sync(0xffffffffu, chunk < g.cpb ? chunk : g.cpb - 1, owner);
+    before = __shfl_sync(0xffffffffu, before, owner);
+    unsigned long long qi = lane < g.ch ? quant(p_of<R>(s[chunk * g.ch + lane])) : 0ULL;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, qi, o);
+      if (lane >= o) qi += v;
     }
-    carry += all;
-  }
-  if (threadIdx.x == 0) {
-    total[0] = (double)carry * 0x1p-62 + (double)n_amps * 0x1p-63;
-    bpre[nb] = carry;
+    const unsigned hit = __ballot_sync(0xffffffffu, lane < g.ch && before + qi > r);
+    const int pick = hit ? __ffs((int)hit) - 1 : g.ch - 1;
+    if (lane == 0) out[k] = (uint64_t)chunk * g.ch + pick;
   }
 }
 
-// One warp per shot, `batch` (1..32) shots one after the other with their draws computed
-// side by side. The block is found 32 ways at a time (2^17 blocks: four dependent loads; a
-// binary search made 17), its chunk by a scan of the block's 256 sums, 64 bytes per lane, the
-// amplitude by a scan of the chunk. Bound by the latency of these loads (30 qubits, 10^6
-// shots: 977 us with the binary search and one Philox draw per lane and shot).
+// Half a warp per shot, `batch` (1..16) shots one after the other with their draws computed
+// side by side. The block is found 16 ways at a time among (up to) 4096 evenly spaced
+// prefixes that each CTA keeps in shared memory, every level of that tree packed, and from
+// there 32 ways in bpre, where 2^17 blocks leave 32 consecutive prefixes. The chunk comes
+// from the sums of 16 chunks and then the chunks' own, the amplitude from a scan of the
+// chunk, all contiguous. Bound by instruction issue and the latency of scattered reads (30
+// qubits, 10^6 shots: 977 us with a binary search and one Philox draw per lane and shot, 727 us
+// with 32-way steps through bpre, a line per lane, and all 256 chunk sums of the block read,
+// 441 us with a warp per shot, 283 us).
+constexpr int kTop = 4096;
 template <typename R>
-__global__ void __launch_bounds__(256) k_samp_resolve(const typename C2<R>::T* __restrict__ s, SampleGeom g,
-                                                      const unsigned long long* __restrict__ csum,
-                                                      const unsigned long long* __restrict__ bpre, uint64_t shots,
-                                                      uint64_t seed, int batch, uint64_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t stride = (((uint64_t)gridDim.x * blockDim.x) >> 5) * (uint64_t)batch;
+__global__ void __launch_bounds__(512, 3) k_samp_resolve(const typename C2<R>::T* __restrict__ s, SampleGeom g,
+                                                         const unsigned long long* __restrict__ csum,
+                                                         const unsigned long long* __restrict__ gsum,
+                                                         const unsigned long long* __restrict__ bpre, uint64_t shots,
+                                                         uint64_t seed, int batch, uint64_t* __restrict__ out) {
+  // top[i] = bpre at the end of the i-th of `tops` equal runs of blocks; mid and head hold
+  // every 16th entry of the level below (entries past the end read T)
+  __shared__ unsigned long long top[kTop], mid[kTop / 16], head[16];
+  const int lane = threadIdx.x & 15, half = threadIdx.x & 16;
   const unsigned long long T = bpre[g.nb];
-  const int per = (g.cpb + 31) / 32;
-  for (uint64_t first = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (uint64_t)batch; first < shots;
-       first += stride) {
-    const int cnt = (int)(shots - first < (uint64_t)batch ? shots - first : (uint64_t)batch);
-    if (T == 0) {
-      if (lane < cnt) out[first + lane] = 0;
-      continue;
+  const int tops = (int)(g.nb < kTop ? g.nb : kTop);  // a power of two, as g.nb
+  const uint64_t run = g.nb / (uint64_t)tops;
+  for (int i = threadIdx.x; i < tops; i += blockDim.x) top[i] = bpre[(uint64_t)(i + 1) * run];
+  __syncthreads();
+  if (tops > 16) {
+    if (threadIdx.x < kTop / 16) mid[threadIdx.x] = threadIdx.x < tops / 16 ? top[16 * threadIdx.x + 15] : T;
+    if (threadIdx.x < 16) head[threadIdx.x] = threadIdx.x < tops / 256 ? top[256 * threadIdx.x + 255] : T;
+    __syncthreads();
+  }
+  auto vote = [&](bool p) { return (__ballot_sync(0xffffffffu, p) >> half) & 0xffffu; };
+  // the last lane without a hit: sums that wrapped (infinite amplitudes) stay in bounds
+  auto first_of = [&](bool p) { return __ffs((int)(vote(p) | 0x8000u)) - 1; };
+  auto scan = [&](unsigned long long v) {  // inclusive, over the half-warp
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, v, o, 16);
+      if (lane >= o) v += up;
     }
+    return v;
+  };
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t at = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2 * batch; at < shots;
+       at += warps * 2 * batch) {
+    const uint64_t first = at + (half ? (uint64_t)batch : 0);
+    const int cnt = first >= shots ? 0 : (int)(shots - first < (uint64_t)batch ? shots - first : (uint64_t)batch);
+    const int most = (int)(shots - at < (uint64_t)batch ? shots - at : (uint64_t)batch);  // the lower half's count
     unsigned long long draw = 0, picked = 0;
     if (lane < cnt) draw = __umul64hi(draw64(seed, first + lane, 0u), T);
-    for (int q = 0; q < cnt; ++q) {
-      const unsigned long long u = __shfl_sync(0xffffffffu, draw, q);
-      // block: first b with bpre[b + 1] > u; bpre[nb] = T > u
-      uint64_t b = 0, len = g.nb;
-      while (len > 1) {
-        const uint64_t step = (len + 31) >> 5, at = (uint64_t)(lane + 1) * step;
-        const unsigned hit = __ballot_sync(0xffffffffu, bpre[b + (at < len ? at : len)] > u);
-        const uint64_t skip = (uint64_t)(__ffs((int)hit) - 1) * step;
-        b += skip;
-        len = len - skip < step ? len - skip : step;
-      }
-      const unsigned long long r = u - bpre[b];
-      // chunk within block: cpb <= 256 chunk sums, 8 per lane
-      unsigned long long loc[8];
-      unsigned long long mine = 0;
-      if (g.cpb == 256) {
-        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(csum + b * 256) + lane * 4;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const ulonglong2 x = src[k];
-          loc[2 * k] = x.x;
-          loc[2 * k + 1] = x.y;
+    if (T != 0)
+      for (int q = 0; q < most; ++q) {  // past its count the upper half looks for 0
+        const unsigned long long u = __shfl_sync(0xffffffffu, draw, q, 16);
+        // block: first b with bpre[b + 1] > u; bpre[nb] = T > u, so every vote has a winner
+        int t = 0;
+        if (tops > 256) t = first_of(head[lane] > u);
+        if (tops > 16) t = 16 * t + first_of(mid[16 * t + lane] > u);
+        t = 16 * t + first_of(lane >= tops || top[16 * t + lane] > u);
+        uint64_t b = (uint64_t)t * run, len = run;
+        while (len > 1) {  // 32 ways, two per lane; len is a power of two
+          const uint64_t step = (len + 31) >> 5, to = (uint64_t)(2 * lane + 1) * step;
+          const unsigned odd = vote(bpre[b + (to < len ? to : len)] > u);
+          const int l = first_of(bpre[b + (to + step < len ? to + step : len)] > u);
+          b += (uint64_t)(2 * l + 1 - (int)((odd >> l) & 1u)) * step;
+          len = step;
         }
-      } else {
+        unsigned long long r = u - bpre[b];
+        // one of 16 groups of 16 chunks, then the chunk: two lines of memory instead of 2 KB
+        uint64_t chunk = b * 16;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int c = lane * per + k;
-          loc[k] = k < per && c < g.cpb ? csum[b * g.cpb + c] : 0ULL;
+        for (int level = 0; level < 2; ++level) {
+          const unsigned long long mine = (level == 0 ? gsum : csum)[chunk + lane], incl = scan(mine);
+          const int owner = first_of(incl > r);
+          r -= __shfl_sync(0xffffffffu, incl - mine, owner, 16);
+          chunk += owner;
+          if (level == 0) chunk *= 16;
         }
-      }
+        // its 32 amplitudes, two per lane: the fixed-point path as in k_samp_sums, the FP64
+        // expression past its guard
+        unsigned long long qa[2];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) mine += loc[k];
-      unsigned long long incl = mine;
-      for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const unsigned ballot = __ballot_sync(0xffffffffu, incl > r);
-      const int owner = ballot ? __ffs(ballot) - 1 : 31;
-      // the owner's first chunk whose cumulative sum exceeds r (its last one otherwise)
-      unsigned long long before = incl - mine;
-      int kk = 0;
-#pragma unroll
-      for (int k = 0; k < 7; ++k)
-        if (kk == k && k < per - 1 && before + loc[k] <= r) {
-          before += loc[k];
-          kk = k + 1;
+        for (int e = 0; e < 2; ++e) {
+          const typename C2<R>::T a = s[chunk * 32 + 2 * lane + e];
+          uint64_t x;
+          if (!qg_quant62_sq_fast(a.x, a.y, &x)) x = quant(p_of<R>(a));
+          qa[e] = x;
         }
-      int chunk_in_block = lane * per + kk;
-      if (chunk_in_block >= g.cpb) chunk_in_block = g.cpb - 1;
-      chunk_in_block = __shfl_sync(0xffffffffu, chunk_in_block, owner);
-      before = __shfl_sync(0xffffffffu, before, owner);
-      const unsigned long long r2 = r - before;
-      const uint64_t chunk = b * g.cpb + chunk_in_block;
-      unsigned long long qi = lane < g.ch ? quant(p_of<R>(s[chunk * g.ch + lane])) : 0ULL;
-      for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long v = __shfl_up_sync(0xffffffffu, qi, o);
-        if (lane >= o) qi += v;
+        const unsigned long long incl = scan(qa[0] + qa[1]);
+        const unsigned even = vote(incl - qa[1] > r);
+        const int l = first_of(incl > r);
+        if (lane == q) picked = chunk * 32 + 2 * l + 1 - ((even >> l) & 1u);
       }
-      const unsigned bl = __ballot_sync(0xffffffffu, (lane < g.ch) && qi > r2);
-      const int pick = bl ? __ffs(bl) - 1 : g.ch - 1;
-      if (lane == q) picked = chunk * g.ch + pick;
-    }
     if (lane < cnt) out[first + lane] = picked;
   }
 }
@@ -1158,29 +1270,42 @@ cudaError_t launch_sample(const void* s, int precision, int n, uint64_t shots, u
                           uint64_t* d_outcomes, double* d_total, cudaStream_t st) {
   SampleGeom g = sample_geom(n);
   unsigned long long* csum = (unsigned long long*)d_scratch;
-  unsigned long long* bsum = csum + g.nchunks;
+  unsigned long long* gsum = csum + g.nchunks;
+  unsigned long long* bsum = gsum + 16 * g.nb;
   unsigned long long* bpre = bsum + g.nb;
   int grid = (int)(g.nb < (uint64_t)kSMs * 8 ? g.nb : (uint64_t)kSMs * 8);
   if (precision == QG_C64)
-    k_samp_sums<float><<<grid, 256, 0, st>>>((const float2*)s, g, csum, bsum);
+    k_samp_sums<float><<<grid, 256, 0, st>>>((const float2*)s, g, csum, gsum, bsum);
   else
-    k_samp_sums<double><<<grid, 256, 0, st>>>((const double2*)s, g, csum, bsum);
+    k_samp_sums<double><<<grid, 256, 0, st>>>((const double2*)s, g, csum, gsum, bsum);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_samp_scan<<<1, 1024, 0, st>>>(bsum, g.nb, g.N, bpre, d_total);
+  const unsigned scans = (unsigned)((g.nb + kScanStep - 1) / kScanStep);
+  k_samp_scan<<<scans, 1024, 0, st>>>(bsum, g.nb, g.N, bpre, d_total);
+  if (scans > 1) k_samp_scan_add<<<scans, 1024, 0, st>>>(bsum, g.nb, g.N, bpre, d_total);
   e = cudaGetLastError();
-  counted(2);
+  counted(scans > 1 ? 3 : 2);
   if (e != cudaSuccess || shots == 0) return e;
-  const uint64_t most = (uint64_t)kSMs * 16 * 8;  // warps of a full grid
-  const int batch = (int)std::min<uint64_t>(32, (shots + most - 1) / most);
-  const uint64_t warps_needed = (shots + batch - 1) / batch;
-  const uint64_t blocks = std::min<uint64_t>((warps_needed + 7) / 8, (uint64_t)kSMs * 16);
-  if (precision == QG_C64)
-    k_samp_resolve<float><<<(unsigned)blocks, 256, 0, st>>>((const float2*)s, g, csum, bpre, shots, seed, batch,
-                                                            d_outcomes);
-  else
-    k_samp_resolve<double><<<(unsigned)blocks, 256, 0, st>>>((const double2*)s, g, csum, bpre, shots, seed, batch,
-                                                             d_outcomes);
+  if (g.cpb < 256) {
+    const unsigned blocks = (unsigned)std::min<uint64_t>((shots + 7) / 8, (uint64_t)kSMs * 8);
+    if (precision == QG_C64)
+      k_samp_resolve_small<float><<<blocks, 256, 0, st>>>((const float2*)s, g, csum, bpre, shots, seed, d_outcomes);
+    else
+      k_samp_resolve_small<double><<<blocks, 256, 0, st>>>((const double2*)s, g, csum, bpre, shots, seed, d_outcomes);
+  } else {
+    // equal batches of at most 16 in whole rounds of the grid (three CTAs of 32 half-warps per SM)
+    const uint64_t most = (uint64_t)kSMs * 3 * 32, round = 16 * most;
+    const uint64_t rounds = std::max<uint64_t>(1, (shots + round - 1) / round);
+    const int batch = (int)std::max<uint64_t>(1, (shots + rounds * most - 1) / (rounds * most));
+    const uint64_t halves = (shots + batch - 1) / batch;
+    const unsigned blocks = (unsigned)std::min<uint64_t>((halves + 31) / 32, (uint64_t)kSMs * 3);
+    if (precision == QG_C64)
+      k_samp_resolve<float><<<blocks, 512, 0, st>>>((const float2*)s, g, csum, gsum, bpre, shots, seed, batch,
+                                                    d_outcomes);
+    else
+      k_samp_resolve<double><<<blocks, 512, 0, st>>>((const double2*)s, g, csum, gsum, bpre, shots, seed, batch,
+                                                     d_outcomes);
+  }
   counted();
   return cudaGetLastError();
 }

@@ -487,15 +487,15 @@ cudaError_t launch_density(const void* s, int precision, int n, double* d_rho, c
 
 // Hierarchical shot sampler. Scratch sized by sampler_scratch_bytes(); its layout:
 // chunks of min(2^n, 32) amplitudes, blocks of min(chunks, 256) chunks, then one u64
-// sum per chunk, one u64 sum per block, the blocks' exclusive prefixes plus a total,
-// and FP64 per-block sums plus two (compensated total), with 256 bytes of slack.
+// sum per chunk, sixteen per block (16 chunks each, blocks of 256 chunks), one per block
+// and the blocks' exclusive prefixes plus a total, with 256 bytes of slack.
 constexpr size_t sampler_scratch_bytes_at(int n) {
   const uint64_t N = 1ULL << n;
   const uint64_t ch = N < 32 ? N : 32;
   const uint64_t nch = N / ch;
   const uint64_t cpb = nch < 256 ? nch : 256;
   const uint64_t nb = nch / cpb;
-  return sizeof(unsigned long long) * (nch + nb + (nb + 1)) + sizeof(double) * (nb + 2) + 256;
+  return sizeof(unsigned long long) * (nch + 16 * nb + nb + (nb + 1)) + 256;
 }
 size_t sampler_scratch_bytes(int n, uint64_t shots);
 cudaError_t launch_sample(const void* s, int precision, int n, uint64_t shots, uint64_t seed, void* d_scratch,

@@ -56,6 +56,16 @@ QG_QHD uint32_t qg_bits_of(float f) {
   return b;
 #endif
 }
+// v >> r, 0 from r = 64 on (shr clamps its count; C++ leaves that undefined)
+QG_QHD uint64_t qg_shr64(uint64_t v, unsigned r) {
+#if defined(__CUDA_ARCH__)
+  uint64_t o;
+  asm("shr.u64 %0, %1, %2;" : "=l"(o) : "l"(v), "r"(r));
+  return o;
+#else
+  return r > 63u ? 0ull : v >> r;
+#endif
+}
 QG_QHD int qg_clz64(uint64_t v) {  // v != 0
 #if defined(__CUDA_ARCH__)
   return __clzll((long long)v);
@@ -117,8 +127,7 @@ QG_QHD uint64_t qg_sq_fix(float x, bool* big) {
   *big = u >= (117u << 23);
   const uint32_t m7 = ((u << 7) & 0x3FFFFF80u) | 0x40000000u;
   const uint64_t M = (uint64_t)m7 * m7;
-  const unsigned r = 232u - 2u * (u >> 23);  // wraps above 63 when *big: any value then
-  return M >> (r < 63u ? r : 63u);           // M < 2^62: a shift by 63 leaves 0
+  return qg_shr64(M, 232u - 2u * (u >> 23));  // the count wraps above 63 when *big: any value then
 }
 
 // floor(x^2 2^82) for a double with |x| < 2^-10 (*big set otherwise), truncated from
@@ -130,8 +139,7 @@ QG_QHD uint64_t qg_sq_fix(double x, bool* big) {
   *big = e > 1012;
   const uint64_t m11 = (b << 11) | 0x8000000000000000ull;
   const uint64_t hi = qg_umulhi(m11, m11);
-  const unsigned r = 2026u - 2u * (unsigned)e;  // wraps above 63 when *big: any value then
-  return r > 63u ? 0ull : (hi >> r);             // hi >= 2^62: shifts of 64 and more give 0
+  return qg_shr64(hi, 2026u - 2u * (unsigned)e);  // the count wraps above 63 when *big: any value then
 }
 
 // The fixed-point sum and its guard: *q = floor(p 2^62) when the result is true.

@@ -2503,7 +2503,7 @@ static int st_sample_sums(State* s, uint64_t* h_csum, uint64_t count, uint64_t* 
   CK(launch_sample(s->d, s->prec, s->n, 0, 0, d_scratch, nullptr, d_total, s->stream), "sample sums");
   const uint64_t* d_q = (const uint64_t*)d_scratch;
   CK(cudaMemcpyAsync(h_csum, d_q, sizeof(uint64_t) * nch, cudaMemcpyDeviceToHost, s->stream), "D2H chunk sums");
-  CK(cudaMemcpyAsync(h_total, d_q + nch + nb + nb, sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream),
+  CK(cudaMemcpyAsync(h_total, d_q + nch + 16 * nb + nb + nb, sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream),
      "D2H total");
   CK(cudaStreamSynchronize(s->stream), "sync");
   cudaFreeAsync(d_scratch, s->stream);

@@ -83,3 +83,53 @@ def test_sweep_energies_over_chunk_counts(precision, tol):
                         sign *= 1 - 2 * ((i >> (n - 1 - q)) & 1)
                 want += t["coefficient"] * float(np.dot(sign, p))
             assert abs(got[c] - want) <= tol * 5
+
+
+def test_same_draws_over_every_depth_of_the_block_search():
+    """Uniform states of 1, 32, 64, 1024, 2048, 4096, 8192 and 2^18 blocks: one to three packed
+    levels of the search and none, one or two steps below them. T = 2^62 for each, so shot k
+    picks the same leading index bits for all of them."""
+    from qclojure_gb300.state import Context
+
+    want = None
+    with Context() as ctx:
+        for n in (13, 18, 19, 23, 24, 25, 26, 31):
+            with ctx.state(n, "c64") as st:
+                st.apply({"num-qubits": n, "operations": [{"operation-type": "h", "operation-params": {"target": q}}
+                                                          for q in range(n)]})
+                got = st.sample(3001, 9) >> np.uint64(n - 13)
+            want = got if want is None else want
+            assert np.array_equal(got, want)
+
+
+def test_complex64_sums_over_the_fixed_point_range():
+    """Chunk sums of complex64 parts from 2^-149 to just below 2^-10 (whole warps stay on the
+    fixed-point path): around 2^-18 and 2^-41, where its terms vanish, powers of two, zeros;
+    then chunks with a part at 2^-10, a NaN and an infinity. Integers: no tolerance."""
+    from qclojure_gb300.state import Context
+
+    rng = np.random.default_rng(5)
+    N = 1 << 16
+    v = np.exp2(rng.uniform(-46, -10, (N, 2))).astype(np.float32)
+    v[:8192] = np.exp2(-18.0) * (1 + rng.integers(-40, 41, (8192, 2)) * 2.0**-24)
+    v[8192:16384] = np.exp2(-41.0) * (1 + rng.integers(-40, 41, (8192, 2)) * 2.0**-24)
+    v[16384:24576] = np.exp2(rng.integers(-149, -10, (8192, 2)).astype(np.float64))
+    v[24576:28672, 0] = 0
+    v = np.minimum(v, np.nextafter(np.float32(2.0**-10), np.float32(0)))
+    v *= rng.choice([np.float32(-1), np.float32(1)], (N, 2))
+    v[40000, 1] = 2.0**-10
+    a = v.view(np.complex64).ravel()
+    with Context() as ctx, ctx.state(16, "c64") as st:
+        for special in (None, np.nan, np.inf):
+            if special is not None:
+                a = a.copy()
+                a[50000] = special
+            st.upload(a.astype(np.complex128))
+            got, total = st.sample_sums()
+            with np.errstate(invalid="ignore", over="ignore"):
+                w = st.download().astype(np.complex128)
+                p = w.real * w.real + w.imag * w.imag
+                q = [0 if x != x else min(int(x * 2.0**62) if x < 4 else 2**64 - 1, 2**64 - 1) for x in p]
+            want = [sum(q[c:c + 32]) % 2**64 for c in range(0, N, 32)]
+            assert got.tolist() == want
+            assert total == sum(want) % 2**64
