@@ -296,7 +296,8 @@ extern "C" int qg_noisy_run(void* ctx, const qg_circuit* circuit, const qg_noise
       set_op_operator(&t, ch.applied[v].data());
       encode_kops(precision, arith, &t, 1, variants.data() + rec * (4 * s + v));
     }
-    encode_site(tmpl.data() + rec * (size_t)(rec_off[sites[s].pass] + sites[s].at), (int)s);
+    encode_site(tmpl.data() + rec * (size_t)(rec_off[sites[s].pass] + sites[s].at), (int)s,
+                variants.data() + rec * 4 * s);
     site_chan[s] = sites[s].entry;
   }
   std::vector<NoiseChannel> dch(chans.size());

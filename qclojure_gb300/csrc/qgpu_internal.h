@@ -289,7 +289,8 @@ struct NoiseSites {
   const void* variants = nullptr;
   int sites = 0;
 };
-void encode_site(void* record, int site);
+// (its four operators: records of encode_kops)
+void encode_site(void* record, int site, const void* operators);
 cudaError_t launch_tile_pass(int precision, int arithmetic, int io, int n, const PassDesc& pd,
                              void* const* d_states, int nstates, const void* d_kops, int64_t ops_stride,
                              const double* d_dense, cudaStream_t st,

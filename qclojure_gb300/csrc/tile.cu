@@ -261,9 +261,10 @@ struct PolDFT {
   __device__ static dfc zero() { return dfc{0.f, 0.f, 0.f, 0.f}; }
 };
 
-// XOR swizzle of the shared-memory tile: 16-byte units, 8 per 128-byte row.
+// XOR swizzle of the shared-memory tile: 16-byte units, 8 per 128-byte row. Linear over the
+// index bits, so that records hold the slots of single bits and a slot is their XOR.
 template <int ELEM>
-__device__ __forceinline__ int swz(int l) {
+__host__ __device__ __forceinline__ int swz(int l) {
   if (ELEM == 16) return l ^ ((l >> 3) & 7);
   return l ^ (((l >> 4) & 7) << 1);  // 8-byte amplitudes: swizzle pairs, keep each 16-byte pair together
 }
@@ -322,12 +323,13 @@ struct CopyPlan {
 // every thread reads the same record, so the loads are uniform and cheap.
 // ---------------------------------------------------------------------------
 enum KCode : int32_t {  // below 16: everything but gates on registers
-  KC_LAYOUT = 0,   // tmask/tval/rmr = register bits rb0/rb1/rb2, c[0..8) = lj (bit patterns);
-                   // with KF_MAP, as 16-bit halves from c[8]: the map's images of the thread's
-                   // bits 0..9, of the three register bits, and its constant
-  KC_MAPX = 2,     // tmask joins the next map's constant where (base & gmask) == gmask
+  KC_LAYOUT = 0,   // tmask/tval/rmr = register bits rb0/rb1/rb2, c[0..8) = the slots of lj (bit
+                   // patterns); with KF_MAP, as 16-bit halves from c[8]: the slots that the map
+                   // gives the thread's bits 0..9 and the three register bits, and its constant
+  KC_MAPX = 2,     // slot tmask joins the next map's constant where (base & gmask) == gmask
   KC_REMAP = 3,    // registers are written back through the map (fields as KC_LAYOUT)
-  KC_SITE = 4,     // noise site tval: the operator that the state drew (BatchArgs::sites)
+  KC_SITE = 4,     // noise site tval: the operator that the state drew (BatchArgs::sites); bit v of
+                   // tmask: operator v is the identity
   KC_PHASES = 5,   // the next tmask records are phases, by register mask (phase_run)
   KC_DENSE = 1,    // tmask = dk, tval = doff, rmr = dbits (4 bits each)
   KC_U2 = 16,      // + cls * 4 + register position
@@ -336,7 +338,7 @@ enum KCode : int32_t {  // below 16: everything but gates on registers
   KC_BLOCKADE = 62,
   KC_PARITY = 63,
   KC_COLLAPSE = 64,
-  KC_NONE = 65,    // nothing (a noise site whose operator is the identity)
+  KC_NONE = 65,    // nothing (an identity among a noise site's operators)
   KF_COND = 0x100, // the op has control / mask conditions to evaluate
   KF_MAP = 0x200   // the layout reads its registers through a map
 };
@@ -665,17 +667,31 @@ __device__ __forceinline__ void phase_run(typename P::Reg (&r0)[kRegs], typename
   }
 }
 
-// A layout's map on this thread: the image of its index bits and the constant; the images of
-// the register bits go to e[0..3).
-__device__ __forceinline__ uint32_t map_of_thread(const KOp& op, uint32_t (&e)[3]) {
+// A layout's map on this thread: the slot that its index bits and the constant give, and the
+// slots of the register bits in e[0..3). `who` holds the thread's bits as masks, two to a word
+// in the order of the record's halves (a bit at a time, and with the swizzle of every register's
+// slot taken here, a layout change cost about 150 integer instructions; 25 qubits complex64: 7.75
+// ms of passes, 7.47 ms with this; 10,000 noisy shots of 10 qubits, with the record heads: 4807 and 4664 us).
+struct ThreadBits {
+  uint32_t w[5];
+  __device__ __forceinline__ ThreadBits() {
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+      w[i] = ((threadIdx.x >> (2 * i)) & 1u) * 0xFFFFu | ((threadIdx.x >> (2 * i + 1)) & 1u) * 0xFFFF0000u;
+#pragma unroll  // opaque: computed once per tile, not again at every layout
+    for (int i = 0; i < 5; ++i) asm volatile("" : "+r"(w[i]));
+  }
+};
+__device__ __forceinline__ uint32_t map_of_thread(const KOp& op, const ThreadBits& who, uint32_t (&e)[3]) {
   const uint32_t* h = reinterpret_cast<const uint32_t*>(op.c + 8);
-  auto half = [&](int i) { return (h[i >> 1] >> (16 * (i & 1))) & 0xFFFFu; };
-  uint32_t m = half(13);
+  uint32_t m = 0;
 #pragma unroll
-  for (int i = 0; i < 10; ++i) m ^= (0u - ((threadIdx.x >> i) & 1u)) & half(i);
-#pragma unroll
-  for (int q = 0; q < 3; ++q) e[q] = half(10 + q);
-  return m;
+  for (int i = 0; i < 5; ++i) m ^= who.w[i] & h[i];
+  const uint32_t last = h[6];
+  e[0] = h[5] & 0xFFFFu;
+  e[1] = h[5] >> 16;
+  e[2] = last & 0xFFFFu;
+  return (m & 0xFFFFu) ^ (m >> 16) ^ (last >> 16);
 }
 __device__ __forceinline__ uint32_t map_slot(uint32_t m, const uint32_t (&e)[3], int j) {
   return m ^ ((j & 1) ? e[0] : 0u) ^ ((j & 2) ? e[1] : 0u) ^ ((j & 4) ? e[2] : 0u);
@@ -692,32 +708,36 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
   uint32_t lt = 0, mapx = 0;
   // moved: registers were read from other threads' slots, so the next stores wait for all reads
   bool in_regs = false, raw = true, moved = false;
+  const ThreadBits who;
   for (int o = 0; o < nops; ++o) {
     const KOp* rec = sops + o;  // shared memory: a broadcast read
-    int code = rec->code;
+    uint4 head = *reinterpret_cast<const uint4*>(rec);  // code, tmask, tval, rmr
+    int code = (int)head.x;
     if ((code & 0xFF) < 16) {
     const KOp& op = *rec;
     if (code == KC_SITE) {
-      rec = sv.variants + ((size_t)op.tval * 4 + __ldg(sv.choices + op.tval));
-      code = rec->code;
-      if (code == KC_NONE) continue;
+      const uint32_t drawn = __ldg(sv.choices + head.z);
+      if ((head.y >> drawn) & 1u) continue;  // the identity
+      rec = sv.variants + ((size_t)head.z * 4 + drawn);
+      head = *reinterpret_cast<const uint4*>(rec);
+      code = (int)head.x;
     } else {
     if (code == KC_MAPX) {
-      if ((base & op.gmask) == op.gmask) mapx ^= op.tmask;
+      if ((base & op.gmask) == op.gmask) mapx ^= head.y;
       continue;
     }
     if constexpr (P::kPhaseRuns) {
       if (code == KC_PHASES) {
-        phase_run<P, false>(r, r, sops + o + 1, (int)op.tmask, base, 0, lt);
-        o += (int)op.tmask;
+        phase_run<P, false>(r, r, sops + o + 1, (int)head.y, base, 0, lt);
+        o += (int)head.y;
         continue;
       }
     }
     if (code == KC_REMAP) {
       uint32_t e[3];
-      const uint32_t m = map_of_thread(op, e) ^ mapx;
+      const uint32_t m = map_of_thread(op, who, e) ^ mapx;
 #pragma unroll
-      for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>((int)map_slot(m, e, j));
+      for (int j = 0; j < kRegs; ++j) pos[j] = (int)map_slot(m, e, j);
       moved = true;  // the slots are other threads' whatever the layout read
       continue;
     }
@@ -731,18 +751,19 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
       }
       // thread bits: insert zeros at the three register positions (ascending)
       lt = threadIdx.x;
-      const uint32_t rb[3] = {op.tmask, op.tval, op.rmr};
+      const uint32_t rb[3] = {head.y, head.z, head.w};
 #pragma unroll
       for (int q = 0; q < 3; ++q) lt = ((lt >> rb[q]) << (rb[q] + 1)) | (lt & ((1u << rb[q]) - 1));
+      const int at = swz<E>((int)lt);
 #pragma unroll
-      for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>(lt | __float_as_uint(op.c[j]));
+      for (int j = 0; j < kRegs; ++j) pos[j] = at ^ __float_as_int(op.c[j]);
       moved = (code & KF_MAP) != 0;
       uint32_t m = 0, e[3] = {0, 0, 0};
       if (moved) {
-        m = map_of_thread(op, e) ^ mapx;
+        m = map_of_thread(op, who, e) ^ mapx;
         mapx = 0;
       }
-      auto from = [&](int j) { return moved ? swz<E>((int)map_slot(m, e, j)) : pos[j]; };
+      auto from = [&](int j) { return moved ? (int)map_slot(m, e, j) : pos[j]; };
       if (raw) {
 #pragma unroll
         for (int j = 0; j < kRegs; ++j) r[j] = P::load_raw(buf, from(j));
@@ -778,8 +799,8 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
     bool tc = true;
     uint32_t cr = 0;
     if (code & KF_COND) {
-      tc = ((base & op.gmask) == op.gval) && ((lt & op.tmask) == op.tval);
-      cr = op.rmr & 0xFFu;
+      tc = ((base & op.gmask) == op.gval) && ((lt & head.y) == head.z);
+      cr = head.w & 0xFFu;
     }
     switch (code) {
       QG_U2_CASES(U2_GENERAL)
@@ -804,7 +825,7 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
             else swap_regs<P, 1, 2>(r, cr, isw);
           }
         } else if (k == KC_BLOCKADE) {
-          const int cnt = __popcll(base & op.gmask) + __popc(lt & op.tmask);
+          const int cnt = __popcll(base & op.gmask) + __popc(lt & head.y);
           if (cnt <= 1) {
             const typename P::Cst c = kcst<P>(op);
 #pragma unroll
@@ -812,13 +833,13 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
               if (cnt + __popc(j & cr) == 1) r[j] = P::cmul_idx(c, 0, r[j]);
           }
         } else if (k == KC_PARITY) {
-          const int par = (__popcll(base & op.gmask) + __popc(lt & op.tmask)) & 1;
+          const int par = (__popcll(base & op.gmask) + __popc(lt & head.y)) & 1;
           const typename P::Cst c = kcst<P>(op);
 #pragma unroll
           for (int j = 0; j < kRegs; ++j) r[j] = P::cmul_idx(c, par ^ (__popc(j & cr) & 1), r[j]);
         } else if (k == KC_COLLAPSE) {
           const typename P::Cst c = kcst<P>(op);
-          const uint32_t rv = (op.rmr >> 8) & 0xFFu;
+          const uint32_t rv = (head.w >> 8) & 0xFFu;
 #pragma unroll
           for (int j = 0; j < kRegs; ++j) r[j] = (tc && (j & cr) == rv) ? P::scale(c, r[j]) : P::zero();
         }
@@ -895,32 +916,36 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
   uint32_t lt = 0, mapx0 = 0, mapx1 = 0;
   int apart = 0;  // the slots of tile 1 against tile 0's (a map's tile-conditioned parts)
   bool in_regs = false, moved = false;
+  const ThreadBits who;
   for (int o = 0; o < nops; ++o) {
     const KOp* rec = sops + o;
-    int code = rec->code;
+    uint4 head = *reinterpret_cast<const uint4*>(rec);
+    int code = (int)head.x;
     if ((code & 0xFF) < 16) {
     const KOp& op = *rec;
     if (code == KC_SITE) {
-      rec = sv.variants + ((size_t)op.tval * 4 + __ldg(sv.choices + op.tval));
-      code = rec->code;
-      if (code == KC_NONE) continue;
+      const uint32_t drawn = __ldg(sv.choices + head.z);
+      if ((head.y >> drawn) & 1u) continue;  // the identity
+      rec = sv.variants + ((size_t)head.z * 4 + drawn);
+      head = *reinterpret_cast<const uint4*>(rec);
+      code = (int)head.x;
     } else {
     if (code == KC_MAPX) {
-      if ((base0 & op.gmask) == op.gmask) mapx0 ^= op.tmask;
-      if ((base1 & op.gmask) == op.gmask) mapx1 ^= op.tmask;
+      if ((base0 & op.gmask) == op.gmask) mapx0 ^= head.y;
+      if ((base1 & op.gmask) == op.gmask) mapx1 ^= head.y;
       continue;
     }
     if (code == KC_PHASES) {
-      phase_run<P, true>(r0, r1, sops + o + 1, (int)op.tmask, base0, base1, lt);
-      o += (int)op.tmask;
+      phase_run<P, true>(r0, r1, sops + o + 1, (int)head.y, base0, base1, lt);
+      o += (int)head.y;
       continue;
     }
     if (code == KC_REMAP) {
       uint32_t e[3];
-      const uint32_t m = map_of_thread(op, e) ^ mapx0;
+      const uint32_t m = map_of_thread(op, who, e) ^ mapx0;
 #pragma unroll
-      for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>((int)map_slot(m, e, j));
-      apart = swz<E>((int)(mapx0 ^ mapx1));
+      for (int j = 0; j < kRegs; ++j) pos[j] = (int)map_slot(m, e, j);
+      apart = (int)(mapx0 ^ mapx1);
       moved = true;
       continue;
     }
@@ -935,22 +960,23 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
         __syncthreads();
       }
       lt = threadIdx.x;
-      const uint32_t rb[3] = {op.tmask, op.tval, op.rmr};
+      const uint32_t rb[3] = {head.y, head.z, head.w};
 #pragma unroll
       for (int q = 0; q < 3; ++q) lt = ((lt >> rb[q]) << (rb[q] + 1)) | (lt & ((1u << rb[q]) - 1));
+      const int at = swz<E>((int)lt);
 #pragma unroll
-      for (int j = 0; j < kRegs; ++j) pos[j] = swz<E>(lt | __float_as_uint(op.c[j]));
+      for (int j = 0; j < kRegs; ++j) pos[j] = at ^ __float_as_int(op.c[j]);
       moved = (code & KF_MAP) != 0;
       if (moved) {
         uint32_t e[3];
-        const uint32_t m = map_of_thread(op, e) ^ mapx0;
-        const int d = swz<E>((int)(mapx0 ^ mapx1));
+        const uint32_t m = map_of_thread(op, who, e) ^ mapx0;
+        const int d = (int)(mapx0 ^ mapx1);
         mapx0 = mapx1 = 0;
 #pragma unroll
         for (int j = 0; j < kRegs; ++j) {
-          const int at = swz<E>((int)map_slot(m, e, j));
-          r0[j] = P::load_work(buf0, at);
-          r1[j] = P::load_work(buf1, at ^ d);
+          const int from = (int)map_slot(m, e, j);
+          r0[j] = P::load_work(buf0, from);
+          r1[j] = P::load_work(buf1, from ^ d);
         }
       } else {
 #pragma unroll
@@ -985,10 +1011,10 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
     bool tc0 = true, tc1 = true;
     uint32_t cr = 0;
     if (code & KF_COND) {
-      const bool tl = (lt & op.tmask) == op.tval;
+      const bool tl = (lt & head.y) == head.z;
       tc0 = tl && (base0 & op.gmask) == op.gval;
       tc1 = tl && (base1 & op.gmask) == op.gval;
-      cr = op.rmr & 0xFFu;
+      cr = head.w & 0xFFu;
     }
     switch (code) {
       QG_U2_CASES2(U2_GENERAL)
@@ -1019,7 +1045,7 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
           }
         } else if (k == KC_BLOCKADE) {
           const typename P::Cst c = kcst<P>(op);
-          const int ct = __popc(lt & op.tmask);
+          const int ct = __popc(lt & head.y);
           const int cnt0 = __popcll(base0 & op.gmask) + ct, cnt1 = __popcll(base1 & op.gmask) + ct;
 #pragma unroll
           for (int j = 0; j < kRegs; ++j) {
@@ -1028,7 +1054,7 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
           }
         } else if (k == KC_PARITY) {
           const typename P::Cst c = kcst<P>(op);
-          const int pt = __popc(lt & op.tmask);
+          const int pt = __popc(lt & head.y);
           const int par0 = (__popcll(base0 & op.gmask) + pt) & 1, par1 = (__popcll(base1 & op.gmask) + pt) & 1;
 #pragma unroll
           for (int j = 0; j < kRegs; ++j) {
@@ -1037,7 +1063,7 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
           }
         } else if (k == KC_COLLAPSE) {
           const typename P::Cst c = kcst<P>(op);
-          const uint32_t rv = (op.rmr >> 8) & 0xFFu;
+          const uint32_t rv = (head.w >> 8) & 0xFFu;
 #pragma unroll
           for (int j = 0; j < kRegs; ++j) {
             r0[j] = (tc0 && (j & cr) == rv) ? P::scale(c, r0[j]) : P::zero();
@@ -1376,13 +1402,14 @@ __global__ void __launch_bounds__(512, 1) k_job_loop(int n, JobLoopSlot* slots, 
 template <class P>
 void build_kops(KOp* out, const TOp* ops, int64_t nops) {
   std::memset(out, 0, sizeof(KOp) * (size_t)nops);
+  auto slot = [](uint32_t index) { return (uint32_t)swz<P::kElem>((int)index); };
   for (int64_t o = 0; o < nops; ++o) {
     const TOp& t = ops[o];
     KOp& k = out[o];
     if (t.kind == OK_MAPX) {
       k.code = KC_MAPX;
       k.gmask = t.gmask;
-      k.tmask = t.mc0;
+      k.tmask = slot(t.mc0);
       continue;
     }
     if (t.kind == OK_LAYOUT || t.kind == OK_REMAP) {
@@ -1390,14 +1417,17 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
       k.tmask = t.dbits[0];
       k.tval = t.dbits[1];
       k.rmr = t.dbits[2];
-      for (int j = 0; j < 8; ++j) std::memcpy(&k.c[j], &t.lj[j], 4);
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t at = slot((uint32_t)t.lj[j]);
+        std::memcpy(&k.c[j], &at, 4);
+      }
       if (t.mapped) {
         uint16_t h[16] = {0};
         int i = 0;
         for (int b = 0; b < kMaxTileBits && i < 10; ++b)  // thread bits: the others, ascending
-          if (b != t.dbits[0] && b != t.dbits[1] && b != t.dbits[2]) h[i++] = t.mcol[b];
-        for (int q = 0; q < 3; ++q) h[10 + q] = t.mcol[t.dbits[q]];
-        h[13] = t.mc0;
+          if (b != t.dbits[0] && b != t.dbits[1] && b != t.dbits[2]) h[i++] = (uint16_t)slot(t.mcol[b]);
+        for (int q = 0; q < 3; ++q) h[10 + q] = (uint16_t)slot(t.mcol[t.dbits[q]]);
+        h[13] = (uint16_t)slot(t.mc0);
         std::memcpy(&k.c[8], h, sizeof(h));
       }
       continue;
@@ -1519,11 +1549,13 @@ void encode_kops(int precision, int arithmetic, const TOp* tops, int64_t count, 
   else build_kops<PolD>(k, tops, count);
 }
 
-void encode_site(void* record, int site) {
+void encode_site(void* record, int site, const void* operators) {
   KOp* k = reinterpret_cast<KOp*>(record);
   std::memset(k, 0, sizeof(KOp));
   k->code = KC_SITE;
   k->tval = (uint32_t)site;
+  for (int v = 0; v < 4; ++v)
+    if (reinterpret_cast<const KOp*>(operators)[v].code == KC_NONE) k->tmask |= 1u << v;
 }
 
 template <class P>
