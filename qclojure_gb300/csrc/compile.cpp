@@ -861,9 +861,13 @@ void plan_interpreted(const std::vector<TOp>& ops, int k, std::vector<TOp>* reco
       continue;
     }
     blank(OK_PHASES).dk = (int)(j - i);
+    // within a mask: general ones without and with tile bits, then the powers of i
     for (uint32_t m = 0; m < 8; ++m)
-      for (size_t q = i; q < j; ++q)
-        if ((plan.ops[q].rmask & 7u) == m) records->push_back(plan.ops[q]);
+      for (int kind = 0; kind < 3; ++kind)
+        for (size_t q = i; q < j; ++q) {
+          const TOp& ph = plan.ops[q];
+          if ((ph.rmask & 7u) == m && (ph.cls != PH_GENERAL ? 2 : ph.gmask != 0 ? 1 : 0) == kind) records->push_back(ph);
+        }
     i = j;
   }
   if (last && !plan.last.identity()) {

@@ -138,7 +138,7 @@ struct PolExact {
   __device__ static V times_i(V x) { V r; r.x = -x.y; r.y = x.x; return r; }
   __device__ static V minus(V x) { V r; r.x = -x.x; r.y = -x.y; return r; }
   __device__ static V one() { V r; r.x = 1; r.y = 0; return r; }
-  __device__ static V factor(const KOp& op, V f);  // the phase of a record times f
+  __device__ static V factor(const uint4& head, const KOp& op, V f);  // the phase of a record times f
   __device__ static V mul(V f, V x) { return cm(f.x, f.y, x); }
   // phases of one run are multiplied together before they meet the amplitudes (not in FP64,
   // which keeps the reference's order of roundings)
@@ -245,7 +245,7 @@ struct PolDFT {
   static constexpr bool kPhaseRuns = true;
   __device__ static dfc minus(const dfc& x) { return dfc{-x.rh, -x.ih, -x.rl, -x.il}; }
   __device__ static dfc one() { return dfc{1.f, 0.f, 0.f, 0.f}; }
-  __device__ static dfc factor(const KOp& op, const dfc& f);
+  __device__ static dfc factor(const uint4& head, const KOp& op, const dfc& f);
   __device__ static dfc mul(const dfc& f, const dfc& x) { return cmul_df(f.rh, f.rl, f.ih, f.il, x); }
   __device__ static dfc times_i(const dfc& x) { return dfc{-x.ih, x.rh, -x.il, x.rl}; }
   __device__ static dfc cmul_idx(const Cst& c, int which, const dfc& x) {
@@ -330,7 +330,7 @@ enum KCode : int32_t {  // below 16: everything but gates on registers
   KC_REMAP = 3,    // registers are written back through the map (fields as KC_LAYOUT)
   KC_SITE = 4,     // noise site tval: the operator that the state drew (BatchArgs::sites); bit v of
                    // tmask: operator v is the identity
-  KC_PHASES = 5,   // the next tmask records are phases, by register mask (phase_run)
+  KC_PHASES = 5,   // the next tmask records are phases, by register mask; c = their counts (phase_run)
   KC_DENSE = 1,    // tmask = dk, tval = doff, rmr = dbits (4 bits each)
   KC_U2 = 16,      // + cls * 4 + register position
   KC_PHASE = 128,  // + phase class * 8 + register mask (the registers whose bits must all be 1)
@@ -584,23 +584,28 @@ struct SiteView {
 };
 
 template <typename R, typename V>
-__device__ __forceinline__ V PolExact<R, V>::factor(const KOp& op, V f) {
-  if constexpr (kFMA) return cm((R)op.c[0], (R)op.c[1], f);
+__device__ __forceinline__ V PolExact<R, V>::factor(const uint4& head, const KOp&, V f) {
+  if constexpr (kFMA) return cm(__uint_as_float(head.z), __uint_as_float(head.w), f);
   else return f;
 }
 template <int IO, bool DENSE>
-__device__ __forceinline__ dfc PolDFT<IO, DENSE>::factor(const KOp& op, const dfc& f) {
-  return cmul_df(op.c[0], op.c[8], op.c[1], op.c[9], f);
+__device__ __forceinline__ dfc PolDFT<IO, DENSE>::factor(const uint4&, const KOp& op, const dfc& f) {
+  const float4 c = *reinterpret_cast<const float4*>(op.c);
+  return cmul_df(c.x, c.z, c.y, c.w, f);
 }
 
-// A run of `cnt` phases, sorted by the register bits they ask for. Per register mask m, the
+// A run of phases, sorted by the register bits they ask for. Per register mask m, the
 // phases whose tile and thread bits hold are multiplied into one factor (powers of i are
 // counted), and the registers that include m take it: one product per phase and thread, where
 // the phases one by one took a dispatch and a product per register each (a controlled phase:
-// four of eight registers of both tiles). Two tiles at a time where r1 is given.
+// four of eight registers of both tiles). Two tiles at a time where r1 is given. The header
+// counts each mask's phases: general ones without tile bits (tiles interpreted together share
+// them), general ones with, then the others; with one loop that took all three, the compiler
+// turned every choice into selects, 70 instructions per phase and pair of tiles (25-qubit
+// complex64 circuit with a transform: 7.41 ms of passes, now 6.74 ms).
 template <class P, bool TWO>
 __device__ __forceinline__ void phase_run(typename P::Reg (&r0)[kRegs], typename P::Reg (&r1)[kRegs],
-                                          const KOp* __restrict__ ph, int cnt, uint64_t base0, uint64_t base1,
+                                          const KOp* __restrict__ run, uint64_t base0, uint64_t base1,
                                           uint32_t lt) {
   using Reg = typename P::Reg;
   auto turn = [](Reg x, int pw) {
@@ -608,35 +613,49 @@ __device__ __forceinline__ void phase_run(typename P::Reg (&r0)[kRegs], typename
     if (pw & 2) x = P::minus(x);
     return x;
   };
-  int i = 0;
-#pragma unroll
+  const KOp* p = run + 1;
+#pragma unroll(P::kDF ? 1 : kRegs)  // DF: eight copies of the loops crowd the instruction cache
   for (int m = 0; m < kRegs; ++m) {
-    if (i >= cnt || (ph[i].code & 7) != m) continue;
-    Reg f0 = P::one(), f1 = P::one();
+    const uint2 n = reinterpret_cast<const uint2*>(run->c)[m];
+    if ((n.x | n.y) == 0) continue;
+    Reg f0 = P::one();
     int pw0 = 0, pw1 = 0;
-    bool general = false, hit0 = false, hit1 = false;
-    do {
-      const KOp& p = ph[i];
-      const int cls = (p.code >> 3) & 3;
-      const bool tl = (lt & p.tmask) == p.tmask;
-      const bool c0 = tl && (base0 & p.gmask) == p.gmask, c1 = TWO && tl && (base1 & p.gmask) == p.gmask;
-      if (cls == PH_GENERAL) {
-        general = true;
-        const Reg g0 = P::factor(p, f0);
-        if (c0) f0 = g0;
-        hit0 = hit0 || c0;
-        if (TWO) {
-          const Reg g1 = P::factor(p, f1);
-          if (c1) f1 = g1;
-          hit1 = hit1 || c1;
-        }
-      } else {
-        const int q = cls == PH_NEG ? 2 : cls == PH_I ? 1 : 3;
-        pw0 += c0 ? q : 0;
-        if (TWO) pw1 += c1 ? q : 0;
+    bool hit0 = false;
+    const bool general = n.x != 0;
+    const KOp* end = p + (n.x & 0xFFFFu);
+#pragma unroll(P::kDF ? 1 : 2)
+    for (; p < end; ++p) {
+      const uint4 head = *reinterpret_cast<const uint4*>(p);
+      const bool c = (lt & head.y) == head.y;
+      const Reg g = P::factor(head, *p, f0);
+      if (c) f0 = g;
+      hit0 = hit0 || c;
+    }
+    Reg f1 = f0;
+    bool hit1 = hit0;
+    for (end = p + (n.x >> 16); p < end; ++p) {
+      const uint64_t gm = p->gmask;
+      const bool t0 = (base0 & gm) == gm, t1 = TWO && (base1 & gm) == gm;
+      if (!t0 && !t1) continue;
+      const uint4 head = *reinterpret_cast<const uint4*>(p);
+      const bool c = (lt & head.y) == head.y;
+      const Reg g0 = P::factor(head, *p, f0);
+      if (t0 && c) f0 = g0;
+      hit0 = hit0 || (t0 && c);
+      if (TWO) {
+        const Reg g1 = P::factor(head, *p, f1);
+        if (t1 && c) f1 = g1;
+        hit1 = hit1 || (t1 && c);
       }
-      ++i;
-    } while (i < cnt && (ph[i].code & 7) == m);
+    }
+    for (end = p + n.y; p < end; ++p) {
+      const uint4 head = *reinterpret_cast<const uint4*>(p);
+      const uint64_t gm = p->gmask;
+      const uint32_t cls = (head.x >> 3) & 3u;
+      const int q = (lt & head.y) != head.y ? 0 : cls == PH_NEG ? 2 : cls == PH_I ? 1 : 3;
+      pw0 += (base0 & gm) == gm ? q : 0;
+      if (TWO) pw1 += (base1 & gm) == gm ? q : 0;
+    }
     if (general) {
       f0 = turn(f0, pw0);
       if (hit0 || (pw0 & 3)) {
@@ -728,7 +747,7 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
     }
     if constexpr (P::kPhaseRuns) {
       if (code == KC_PHASES) {
-        phase_run<P, false>(r, r, sops + o + 1, (int)head.y, base, 0, lt);
+        phase_run<P, false>(r, r, rec, base, 0, lt);
         o += (int)head.y;
         continue;
       }
@@ -936,7 +955,7 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
       continue;
     }
     if (code == KC_PHASES) {
-      phase_run<P, true>(r0, r1, sops + o + 1, (int)head.y, base0, base1, lt);
+      phase_run<P, true>(r0, r1, rec, base0, base1, lt);
       o += (int)head.y;
       continue;
     }
@@ -1402,6 +1421,7 @@ __global__ void __launch_bounds__(512, 1) k_job_loop(int n, JobLoopSlot* slots, 
 template <class P>
 void build_kops(KOp* out, const TOp* ops, int64_t nops) {
   std::memset(out, 0, sizeof(KOp) * (size_t)nops);
+  int run = 0;  // phases left of a run
   auto slot = [](uint32_t index) { return (uint32_t)swz<P::kElem>((int)index); };
   for (int64_t o = 0; o < nops; ++o) {
     const TOp& t = ops[o];
@@ -1455,6 +1475,13 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
       case OK_PHASES:
         k.code = KC_PHASES;
         k.tmask = (uint32_t)t.dk;
+        std::memset(k.c, 0, sizeof(k.c));
+        for (const TOp* p = &t + 1; p <= &t + t.dk; ++p) {
+          uint32_t* n = reinterpret_cast<uint32_t*>(k.c) + 2 * (p->rmask & 7u);
+          if (p->cls != PH_GENERAL) ++n[1];
+          else n[0] += p->gmask != 0 ? 1u << 16 : 1u;
+        }
+        run = t.dk;
         continue;
       case OK_U2:
         k.code = KC_U2 + t.cls * 4 + t.t2;
@@ -1465,6 +1492,16 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
         k.code = KC_PHASE + t.cls * 8 + (int)(t.rmask & 7u);
         k.gmask = k.gval = t.gmask;
         cond = t.tmask != 0 || t.gmask != 0;
+        if (run > 0) {
+          --run;
+          if (P::kCst == 1) {  // the factor beside tmask
+            std::memcpy(&k.tval, &k.c[0], 4);
+            std::memcpy(&k.rmr, &k.c[1], 4);
+          } else {  // re.hi, im.hi, re.lo, im.lo
+            k.c[2] = k.c[8];
+            k.c[3] = k.c[9];
+          }
+        }
         break;
       case OK_SWAP: {
         const int a = t.dbits[0], b = t.dbits[1];
