@@ -355,7 +355,7 @@ std::shared_ptr<const PassKernels> pass_kernels_for(const Program& prog, int pre
 // The program's kernels if an earlier call compiled them (no compile here).
 std::shared_ptr<const PassKernels> pass_kernels_cached(const Program& prog, int prec, int device);
 // Programs with equal keys share table-form kernels (coefficients left out).
-std::string pass_structure_key(const Program& prog, bool table);
+std::string pass_structure_key(const Program& prog, int prec, bool table);
 // Launch the table form over nstates states; d_coefs holds nstates rows of
 // 16 * (ops of the pass) floats (pass_coefficients of each state's program).
 cudaError_t launch_pass_kernel_batch(const PassKernels& pk, size_t step, int n, const PassDesc& pd,

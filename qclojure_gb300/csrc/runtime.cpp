@@ -2938,9 +2938,9 @@ static void setup_group_pass_kernels(Sweep* sw, SweepGroup& g) {
   const Ctx* c = sw->ctx;
   if (c->cfg.pass_kernels == QG_PASS_KERNELS_OFF) return;
   if (sw->prec == QG_C128 && sw->arith != QG_ARITH_DOUBLE_FLOAT) return;
-  const std::string k0 = pass_structure_key(g.progs[0], true);
+  const std::string k0 = pass_structure_key(g.progs[0], sw->prec, true);
   for (size_t m = 1; m < g.progs.size(); ++m)
-    if (pass_structure_key(g.progs[m], true) != k0) return;
+    if (pass_structure_key(g.progs[m], sw->prec, true) != k0) return;
   std::string why;
   auto pk = pass_kernels_for(g.progs[0], sw->prec, c->device, &why, true);
   if (!pk) return;
@@ -3407,7 +3407,7 @@ int qg_sweep_update(void* sweep, const qg_circuit* circuits, int32_t count) {
     SweepGroup& g = sw->groups[sw->where[i].first];
     Program& old = g.progs[sw->where[i].second];
     if (pass_signature(prog) != pass_signature(old) ||
-        (g.pk && pass_structure_key(prog, true) != pass_structure_key(old, true))) {
+        (g.pk && pass_structure_key(prog, sw->prec, true) != pass_structure_key(old, sw->prec, true))) {
       set_ctx_error(sw->ctx, "circuit " + std::to_string(i) + " changed its structure; create a new sweep");
       return QG_ERR_INVALID_ARG;
     }

@@ -1,6 +1,6 @@
-"""A sweep whose members' rotation angles lie on both sides of zero runs as specialised kernels
-(the sign of a sine is a value, not a structure), before and after an update that moves them
-across; energies equal the oracle's."""
+"""A complex128 sweep whose members' rotation angles lie on both sides of zero runs as specialised
+kernels (the sign of a sine is a value, not a structure), before and after an update that moves
+them across; a complex64 one stays interpreted. Energies equal the oracle's."""
 import numpy as np
 import pytest
 
@@ -26,7 +26,8 @@ def test_angles_of_both_signs_share_kernels(oracle, precision, tol):
             cs = circuits(shift)
             sw.update(cs)
             got, stats = sw.run([ham] * len(cs))
-            assert stats["specialised"] == stats["groups"] == 1
+            assert stats["groups"] == 1
+            assert stats["specialised"] == (1 if precision == "c128" else 0)
             for e, c in zip(got, cs):
                 ref = oracle.run(c)
                 want = sum(t["coefficient"] * oracle.pauli_expectation(ref, t["pauli-string"]) for t in ham)
