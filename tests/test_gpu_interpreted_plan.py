@@ -74,3 +74,24 @@ def test_small_jobs(oracle, n, precision, tol):
             assert np.max(np.abs(sv - oracle.run(c))) <= tol
         finally:
             sim.close()
+
+
+def test_complex64_plans_of_large_states():
+    """complex64 is planned from 25 qubits on, two tiles per dispatch: phases over thread and tile
+    bits, permutations, gates, against the same circuit in complex128. Tolerance: two roundings
+    of 2^-24 per operation."""
+    from qclojure_gb300 import workloads
+    from qclojure_gb300.state import Context
+
+    n = 25
+    rng = np.random.default_rng(25)
+    ops = _some(n, 60, _PHASE, rng) + [_op("h", target=q) for q in range(n)] + _some(n, 150, _ALL, rng)
+    ops += workloads.qft_ops(n) + _some(n, 10, _PERM, rng)
+    c = {"num-qubits": n, "operations": ops}
+    got = []
+    with Context(pass_kernels="off", arithmetic="double-float") as ctx:
+        for precision in ("c64", "c128"):
+            with ctx.state(n, precision) as st:
+                st.apply(c)
+                got.append(st.download())
+    assert np.linalg.norm(got[0] - got[1]) <= len(ops) * 2 * 2.0**-24
