@@ -630,9 +630,8 @@ def main():
                      if dom_kind == 3 else ("k_tile2<PolDFT>" if args.precision == "c128" else "k_tile2<PolF>"),
                      "peak_source": peak_src, "pass_bytes": pass_bytes, "mean_pass_ms": mean_pass,
                      "passes": len(dom),
-                     "note": ("passes are bound by FP32 instruction issue, not HBM: ncu on the same kernel "
-                              "and shape (26 qubits) shows 59-68% issue active and 31-32% DRAM throughput "
-                              "for double-float complex128")
+                     "note": ("passes are bound by the FP32 pipe, not HBM: ncu on the same kernel shows it "
+                              "68-73% busy for double-float complex128")
                      if dom_kind == 3 and args.precision == "c128" else None},
         "gpu_launches": int(l1.value - l0.value),
         "clocks": ck,
