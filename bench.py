@@ -631,7 +631,7 @@ def main():
                      "peak_source": peak_src, "pass_bytes": pass_bytes, "mean_pass_ms": mean_pass,
                      "passes": len(dom),
                      "note": ("passes are bound by the FP32 pipe, not HBM: ncu on the same kernel shows it "
-                              "68-73% busy for double-float complex128")
+                              "69-81% busy for double-float complex128")
                      if dom_kind == 3 and args.precision == "c128" else None},
         "gpu_launches": int(l1.value - l0.value),
         "clocks": ck,
