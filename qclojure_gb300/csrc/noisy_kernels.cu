@@ -93,14 +93,15 @@ __global__ void __launch_bounds__(256) k_noise_readout(uint64_t* __restrict__ ou
   outcomes[m] = bits;
 }
 
-// out[t] = state state_of[first + t] without its padding qubits, as complex128
+// out[t] = state state_of[first + t] without its padding qubits, as complex128. The shot is the
+// grid's x: up to 65536 shots of one batch are collected at once, and y ends at 65535.
 template <typename T>
 __global__ void __launch_bounds__(256) k_noise_collect(void* const* __restrict__ states,
                                                        const int32_t* __restrict__ state_of, int first, int n, int shift,
                                                        double2* __restrict__ out) {
-  const T* s = reinterpret_cast<const T*>(states[state_of[first + (int)blockIdx.y]]);
-  double2* o = out + ((uint64_t)blockIdx.y << n);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (1ULL << n); i += (uint64_t)gridDim.x * blockDim.x) {
+  const T* s = reinterpret_cast<const T*>(states[state_of[first + (int)blockIdx.x]]);
+  double2* o = out + ((uint64_t)blockIdx.x << n);
+  for (uint64_t i = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; i < (1ULL << n); i += (uint64_t)gridDim.y * blockDim.x) {
     const T v = s[i << shift];
     o[i] = make_double2((double)v.x, (double)v.y);
   }
@@ -135,11 +136,11 @@ cudaError_t launch_noise_readout(uint64_t* d_outcomes, int shots, int n, uint64_
 
 cudaError_t launch_noise_collect(int precision, void* const* d_states, const int32_t* d_state_of, int first, int count,
                                  int n, int shift, double* d_out, cudaStream_t st) {
-  const unsigned gx = (unsigned)std::min<uint64_t>(((1ULL << n) + 255) / 256, 1024);
+  const dim3 grid((unsigned)count, (unsigned)std::min<uint64_t>(((1ULL << n) + 255) / 256, 1024));
   if (precision == QG_C64)
-    k_noise_collect<float2><<<dim3(gx, (unsigned)count), 256, 0, st>>>(d_states, d_state_of, first, n, shift, (double2*)d_out);
+    k_noise_collect<float2><<<grid, 256, 0, st>>>(d_states, d_state_of, first, n, shift, (double2*)d_out);
   else
-    k_noise_collect<double2><<<dim3(gx, (unsigned)count), 256, 0, st>>>(d_states, d_state_of, first, n, shift, (double2*)d_out);
+    k_noise_collect<double2><<<grid, 256, 0, st>>>(d_states, d_state_of, first, n, shift, (double2*)d_out);
   count_launch(1);
   return cudaGetLastError();
 }
