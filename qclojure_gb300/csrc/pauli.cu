@@ -6,18 +6,20 @@
 // clear, of Re or Im of conj(a_i) a_{i^x} (each pair counts twice). Pair index q is i without
 // that bit; a string's sign is the parity of q & zq.
 //
-// What bounds it: the FP64 pipe (two instructions per clock and SM on this part). One kernel per
+// What bounds it: the FP64 pipe (two lanes per clock and SM on this part). One kernel per
 // string cost three to four FP64 instructions for the value and seven for a TwoSum per
 // amplitude, and one host round trip per string: 24 qubits, complex128, a Heisenberg chain of
-// 93 strings took 93 x 320 us. Here a group's values are formed once for all of its strings, 16
-// values are summed as a tree before one TwoSum, and all groups run in one launch:
-//   * up to two strings per group (XX and YY on a pair): the values on which their signs agree
-//     and those on which they differ are summed apart; sum and difference give both strings
-//     (one add per value instead of one per value and string);
+// 93 strings took 93 x 320 us. Here a group's values are formed once for all of its strings (two
+// FP64 instructions each), summed exactly in fixed point on the integer pipes (fixed_sum.cuh), and
+// all groups run in one launch; every string's sum is that of its rounded values, in any company:
+//   * up to two strings per group (XX and YY on a pair): each thread adds its 16 values of a tile
+//     to both sums with their signs, then one TwoSum takes each;
 //   * more strings (the Z and ZZ terms): a Walsh-Hadamard transform of the tile over 8 of its 12
-//     index bits (4 in registers, 4 after an exchange through shared memory; 8 adds per value
-//     whatever the number of strings), then one thread per string adds its 16 remaining signed
-//     values and does one TwoSum per tile of 4096.
+//     index bits (4 in registers, 4 after an exchange through shared memory), of the upper and the
+//     lower integers in turn, then one thread per string adds its 16 remaining signed values and
+//     does one TwoSum per tile of 4096.
+// 24 qubits, complex128, the 93 strings: 2.60 ms (3.28 ms with the 16 values added in FP64 before
+// a TwoSum, which also lost what the TwoSum is for: cancelling terms were off by ulps of the terms).
 // Neighbouring CTAs work on the same chunk of different groups, so the state is read from L2 by
 // all but the first of them.
 #include <algorithm>
@@ -27,8 +29,8 @@
 #include <utility>
 #include <vector>
 
+#include "fixed_sum.cuh"
 #include "qgpu_internal.h"
-#include "quant.cuh"
 
 namespace qg {
 
@@ -36,7 +38,7 @@ namespace {
 
 constexpr int kTileBits = 12;      // values per tile: 16 per thread, 256 threads
 constexpr int kGroupStrings = 256; // strings per group at most (one thread each)
-constexpr int kPitch = 256 + 16;   // doubles per transform row: t + t / 16, free of bank conflicts
+constexpr int kPitch = 256 + 16;   // words per transform row: t + t / 16, free of bank conflicts
 
 struct PauliGroup {
   uint64_t xm;
@@ -54,10 +56,6 @@ __device__ __forceinline__ void two_sum(double& s, double& c, double x) {
   const double bp = __dsub_rn(t, s);
   c = __dadd_rn(c, __dadd_rn(__dsub_rn(s, __dsub_rn(t, bp)), __dsub_rn(x, bp)));
   s = t;
-}
-
-__device__ __forceinline__ double flip(double v, uint32_t sign) {  // sign 0 or 1
-  return __hiloint2double(__double2hiint(v) ^ (int)(sign << 31), __double2loint(v));
 }
 
 // (double)f with integer instructions (the conversion runs at the FP64 rate)
@@ -106,23 +104,29 @@ __device__ __forceinline__ void tile_values(const T* __restrict__ s, const Pauli
   }
 }
 
-// the parity of r & zr for the 16 register positions r (index bits 8..11), as a bit pattern
-__device__ __forceinline__ uint32_t reg_pattern(uint64_t zq) {
-  const uint32_t z = (uint32_t)(zq >> 8) & 15u;
+// the parity of r & z for r = 0..15, as a bit pattern
+__device__ __forceinline__ uint32_t parities(uint32_t z) {
   return ((z & 1) ? 0xAAAAu : 0u) ^ ((z & 2) ? 0xCCCCu : 0u) ^ ((z & 4) ? 0xF0F0u : 0u) ^ ((z & 8) ? 0xFF00u : 0u);
 }
 
-// pd, the parity pattern of a mask that holds bit B: of every pair (r, r ^ B) one position has
-// parity 0 (into a) and one has parity 1 (into d)
-template <int B>
-__device__ __forceinline__ void split(const double (&v)[16], uint32_t pd, double (&a)[8], double (&d)[8]) {
+__device__ __forceinline__ uint32_t top_key(const double (&v)[16]) {
+  uint32_t key = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int r = (k & (B - 1)) | ((k & ~(B - 1)) << 1);
-    const bool f = (pd >> r) & 1u;
-    a[k] = f ? v[r ^ B] : v[r];
-    d[k] = f ? v[r] : v[r ^ B];
-  }
+  for (int r = 0; r < 16; ++r) key = max(key, qg_fix_key(v[r]));
+  return key;
+}
+
+// sums and differences over 4 index bits
+__device__ __forceinline__ void transform(int64_t (&v)[16]) {
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1)
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (!(r & o)) {
+        const int64_t x = v[r], y = v[r + o];
+        v[r] = x + y;
+        v[r + o] = x - y;
+      }
 }
 
 template <typename T>
@@ -130,7 +134,8 @@ __global__ void __launch_bounds__(256, 3) k_pauli_sums(const T* __restrict__ s, 
                                                        const PauliGroup* __restrict__ groups,
                                                        const PauliString* __restrict__ strings, int ngroups,
                                                        int nchunks, double2* __restrict__ partial) {
-  __shared__ double sh[16 * kPitch];
+  __shared__ int64_t sh[16 * kPitch];
+  __shared__ uint32_t keys[8];
   const int chunk = (int)(blockIdx.x / (unsigned)ngroups);
   const PauliGroup g = groups[blockIdx.x - (unsigned)chunk * (unsigned)ngroups];
   const uint64_t count = (1ULL << n) >> (g.hb < 0 ? 0 : 1);
@@ -139,37 +144,29 @@ __global__ void __launch_bounds__(256, 3) k_pauli_sums(const T* __restrict__ s, 
   const int tid = (int)threadIdx.x;
   if (g.nt <= 2) {
     const uint64_t z0 = strings[g.t0].zq, z1 = strings[g.t0 + g.nt - 1].zq;
-    const uint32_t p0 = reg_pattern(z0), pd = p0 ^ reg_pattern(z1);  // signs of string 0; where the two differ
+    const uint32_t p0 = parities((uint32_t)(z0 >> 8)), p1 = parities((uint32_t)(z1 >> 8));  // register positions: bits 8..11
     double s0 = 0, c0 = 0, s1 = 0, c1 = 0;
     for (uint64_t t = w0; t < w1; ++t) {
       const uint64_t q0 = (t << kTileBits) + (uint64_t)tid;
       double v[16];
       tile_values(s, g, q0, count, v);
+      const int E = qg_fix_exponent(top_key(v));
       const uint32_t t0 = (uint32_t)__popcll(q0 & z0) & 1u, t1 = (uint32_t)__popcll(q0 & z1) & 1u;
+      int64_t h0 = 0, l0 = 0, h1 = 0, l1 = 0;
 #pragma unroll
-      for (int r = 0; r < 16; ++r) v[r] = flip(v[r], ((p0 >> r) & 1u) ^ t0);
-      if (pd == 0) {  // one string, or two whose signs agree over the whole tile up to one factor
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-          for (int r = 0; r < o; ++r) v[r] = __dadd_rn(v[r], v[r + o]);
-        two_sum(s0, c0, v[0]);
-        if (g.nt == 2) two_sum(s1, c1, flip(v[0], t0 ^ t1));
-      } else {
-        double a[8], d[8];  // string 1's sign agrees with string 0's; differs
-        if (pd & 0x2u) split<1>(v, pd, a, d);
-        else if (pd & 0x4u) split<2>(v, pd, a, d);
-        else if (pd & 0x10u) split<4>(v, pd, a, d);
-        else split<8>(v, pd, a, d);
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-          for (int r = 0; r < o; ++r) {
-            a[r] = __dadd_rn(a[r], a[r + o]);
-            d[r] = __dadd_rn(d[r], d[r + o]);
-          }
-        two_sum(s0, c0, __dadd_rn(a[0], d[0]));
-        two_sum(s1, c1, flip(__dsub_rn(a[0], d[0]), t0 ^ t1));
+      for (int r = 0; r < 16; ++r) {
+        const qg_fixed x = qg_fix(v[r], E, ((p0 >> r) & 1u) ^ t0);
+        const int64_t other = -(int64_t)((((p0 ^ p1) >> r) & 1u) ^ t0 ^ t1);  // string 1's sign against string 0's
+        h0 += x.h;
+        l0 += x.l;
+        h1 += (x.h ^ other) - other;
+        l1 += (x.l ^ other) - other;
+      }
+      two_sum(s0, c0, qg_fix_hi(h0, E));
+      c0 = __dadd_rn(c0, qg_fix_lo(l0, E));
+      if (g.nt == 2) {
+        two_sum(s1, c1, qg_fix_hi(h1, E));
+        c1 = __dadd_rn(c1, qg_fix_lo(l1, E));
       }
     }
     __shared__ double2 red[2][8];
@@ -198,50 +195,52 @@ __global__ void __launch_bounds__(256, 3) k_pauli_sums(const T* __restrict__ s, 
   const bool mine = tid < g.nt;
   const uint64_t zq = mine ? strings[g.t0 + tid].zq : 0;
   const int row = (int)(zq >> 8) & 15, col = (int)zq & 15;
-  const uint32_t zh = (uint32_t)(zq >> 4) & 15u;
+  const uint32_t ph = parities((uint32_t)(zq >> 4));
   double acc = 0, comp = 0;
   for (uint64_t t = w0; t < w1; ++t) {
-    double v[16];
-    tile_values(s, g, (t << kTileBits) + (uint64_t)tid, count, v);
+    const uint32_t ts = (uint32_t)__popcll((t << kTileBits) & zq) & 1u;
+    int E = 0;
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {  // the upper integers, then the lower ones of the same values
+      double v[16];
+      tile_values(s, g, (t << kTileBits) + (uint64_t)tid, count, v);
+      if (part == 0) {
+        const uint32_t key = __reduce_max_sync(0xffffffffu, top_key(v));
+        if ((tid & 31) == 0) keys[tid >> 5] = key;
+        __syncthreads();  // and the previous tile's readers are done
+        uint32_t top = 0;
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1)
+        for (int w = 0; w < 8; ++w) top = max(top, keys[w]);
+        E = qg_fix_exponent(top);
+      }
+      int64_t x[16];
 #pragma unroll
-      for (int r = 0; r < 16; ++r)
-        if (!(r & o)) {
-          const double x = v[r], y = v[r + o];
-          v[r] = __dadd_rn(x, y);
-          v[r + o] = __dsub_rn(x, y);
+      for (int r = 0; r < 16; ++r) {
+        const qg_fixed f = qg_fix(v[r], E, 0);
+        x[r] = part ? f.l : f.h;
+      }
+      transform(x);
+      if (part) __syncthreads();  // the readers of the upper integers are done
+#pragma unroll
+      for (int r = 0; r < 16; ++r) sh[r * kPitch + tid + (tid >> 4)] = x[r];
+      __syncthreads();
+      int64_t* mr = sh + (tid >> 4) * kPitch + (tid & 15) * 17;  // 16 values of one row, index bits 0..3
+#pragma unroll
+      for (int l = 0; l < 16; ++l) x[l] = mr[l];
+      transform(x);
+#pragma unroll
+      for (int l = 0; l < 16; ++l) mr[l] = x[l];
+      __syncthreads();
+      if (mine) {
+        int64_t sum = 0;
+#pragma unroll
+        for (int h = 0; h < 16; ++h) {
+          const int64_t f = -(int64_t)(((ph >> h) & 1u) ^ ts);
+          sum += (sh[row * kPitch + h * 17 + col] ^ f) - f;
         }
-    __syncthreads();  // the previous tile's readers are done
-#pragma unroll
-    for (int r = 0; r < 16; ++r) sh[r * kPitch + tid + (tid >> 4)] = v[r];
-    __syncthreads();
-    double* mr = sh + (tid >> 4) * kPitch + (tid & 15) * 17;  // 16 values of one row, index bits 0..3
-#pragma unroll
-    for (int l = 0; l < 16; ++l) v[l] = mr[l];
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1)
-#pragma unroll
-      for (int r = 0; r < 16; ++r)
-        if (!(r & o)) {
-          const double x = v[r], y = v[r + o];
-          v[r] = __dadd_rn(x, y);
-          v[r + o] = __dsub_rn(x, y);
-        }
-#pragma unroll
-    for (int l = 0; l < 16; ++l) mr[l] = v[l];
-    __syncthreads();
-    if (mine) {
-      const uint32_t ts = (uint32_t)__popcll((t << kTileBits) & zq) & 1u;
-      double x[16];
-#pragma unroll
-      for (int h = 0; h < 16; ++h)
-        x[h] = flip(sh[row * kPitch + h * 17 + col], ((uint32_t)__popc((uint32_t)h & zh) & 1u) ^ ts);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-        for (int r = 0; r < o; ++r) x[r] = __dadd_rn(x[r], x[r + o]);
-      two_sum(acc, comp, x[0]);
+        if (part) comp = __dadd_rn(comp, qg_fix_lo(sum, E));
+        else two_sum(acc, comp, qg_fix_hi(sum, E));
+      }
     }
   }
   if (mine) partial[(size_t)(g.t0 + tid) * nchunks + chunk] = make_double2(acc, comp);
