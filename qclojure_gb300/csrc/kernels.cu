@@ -15,8 +15,8 @@
 #include <atomic>
 #include <cstdio>
 
+#include "fixed_sum.cuh"
 #include "qgpu_internal.h"
-#include "quant.cuh"
 
 namespace qg {
 
@@ -404,9 +404,9 @@ __global__ void __launch_bounds__(256) k_compare(const typename C2<R>::T* __rest
 // Measurement of m distinct qubits without a trip to the host: k_marginal sums every outcome's
 // probability (compensated FP64) and quantised probability (integers), k_measure_pick draws
 // the outcome and k_collapse projects on it. Bound by the FP64 pipe: three instructions per
-// probability, a tree over 16 of them before each TwoSum (20 qubits, three measured: 56 us with
-// a TwoSum per amplitude and an FP64 quantisation), and by launches: the host used to wait for
-// the partial sums of every measurement (about 70 us each).
+// probability, 16 of them summed exactly in fixed point (fixed_sum.cuh) before each TwoSum (20
+// qubits, three measured: 56 us with a TwoSum per amplitude and an FP64 quantisation), and by
+// launches: the host used to wait for the partial sums of every measurement (about 70 us each).
 struct MeasuredBits {
   int m;
   int pos[16];   // the measured bits, ascending
@@ -431,17 +431,24 @@ __global__ void __launch_bounds__(256) k_marginal(const typename C2<R>::T* __res
   unsigned long long qs = 0;
   for (uint64_t t = (uint64_t)blockIdx.x * 4096; t < work; t += (uint64_t)gridDim.x * 4096) {
     double v[16];
+    uint32_t key = 0;
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
       const uint64_t j = t + threadIdx.x + (uint64_t)r * 256;
       v[r] = j < work ? p_of<R>(s[spread(j, f, o)]) : 0.0;
       qs += quant(v[r]);
+      key = max(key, qg_fix_key(v[r]));
     }
+    const int E = qg_fix_exponent(key);
+    int64_t h = 0, l = 0;
 #pragma unroll
-    for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-      for (int r = 0; r < w; ++r) v[r] = __dadd_rn(v[r], v[r + w]);
-    two_sum_acc(acc, v[0]);
+    for (int r = 0; r < 16; ++r) {
+      const qg_fixed x = qg_fix(v[r], E, 0);
+      h += x.h;
+      l += x.l;
+    }
+    two_sum_acc(acc, qg_fix_hi(h, E));
+    acc.c = __dadd_rn(acc.c, qg_fix_lo(l, E));
   }
   const int slot = (int)(o * gridDim.x + blockIdx.x);
   block_reduce_store<256>(acc, d_pm, slot);

@@ -4,8 +4,10 @@ Pauli strings of states with real integer amplitudes (times a power of two): eve
 the result may differ from the exact sum by its own rounding (2^-52, with the final addition's) and
 by what a compensated sum leaves, below 2^-80 of the sum of magnitudes; the terms of most strings
 cancel. Sizes cover one value per tile and less, a tile's edge and several tiles; strings alone, in
-pairs and in larger groups.
+pairs and in larger groups. Outcome probabilities equal the correctly rounded sums of the rounded
+probabilities, and the state after a measurement their scaling, bit for bit.
 """
+import math
 from fractions import Fraction
 
 import numpy as np
@@ -45,3 +47,31 @@ def test_strings_that_cancel(n, precision, bits):
             among = st.hamiltonian([(1.0, t)] + [(0.0, s) for _, s in others])
             for got in (alone, among):
                 assert abs(Fraction(got) - want) <= tol, (t, got, float(want))
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("n,qubits", [(3, [1]), (11, [10, 2]), (13, [0]), (15, [7, 14, 3])])
+def test_measured_probabilities(n, qubits, precision):
+    from qclojure_gb300.state import Context
+
+    rng = np.random.default_rng(60 + n)
+    real = np.float32 if precision == "c64" else np.float64
+    with Context() as ctx, ctx.state(n, precision) as st:
+        for seed in range(1, 17):
+            sv = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+            if n > 8 and seed % 2:  # few amplitudes, all in one thread's groups
+                sv[np.arange(1 << n) % 256 != 5] = 0
+            sv /= np.linalg.norm(sv)
+            st.upload(sv)
+            held = st.download()
+            p = held.real * held.real + held.imag * held.imag
+            got, prob = st.measure(qubits, seed)
+            keep = np.ones(1 << n, bool)
+            for k, q in enumerate(qubits):
+                keep &= ((np.arange(1 << n) >> (n - 1 - q)) & 1) == (got >> k) & 1
+            assert prob == math.fsum(p[keep])
+            f = real(1.0 / math.sqrt(prob))
+            after = st.download()
+            for part in ("real", "imag"):
+                want = np.where(keep, getattr(held, part).astype(real) * f, real(0))
+                assert np.array_equal(getattr(after, part), want)
