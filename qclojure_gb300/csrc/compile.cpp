@@ -393,7 +393,8 @@ void factor_global_phases(std::vector<GOp>* gops, std::vector<int>* measure_at, 
       } else if (rotations && (g.cls == U2_IMAG_ANTI || g.cls == U2_ANTIDIAG)) {
         // [[0, a], [b, 0]] = X diag(b, a): a phase and an X (a Y gate needs no register bit then)
         const cd a(m[2], m[3]), b(m[4], m[5]);
-        if (b != cd(0.0, 0.0)) {
+        // (entries of equal size only: the ratio of others leaves the float range)
+        if (std::norm(a) >= 0.25 * std::norm(b) && std::norm(b) >= 0.25 * std::norm(a) && std::norm(b) > 0x1p-40) {
           const cd r = a / b;
           const int t = g.t;
           f = b;
