@@ -592,10 +592,6 @@ void set_op_operator(TOp* t, const double m[8]) {
   set_op_matrix(t, m);
 }
 
-namespace {
-
-}  // namespace
-
 // Register planning: every thread holds 2^R amplitudes
 // whose local indices differ in R "register bits". Consecutive ops whose
 // non-diagonal bits fit in R bits share one layout; the remaining register bits
@@ -606,6 +602,9 @@ namespace {
 // blockade masks are data (they differ between members, for instance between
 // QAOA graphs), so the layout must not depend on them: ops keep their order
 // (no sinking, no look-ahead) and the free register bits ignore those masks.
+// in_order = true: every amplitude goes through the same products and sums in the same order
+// as without a plan, so its bits are the same. Only permutations move, past ops that touch
+// none of their bits; they round nothing.
 namespace {
 
 bool is_permutation(const TOp& t) {
@@ -622,8 +621,8 @@ struct PlanOp {
   bool perm;
 };
 
-LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool table, bool pair0, PermMode mode,
-                             bool emit) {
+LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool table, bool pair0, bool in_order,
+                             PermMode mode, bool emit) {
   LayoutPlan plan;
   std::vector<TOp>& out = plan.ops;
   if (emit) out.reserve(in.size() * 2 + 1);
@@ -673,7 +672,7 @@ LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool t
         taken[j] = 1;
         if (q.perm) ++plan.moves;
       } else {
-        if (table) break;
+        if (table || (in_order && !q.perm)) break;
         changed |= q.req;
         seen |= q.all;
       }
@@ -754,7 +753,8 @@ LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool t
 // or moves. The weights were measured (layers + QFT, ms; register ops only 50.7 at 28 qubits
 // complex128 and 30.4 at 29 qubits complex64): 10, 3, 1 gives 48.2 and 28.4; 10, 0, 3: 50.6 and
 // 28.9; 10, 6, 3: 48.5 and 28.8; 10, 10, 1: 48.9 and 29.8.
-LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool pair0, int move_cost) {
+LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool pair0, bool in_order,
+                        int move_cost) {
   auto describe = [&](const TOp& t) {
     PlanOp p{&t, 0, 0, 0, false};
     if (t.kind == OK_U2) p.req = 1u << t.t;
@@ -784,7 +784,7 @@ LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool
     const TOp& t = ops[i];
     if (t.kind == OK_LAYOUT) continue;
     const PlanOp p = describe(t);
-    if (t.kind == OK_PHASE && !table) {
+    if (t.kind == OK_PHASE && !table && !in_order) {
       waiting.push_back(p);
       continue;
     }
@@ -798,7 +798,7 @@ LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool
   if (!table && perms) {
     int least = -1;
     for (const PermMode m : {kPermRegisters, kPermBoth, kPermLayouts}) {
-      const LayoutPlan p = plan_layouts_mode(in, k, R, table, pair0, m, false);
+      const LayoutPlan p = plan_layouts_mode(in, k, R, table, pair0, in_order, m, false);
       int mapped = p.last.identity() ? 0 : 1;
       for (const LayoutMap& x : p.maps) mapped += x.identity() ? 0 : 1;
       const int cost = 10 * p.layouts + 3 * mapped + move_cost * p.moves;
@@ -808,23 +808,18 @@ LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool
       }
     }
   }
-  return plan_layouts_mode(in, k, R, table, pair0, mode, true);
+  return plan_layouts_mode(in, k, R, table, pair0, in_order, mode, true);
 }
 
 namespace {
 
-// complex64 states of fewer qubits keep the pass's order and one product per phase: another
-// order moves every FP32 rounding (1e-7), and that shows in the FP64 energies that callers
-// read from states of such sizes. From here on a pass is larger than L2 (2^25 amplitudes:
-// 268 MB) and the plan saves milliseconds: 25 qubits 13.3 ms in order, 7.5 ms planned.
-constexpr int kPlannedC64Qubits = 25;
-
 // The interpreter's records of a planned pass: layouts with the map their registers are read
 // through, the tile-conditioned parts of a map before it, and a map at the end before the
 // registers are written back. A permutation of registers costs the interpreter a dispatch and
-// selects on sixteen values, about as much as a layout change.
-void plan_interpreted(const std::vector<TOp>& ops, int k, std::vector<TOp>* records) {
-  LayoutPlan plan = plan_layouts(ops.data(), (int)ops.size(), k, 3, false, false, 7);
+// selects on sixteen values, about as much as a layout change. in_order: as in plan_layouts,
+// and every phase is a product of its own.
+void plan_interpreted(const std::vector<TOp>& ops, int k, bool in_order, std::vector<TOp>* records) {
+  LayoutPlan plan = plan_layouts(ops.data(), (int)ops.size(), k, 3, false, false, in_order, 7);
   auto blank = [&](int32_t kind) -> TOp& {
     records->emplace_back();
     TOp& t = records->back();
@@ -861,7 +856,7 @@ void plan_interpreted(const std::vector<TOp>& ops, int k, std::vector<TOp>* reco
     // register mask. A single phase is cheaper as an op of its own (noisy circuits, where an
     // operator follows every gate: 4.7 against 5.8 ms of passes).
     size_t j = i;
-    while (j < plan.ops.size() && plan.ops[j].kind == OK_PHASE) ++j;
+    while (!in_order && j < plan.ops.size() && plan.ops[j].kind == OK_PHASE) ++j;
     if (j <= i + 1) {
       records->push_back(t);
       ++i;
@@ -1193,11 +1188,13 @@ int schedule(int n, int precision, int fusion, int fuse_k, const std::vector<GOp
       s.raw_end = (int64_t)prog->raw.size();
     }
     // The exact policy keeps the circuit's order of roundings and sweeps one pass structure
-    // for all members; the others gather commuting ops under fewer layouts and move X, CNOT
-    // and SWAP into the layout changes. complex64 only from kPlannedC64Qubits on.
+    // for all members. The others move X, CNOT and SWAP into the layout changes; double-float
+    // also gathers commuting ops under fewer layouts and multiplies phases together, which
+    // moves roundings of 2^-48. In FP32 they are of 2^-24 and would show in the FP64 energies
+    // and the shots that callers read from complex64 states: those keep the pass's order.
     s.pass.op_begin = (int64_t)prog->tops.size();
-    if (reorder && !dense && (precision != QG_C64 || n >= kPlannedC64Qubits)) {
-      plan_interpreted(pass_ops, s.pass.k, &prog->tops);
+    if (reorder && !dense) {
+      plan_interpreted(pass_ops, s.pass.k, precision == QG_C64, &prog->tops);
     } else {
       plan_register_groups(pass_ops, s.pass.k);
       prog->tops.insert(prog->tops.end(), pass_ops.begin(), pass_ops.end());

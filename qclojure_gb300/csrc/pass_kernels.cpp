@@ -169,7 +169,7 @@ class PassGen {
       if (ops[i].kind == OK_DENSE) unsupported_ = true;
       if (table && (ops[i].kind == OK_BLOCKADE || ops[i].kind == OK_COLLAPSE)) unsupported_ = true;
     }
-    if (!unsupported_) plan_ = plan_layouts(tagged.data(), nops, pd.k, sh_.rbits, table, !df_, 1);
+    if (!unsupported_) plan_ = plan_layouts(tagged.data(), nops, pd.k, sh_.rbits, table, !df_, false, 1);
     // pairs handed over by the previous pass may carry unnormalised operations
     if (io & kTileInPairs) carry_ = kRenormEvery / 2 - 1;
     ops_ = plan_.ops.data();
@@ -1745,7 +1745,7 @@ void pass_coefficients(const Program& prog, size_t step, int prec, float* out) {
   std::vector<TOp> tagged(ops, ops + nops);
   for (int i = 0; i < nops; ++i) tagged[i].pad1 = i;
   const std::vector<TOp> plan =
-      plan_layouts(tagged.data(), nops, pd.k, shape_of(prog, prec).rbits, true, prec == QG_C64, 1).ops;
+      plan_layouts(tagged.data(), nops, pd.k, shape_of(prog, prec).rbits, true, prec == QG_C64, false, 1).ops;
   const int ns = 1 << shape_of(prog, prec).rbits;  // registers per thread
   auto put = [&](float* at, std::complex<double> v) {
     if (prec == QG_C128) {

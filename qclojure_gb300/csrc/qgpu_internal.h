@@ -224,8 +224,9 @@ struct LayoutPlan {
 
 // Plans a pass's ops (k local bits, R register bits). table: members of a sweep share the plan,
 // so it keeps circuit order and ignores parity masks; pair0: complex64 kernels pair registers on
-// tile bit 0; move_cost: of a permutation of registers, against 10 for a layout change.
-LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool pair0, int move_cost);
+// tile bit 0; in_order: ops other than permutations keep their order; move_cost: of a permutation
+// of registers, against 10 for a layout change.
+LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool pair0, bool in_order, int move_cost);
 
 // A compiled step sequence.
 struct Step {

@@ -136,13 +136,7 @@ struct PolExact {
     return r;
   }
   __device__ static V times_i(V x) { V r; r.x = -x.y; r.y = x.x; return r; }
-  __device__ static V minus(V x) { V r; r.x = -x.x; r.y = -x.y; return r; }
-  __device__ static V one() { V r; r.x = 1; r.y = 0; return r; }
-  __device__ static V factor(const uint4& head, const KOp& op, V f);  // the phase of a record times f
-  __device__ static V mul(V f, V x) { return cm(f.x, f.y, x); }
-  // phases of one run are multiplied together before they meet the amplitudes (not in FP64,
-  // which keeps the reference's order of roundings)
-  static constexpr bool kPhaseRuns = kFMA;
+  static constexpr bool kPhaseRuns = false;  // every phase is a product of its own: same bits in any plan
   // entry 0 or 1 of a phase pair (selected without indexing the constant array)
   __device__ static V cmul_idx(const Cst& c, int which, V x) {
     return which ? cm(c.m[2], c.m[3], x) : cm(c.m[0], c.m[1], x);
@@ -242,10 +236,14 @@ struct PolDFT {
     if (CLS == PH_I) return dfc{-x.ih, x.rh, -x.il, x.rl};
     return dfc{x.ih, -x.rh, x.il, -x.rl};
   }
+  // phases of one run are multiplied together before they meet the amplitudes: fewer products,
+  // and states no further from 64 bits (12 layers and a transform, 2-norm, mean of three: 14 qubits
+  // 1.7e-14 one by one, 1.5e-14 in runs; 22 qubits 2.4e-14, 2.0e-14). In FP32, reordered circuits
+  // with runs were 10 to 20 % further off.
   static constexpr bool kPhaseRuns = true;
   __device__ static dfc minus(const dfc& x) { return dfc{-x.rh, -x.ih, -x.rl, -x.il}; }
   __device__ static dfc one() { return dfc{1.f, 0.f, 0.f, 0.f}; }
-  __device__ static dfc factor(const uint4& head, const KOp& op, const dfc& f);
+  __device__ static dfc factor(const KOp& op, const dfc& f);  // the phase of a record times f
   __device__ static dfc mul(const dfc& f, const dfc& x) { return cmul_df(f.rh, f.rl, f.ih, f.il, x); }
   __device__ static dfc times_i(const dfc& x) { return dfc{-x.ih, x.rh, -x.il, x.rl}; }
   __device__ static dfc cmul_idx(const Cst& c, int which, const dfc& x) {
@@ -583,13 +581,8 @@ struct SiteView {
   const KOp* variants;
 };
 
-template <typename R, typename V>
-__device__ __forceinline__ V PolExact<R, V>::factor(const uint4& head, const KOp&, V f) {
-  if constexpr (kFMA) return cm(__uint_as_float(head.z), __uint_as_float(head.w), f);
-  else return f;
-}
 template <int IO, bool DENSE>
-__device__ __forceinline__ dfc PolDFT<IO, DENSE>::factor(const uint4&, const KOp& op, const dfc& f) {
+__device__ __forceinline__ dfc PolDFT<IO, DENSE>::factor(const KOp& op, const dfc& f) {
   const float4 c = *reinterpret_cast<const float4*>(op.c);
   return cmul_df(c.x, c.z, c.y, c.w, f);
 }
@@ -598,14 +591,11 @@ __device__ __forceinline__ dfc PolDFT<IO, DENSE>::factor(const uint4&, const KOp
 // phases whose tile and thread bits hold are multiplied into one factor (powers of i are
 // counted), and the registers that include m take it: one product per phase and thread, where
 // the phases one by one took a dispatch and a product per register each (a controlled phase:
-// four of eight registers of both tiles). Two tiles at a time where r1 is given. The header
-// counts each mask's phases: general ones without tile bits (tiles interpreted together share
-// them), general ones with, then the others; with one loop that took all three, the compiler
-// turned every choice into selects, 70 instructions per phase and pair of tiles (25-qubit
-// complex64 circuit with a transform: 7.41 ms of passes, now 6.74 ms).
-template <class P, bool TWO>
-__device__ __forceinline__ void phase_run(typename P::Reg (&r0)[kRegs], typename P::Reg (&r1)[kRegs],
-                                          const KOp* __restrict__ run, uint64_t base0, uint64_t base1,
+// four of eight registers). The header counts each mask's phases: general ones without tile
+// bits, general ones with, then the others. 22 qubits with a transform: 4.14 ms one by one,
+// 2.94 ms.
+template <class P>
+__device__ __forceinline__ void phase_run(typename P::Reg (&r)[kRegs], const KOp* __restrict__ run, uint64_t base,
                                           uint32_t lt) {
   using Reg = typename P::Reg;
   auto turn = [](Reg x, int pw) {
@@ -614,74 +604,50 @@ __device__ __forceinline__ void phase_run(typename P::Reg (&r0)[kRegs], typename
     return x;
   };
   const KOp* p = run + 1;
-#pragma unroll(P::kDF ? 1 : kRegs)  // DF: eight copies of the loops crowd the instruction cache
+#pragma unroll 1  // eight copies of the loops crowd the instruction cache
   for (int m = 0; m < kRegs; ++m) {
     const uint2 n = reinterpret_cast<const uint2*>(run->c)[m];
     if ((n.x | n.y) == 0) continue;
-    Reg f0 = P::one();
-    int pw0 = 0, pw1 = 0;
-    bool hit0 = false;
+    Reg f = P::one();
+    int pw = 0;
+    bool hit = false;
     const bool general = n.x != 0;
     const KOp* end = p + (n.x & 0xFFFFu);
-#pragma unroll(P::kDF ? 1 : 2)
+#pragma unroll 1
     for (; p < end; ++p) {
       const uint4 head = *reinterpret_cast<const uint4*>(p);
       const bool c = (lt & head.y) == head.y;
-      const Reg g = P::factor(head, *p, f0);
-      if (c) f0 = g;
-      hit0 = hit0 || c;
+      const Reg g = P::factor(*p, f);
+      if (c) f = g;
+      hit = hit || c;
     }
-    Reg f1 = f0;
-    bool hit1 = hit0;
     for (end = p + (n.x >> 16); p < end; ++p) {
       const uint64_t gm = p->gmask;
-      const bool t0 = (base0 & gm) == gm, t1 = TWO && (base1 & gm) == gm;
-      if (!t0 && !t1) continue;
+      if ((base & gm) != gm) continue;
       const uint4 head = *reinterpret_cast<const uint4*>(p);
       const bool c = (lt & head.y) == head.y;
-      const Reg g0 = P::factor(head, *p, f0);
-      if (t0 && c) f0 = g0;
-      hit0 = hit0 || (t0 && c);
-      if (TWO) {
-        const Reg g1 = P::factor(head, *p, f1);
-        if (t1 && c) f1 = g1;
-        hit1 = hit1 || (t1 && c);
-      }
+      const Reg g = P::factor(*p, f);
+      if (c) f = g;
+      hit = hit || c;
     }
     for (end = p + n.y; p < end; ++p) {
       const uint4 head = *reinterpret_cast<const uint4*>(p);
       const uint64_t gm = p->gmask;
       const uint32_t cls = (head.x >> 3) & 3u;
       const int q = (lt & head.y) != head.y ? 0 : cls == PH_NEG ? 2 : cls == PH_I ? 1 : 3;
-      pw0 += (base0 & gm) == gm ? q : 0;
-      if (TWO) pw1 += (base1 & gm) == gm ? q : 0;
+      pw += (base & gm) == gm ? q : 0;
     }
     if (general) {
-      f0 = turn(f0, pw0);
-      if (hit0 || (pw0 & 3)) {
+      f = turn(f, pw);
+      if (hit || (pw & 3)) {
 #pragma unroll
         for (int j = 0; j < kRegs; ++j)
-          if ((j & m) == m) r0[j] = P::mul(f0, r0[j]);
+          if ((j & m) == m) r[j] = P::mul(f, r[j]);
       }
-      if (TWO) {
-        f1 = turn(f1, pw1);
-        if (hit1 || (pw1 & 3)) {
+    } else if (pw & 3) {
 #pragma unroll
-          for (int j = 0; j < kRegs; ++j)
-            if ((j & m) == m) r1[j] = P::mul(f1, r1[j]);
-        }
-      }
-    } else {
-      if (pw0 & 3) {
-#pragma unroll
-        for (int j = 0; j < kRegs; ++j)
-          if ((j & m) == m) r0[j] = turn(r0[j], pw0);
-      }
-      if (TWO && (pw1 & 3)) {
-#pragma unroll
-        for (int j = 0; j < kRegs; ++j)
-          if ((j & m) == m) r1[j] = turn(r1[j], pw1);
-      }
+      for (int j = 0; j < kRegs; ++j)
+        if ((j & m) == m) r[j] = turn(r[j], pw);
     }
   }
 }
@@ -747,7 +713,7 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
     }
     if constexpr (P::kPhaseRuns) {
       if (code == KC_PHASES) {
-        phase_run<P, false>(r, r, rec, base, 0, lt);
+        phase_run<P>(r, rec, base, lt);
         o += (int)head.y;
         continue;
       }
@@ -952,11 +918,6 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
     if (code == KC_MAPX) {
       if ((base0 & op.gmask) == op.gmask) mapx0 ^= head.y;
       if ((base1 & op.gmask) == op.gmask) mapx1 ^= head.y;
-      continue;
-    }
-    if (code == KC_PHASES) {
-      phase_run<P, true>(r0, r1, rec, base0, base1, lt);
-      o += (int)head.y;
       continue;
     }
     if (code == KC_REMAP) {
@@ -1494,13 +1455,8 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
         cond = t.tmask != 0 || t.gmask != 0;
         if (run > 0) {
           --run;
-          if (P::kCst == 1) {  // the factor beside tmask
-            std::memcpy(&k.tval, &k.c[0], 4);
-            std::memcpy(&k.rmr, &k.c[1], 4);
-          } else {  // re.hi, im.hi, re.lo, im.lo
-            k.c[2] = k.c[8];
-            k.c[3] = k.c[9];
-          }
+          k.c[2] = k.c[8];  // re.hi, im.hi, re.lo, im.lo
+          k.c[3] = k.c[9];
         }
         break;
       case OK_SWAP: {
