@@ -1319,7 +1319,7 @@ bool generate_units(const Program& prog, int prec, std::vector<Unit>* units, std
   // one unit per host thread; passes dealt largest first to the smallest unit (the
   // compile time of a pass grows faster than its source, so big passes go alone)
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t nunits = std::min<size_t>(pieces.size(), 2 * std::min(hw, 32u));
+  const size_t nunits = std::min<size_t>(pieces.size(), std::min(hw, 32u));
   units->assign(nunits, Unit());
   std::vector<size_t> load(nunits, 0), order(pieces.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
@@ -1585,7 +1585,7 @@ std::shared_ptr<const PassKernels> level_kernels_for(const std::vector<const Pro
   }
   // units: levels dealt largest first, one unit per host thread
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t nunits = std::min<size_t>(pieces.size(), 2 * std::min(hw, 32u));
+  const size_t nunits = std::min<size_t>(pieces.size(), std::min(hw, 32u));
   std::vector<Unit> units(nunits);
   std::vector<size_t> load(nunits, 0), order(pieces.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
