@@ -493,7 +493,6 @@ TOp localize(const GOp& g, const int* lpos /* abs bit -> local or -1 */, int n) 
   }
   split(g.cmask, &t.lcmask, &t.gcmask);
   split(g.mask, &t.lmask, &t.gmask);
-  split(g.val, &t.lval, &t.gval);
   for (int j = 0; j < g.dk; ++j) t.dbits[j] = lpos[g.dbits[j]];
   return t;
 }
@@ -730,15 +729,11 @@ LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool t
         m = v = t.lcmask;
       } else if (t.kind == OK_PHASE) {
         m = v = t.lmask;
-      } else if (t.kind == OK_COLLAPSE) {
-        m = t.lmask;
-        v = t.lval;
       } else {  // BLOCKADE, PARITY: the mask selects the bits to count
         m = t.lmask;
         v = 0;
       }
       t.rmask = reg_part(m);
-      t.rval = reg_part(v);
       t.tmask = m & ~rb;
       t.tval = v & ~rb;
     }
@@ -788,7 +783,7 @@ LayoutPlan plan_layouts(const TOp* ops, int nops, int k, int R, bool table, bool
       waiting.push_back(p);
       continue;
     }
-    const bool diagonal_other = t.kind == OK_BLOCKADE || t.kind == OK_PARITY || t.kind == OK_COLLAPSE;
+    const bool diagonal_other = t.kind == OK_BLOCKADE || t.kind == OK_PARITY;
     flush(p.req, diagonal_other || t.kind == OK_DENSE);
     in.push_back(p);
     perms = perms || p.perm;
@@ -949,15 +944,11 @@ void plan_register_groups(std::vector<TOp>& ops, int k) {
         m = v = t.lcmask;
       } else if (t.kind == OK_PHASE) {
         m = v = t.lmask;
-      } else if (t.kind == OK_COLLAPSE) {
-        m = t.lmask;
-        v = t.lval;
       } else {  // BLOCKADE, PARITY: the mask selects the bits to count
         m = t.lmask;
         v = 0;
       }
       t.rmask = reg_part(m);
-      t.rval = reg_part(v);
       t.tmask = m & ~rbm;
       t.tval = v & ~rbm;
       out.push_back(t);

@@ -88,16 +88,6 @@ __device__ __forceinline__ void lin2(float ah, float al, float uh, float ul, flo
   yl = t - (yh - s);
 }
 
-// a*u for double-float a, u (normalised result)
-__device__ __forceinline__ void mul1(float ah, float al, float uh, float ul, float& yh, float& yl) {
-  const float p = ah * uh;
-  float e = fmaf(ah, uh, -p);
-  e = fmaf(ah, ul, e);
-  e = fmaf(al, uh, e);
-  yh = p + e;
-  yl = e - (yh - p);
-}
-
 // (xh + xl) + (yh + yl), normalised
 __device__ __forceinline__ void add2(float xh, float xl, float yh, float yl, float& zh, float& zl) {
   const float s = xh + yh;

@@ -167,7 +167,7 @@ class PassGen {
     for (int i = 0; i < nops; ++i) {
       tagged[i].pad1 = i;  // the op's row in the coefficient table
       if (ops[i].kind == OK_DENSE) unsupported_ = true;
-      if (table && (ops[i].kind == OK_BLOCKADE || ops[i].kind == OK_COLLAPSE)) unsupported_ = true;
+      if (table && ops[i].kind == OK_BLOCKADE) unsupported_ = true;
     }
     if (!unsupported_) plan_ = plan_layouts(tagged.data(), nops, pd.k, sh_.rbits, table, !df_, false, 1);
     // pairs handed over by the previous pass may carry unnormalised operations
@@ -667,24 +667,6 @@ class PassGen {
         }
         o_ << "    }\n";
         for (int j = 0; j < ns_; ++j) touched(j);
-      } break;
-      case OK_COLLAPSE: {
-        materialise(cr);
-        const std::string c = cond(t.gmask, t.gval, t.tmask, t.tval);
-        const uint32_t rv = t.rval & (uint32_t)(ns_ - 1);
-        o_ << "    {  // collapse\n      const bool tc = " << (c.empty() ? "true" : c) << ";\n";
-        for (int j = 0; j < ns_; ++j) {
-          if ((j & cr) == rv) {
-            const std::string sc = df_ ? "df_scale<" + b(lo_nz(t, 0)) + ">(" + h(t, 0) + ", " + l(t, 0) + ", " +
-                                             r(j) + ")"
-                                       : "f_scale(" + h(t, 0) + ", " + r(j) + ")";
-            o_ << "      " << r(j) << " = tc ? " << sc << " : " << pol() << "::zero();\n";
-          } else {
-            o_ << "      " << r(j) << " = " << pol() << "::zero();\n";
-          }
-          touched(j);
-        }
-        o_ << "    }\n";
       } break;
       default: break;
     }
@@ -1412,10 +1394,10 @@ std::string pass_structure_key(const Program& prog, int prec, bool table) {
         std::memset(t.m, 0, sizeof(t.m));
         std::memset(t.mf, 0, sizeof(t.mf));
         t.t2 = t.kind == OK_U2 ? 0 : t.t2;
-        t.rmask = t.rval = t.tmask = t.tval = 0;
+        t.rmask = t.tmask = t.tval = 0;
         std::memset(t.dbits, 0, sizeof(t.dbits));
         std::memset(t.lj, 0, sizeof(t.lj));
-        if (t.kind == OK_PARITY) t.lmask = t.lval = 0, t.gmask = t.gval = 0;
+        if (t.kind == OK_PARITY) t.lmask = 0, t.gmask = 0;
         key.append(shape, 5);
       }
       key.append(reinterpret_cast<const char*>(&t), sizeof(TOp));

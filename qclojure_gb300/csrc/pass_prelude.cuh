@@ -218,7 +218,6 @@ struct DF {
     reinterpret_cast<double2*>(b)[pos] = qg::store_dfc(unpack(y));
   }
   static __device__ __forceinline__ V renorm(const V& v) { return unpack(fast2(pack(v))); }
-  static __device__ __forceinline__ V zero() { return dfc{0.f, 0.f, 0.f, 0.f}; }
   static __device__ __forceinline__ V neg(const V& x) { return dfc{-x.rh, -x.ih, -x.rl, -x.il}; }
   static __device__ __forceinline__ V mul_i(const V& x) { return dfc{-x.ih, x.rh, -x.il, x.rl}; }
   static __device__ __forceinline__ V mul_mi(const V& x) { return dfc{x.ih, -x.rh, x.il, -x.rl}; }
@@ -238,11 +237,6 @@ __device__ __forceinline__ dfc df_cmul(float grh, float grl, float gih, float gi
 template <bool AL, bool NEG>
 __device__ __forceinline__ dfc df_cmul_diag(float ah, float al, const dfc& x) {
   return unpack(prod<AL>(konst(ah, al), sum(pack(x), pack(NEG ? DF::mul_mi(x) : DF::mul_i(x)))));
-}
-// a real scalar times x
-template <bool AL>
-__device__ __forceinline__ dfc df_scale(float ah, float al, const dfc& x) {
-  return unpack(prod<AL>(konst(ah, al), pack(x)));
 }
 // y = a*x0 + b*x1 for complex constants a, b (8 floats: a.re h/l, a.im h/l, b.re h/l, b.im h/l)
 __device__ __forceinline__ dfc df_row(float arh, float arl, float aih, float ail, float brh, float brl, float bih,
@@ -340,7 +334,6 @@ struct F32 {
   static __device__ __forceinline__ void st_pair(unsigned char* b, int pos, const V& a, const V& c) {
     *reinterpret_cast<float4*>(b + pos * 8) = make_float4(a.x, a.y, c.x, c.y);
   }
-  static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
   static __device__ __forceinline__ V neg(const V& x) { return make_float2(-x.x, -x.y); }
   static __device__ __forceinline__ V mul_i(const V& x) { return make_float2(-x.y, x.x); }
   static __device__ __forceinline__ V mul_mi(const V& x) { return make_float2(x.y, -x.x); }
@@ -348,7 +341,6 @@ struct F32 {
 __device__ __forceinline__ float2 f_cmul(float gr, float gi, float2 x) {
   return make_float2(fmaf(gr, x.x, -(gi * x.y)), fmaf(gr, x.y, gi * x.x));
 }
-__device__ __forceinline__ float2 f_scale(float a, float2 x) { return make_float2(a * x.x, a * x.y); }
 __device__ __forceinline__ float2 f_row(float ar, float ai, float br, float bi, float2 x0, float2 x1) {
   return make_float2(fmaf(ar, x0.x, fmaf(-ai, x0.y, fmaf(br, x1.x, -(bi * x1.y)))),
                      fmaf(ar, x0.y, fmaf(ai, x0.x, fmaf(br, x1.y, bi * x1.x))));

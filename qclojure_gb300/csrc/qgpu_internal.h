@@ -40,7 +40,6 @@ enum OpKind : int32_t {
   OK_SWAP = 2,      // exchange bits t,t2 where (idx & cmask) == cmask; flags&1: iSWAP phase i
   OK_BLOCKADE = 3,  // amp *= ph where popcount(idx & mask) == 1
   OK_PARITY = 4,    // amp *= (parity(idx & mask) ? ph1 : ph0)
-  OK_COLLAPSE = 5,  // amp = ((idx & mask) == val) ? amp * scale : 0
   OK_DENSE = 6,     // dense 2^dk x 2^dk block on bits dbits[0..dk) (dbits[0] = least significant)
   OK_LAYOUT = 7,    // tiled executor only: registers hold the local bits dbits[0..3) from here on
   OK_NONE = 8,      // tiled executor only: nothing (a noise site whose operator is the identity)
@@ -76,7 +75,6 @@ struct GOp {
   int32_t dk;
   uint64_t cmask;
   uint64_t mask;
-  uint64_t val;
   double m[8];
   int32_t dbits[5];
   int32_t tag;      // 1 + ordinal of the QG_OP_KRAUS operation it came from, 0 otherwise
@@ -96,11 +94,9 @@ struct TOp {
   int32_t dk;
   uint32_t lcmask;   // local control mask
   uint32_t lmask;    // local part of mask
-  uint32_t lval;     // local part of val
   uint32_t tag;      // GOp::tag
   uint64_t gcmask;   // non-local control bits (absolute)
   uint64_t gmask;    // non-local part of mask (absolute)
-  uint64_t gval;     // non-local part of val (absolute)
   double m[8];
   int32_t dbits[5];  // local bit positions of a dense block; register bits of OK_LAYOUT;
                      // register positions (a < b) of OK_SWAP
@@ -108,9 +104,9 @@ struct TOp {
   int64_t doff;
   float mf[16];      // m split into float pairs: hi in mf[0..8), lo in mf[8..16)
   // Tiled executor: the local mask of the op (controls of U2/SWAP, mask of the
-  // diagonal kinds) split into its register positions (3-bit rmask/rval) and its
+  // diagonal kinds) split into its register positions (3-bit rmask) and its
   // thread bits (tmask/tval), so each thread tests one word per op.
-  uint32_t rmask, rval, tmask, tval;
+  uint32_t rmask, tmask, tval;
   uint32_t lj[8];    // OK_LAYOUT: local offset of register slot j
   // OK_LAYOUT, OK_REMAP: the map registers are read or written through (LayoutMap's columns
   // and constant; mapped = 0: the identity). OK_MAPX: mc0 joins the next one's constant on

@@ -141,8 +141,6 @@ struct PolExact {
   __device__ static V cmul_idx(const Cst& c, int which, V x) {
     return which ? cm(c.m[2], c.m[3], x) : cm(c.m[0], c.m[1], x);
   }
-  __device__ static V scale(const Cst& c, V x) { V r; r.x = mulD(x.x, c.m[0]); r.y = mulD(x.y, c.m[0]); return r; }
-  __device__ static V zero() { V r; r.x = 0; r.y = 0; return r; }
 };
 
 using PolD = PolExact<double, double2>;
@@ -250,13 +248,6 @@ struct PolDFT {
     const bool w = which != 0;
     return cmul_df(w ? c.h[2] : c.h[0], w ? c.l[2] : c.l[0], w ? c.h[3] : c.h[1], w ? c.l[3] : c.l[1], x);
   }
-  __device__ static dfc scale(const Cst& c, const dfc& x) {
-    dfc r;
-    mul1(c.h[0], c.l[0], x.rh, x.rl, r.rh, r.rl);
-    mul1(c.h[0], c.l[0], x.ih, x.il, r.ih, r.il);
-    return r;
-  }
-  __device__ static dfc zero() { return dfc{0.f, 0.f, 0.f, 0.f}; }
 };
 
 // XOR swizzle of the shared-memory tile: 16-byte units, 8 per 128-byte row. Linear over the
@@ -335,7 +326,6 @@ enum KCode : int32_t {  // below 16: everything but gates on registers
   KC_SWAP = 56,    // + register pair (0: {0,1}, 1: {0,2}, 2: {1,2}) + 3 * iswap
   KC_BLOCKADE = 62,
   KC_PARITY = 63,
-  KC_COLLAPSE = 64,
   KC_NONE = 65,    // nothing (an identity among a noise site's operators)
   KF_COND = 0x100, // the op has control / mask conditions to evaluate
   KF_MAP = 0x200   // the layout reads its registers through a map
@@ -343,7 +333,7 @@ enum KCode : int32_t {  // below 16: everything but gates on registers
 
 struct __align__(16) KOp {
   int32_t code;
-  uint32_t tmask, tval, rmr;  // thread-bit mask/value, register mask | register value << 8
+  uint32_t tmask, tval, rmr;  // thread-bit mask/value, register mask
   uint64_t gmask, gval;       // non-local mask/value (controls of U2/SWAP: gval = gmask)
   float c[16];                // coefficients: float pairs (hi[8], lo[8]) or 8 doubles (FP64 policy)
 };
@@ -822,11 +812,6 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
           const typename P::Cst c = kcst<P>(op);
 #pragma unroll
           for (int j = 0; j < kRegs; ++j) r[j] = P::cmul_idx(c, par ^ (__popc(j & cr) & 1), r[j]);
-        } else if (k == KC_COLLAPSE) {
-          const typename P::Cst c = kcst<P>(op);
-          const uint32_t rv = (head.w >> 8) & 0xFFu;
-#pragma unroll
-          for (int j = 0; j < kRegs; ++j) r[j] = (tc && (j & cr) == rv) ? P::scale(c, r[j]) : P::zero();
         }
       } break;
     }
@@ -1040,14 +1025,6 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
           for (int j = 0; j < kRegs; ++j) {
             r0[j] = P::cmul_idx(c, par0 ^ (__popc(j & cr) & 1), r0[j]);
             r1[j] = P::cmul_idx(c, par1 ^ (__popc(j & cr) & 1), r1[j]);
-          }
-        } else if (k == KC_COLLAPSE) {
-          const typename P::Cst c = kcst<P>(op);
-          const uint32_t rv = (head.w >> 8) & 0xFFu;
-#pragma unroll
-          for (int j = 0; j < kRegs; ++j) {
-            r0[j] = (tc0 && (j & cr) == rv) ? P::scale(c, r0[j]) : P::zero();
-            r1[j] = (tc1 && (j & cr) == rv) ? P::scale(c, r1[j]) : P::zero();
           }
         }
       } break;
@@ -1427,7 +1404,7 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
     }
     k.tmask = t.tmask;
     k.tval = t.tval;
-    k.rmr = t.rmask | (t.rval << 8);
+    k.rmr = t.rmask;
     bool cond = t.tmask != 0 || t.rmask != 0;
     switch (t.kind) {
       case OK_NONE:
@@ -1476,11 +1453,7 @@ void build_kops(KOp* out, const TOp* ops, int64_t nops) {
         k.gmask = t.gmask;
         cond = true;
         break;
-      default:  // OK_COLLAPSE
-        k.code = KC_COLLAPSE;
-        k.gmask = t.gmask;
-        k.gval = t.gval;
-        cond = true;
+      default:
         break;
     }
     if (cond) k.code |= KF_COND;
