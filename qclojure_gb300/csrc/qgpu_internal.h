@@ -274,7 +274,7 @@ cudaError_t launch_plain_op(void* s, int precision, int n, const GOp& op, cudaSt
 // device (encode_kops) for state 0, indexed by pd's op range; state s uses the
 // records ops_stride further on (0: all states share one list).
 // io (double-float arithmetic only): bit 0 = the state arrives as float pairs
-// (re.hi, re.lo, im.hi, im.lo) written by the previous pass, bit 1 = leave it as
+// (re.hi, im.hi, re.lo, im.lo) written by the previous pass, bit 1 = leave it as
 // float pairs for the next pass; without the bit the state is IEEE doubles.
 constexpr int kTileInPairs = 1, kTileOutPairs = 2;
 // Noisy trajectories: the records of a pass are shared by all states; a record made by

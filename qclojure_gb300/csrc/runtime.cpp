@@ -209,7 +209,11 @@ constexpr int kPassKernelMinQubits = 29;
 // while the device works through the queue, so the compile costs the job nothing.
 constexpr int kPrecompileMinQubits = 20;
 constexpr int kPrecompileThreads = 2;
-constexpr std::chrono::milliseconds kPrecompileWait{250};  // queued for at least this long
+// Queued for at least this long: most backlogs drain sooner, and compiles for them only took host
+// cores from the jobs' own threads. It costs longer ones nothing (circuits/s with and without
+// the wait: 250 jobs of 8-28 qubits at once 38.6 / 38.7, 16 jobs of 27 qubits in complex128 6.2 / 6.2, 100
+// jobs of 22 qubits in complex64 303 / 302).
+constexpr std::chrono::milliseconds kPrecompileWait{250};
 
 static std::shared_ptr<const PassKernels> maybe_pass_kernels(const State* s, const Program& prog);
 static std::shared_ptr<const PassKernels> forced_pass_kernels(const State* s, const Program& prog);
@@ -651,7 +655,8 @@ static bool will_specialise(const Ctx* c, int n, int prec, int arith, int fusion
 // 50-57 % with one CTA on 2^12), which pays for the extra passes from 22 qubits on (layers +
 // QFT: 22 qubits 0.70 against 0.85 ms, 24 qubits 2.60 / 3.13, 28 qubits 44.7 / 51.3 ms); at 20
 // qubits and below, where a pass is a wave or less, fewer passes win (20 qubits 0.28 / 0.25).
-// complex64 passes are nearer to HBM and keep 2^12 (28 qubits: 14.0 ms either way).
+// complex64 passes are nearer to HBM and keep 2^12 (28 qubits: 14.0 ms either way). More passes
+// are more source to compile: preparing a 28-qubit circuit takes 0.84 s, 0.73 s on 2^12 tiles.
 static qg_tuning default_shape(int n, int prec) {
   qg_tuning t;
   std::memset(&t, 0, sizeof(t));
@@ -682,7 +687,9 @@ static std::shared_ptr<const PassKernels> maybe_pass_kernels(const State* s, con
   if (mode == QG_PASS_KERNELS_OFF) return nullptr;
   if (mode != QG_PASS_KERNELS_ALWAYS && s->n < c->spec_min_qubits[s->prec == QG_C64 ? 1 : 0].load()) {
     // below the crossover a one-off program runs interpreted, unless its kernels were
-    // compiled meanwhile (a queued job's background compile, precompile_loop)
+    // compiled meanwhile (a queued job's background compile, precompile_loop). Those are of the
+    // same program, on the interpreter's tiles: whether they are ready is known only now, and
+    // default_shape's smaller tiles would cost a job that still runs interpreted more passes.
     return s->n >= kPrecompileMinQubits ? pass_kernels_cached(prog, s->prec, c->device) : nullptr;
   }
   std::string why;

@@ -137,6 +137,8 @@ struct PolExact {
   }
   __device__ static V times_i(V x) { V r; r.x = -x.y; r.y = x.x; return r; }
   static constexpr bool kPhaseRuns = false;  // every phase is a product of its own: same bits in any plan
+  static constexpr bool kMaps = kFMA;        // layouts through maps: complex64 plans only
+  static constexpr bool kSites = true;
   // entry 0 or 1 of a phase pair (selected without indexing the constant array)
   __device__ static V cmul_idx(const Cst& c, int which, V x) {
     return which ? cm(c.m[2], c.m[3], x) : cm(c.m[0], c.m[1], x);
@@ -147,7 +149,7 @@ using PolD = PolExact<double, double2>;
 using PolF = PolExact<float, float2>;
 
 // ---------------------------------------------------------------------------
-// double-float policy: registers and shared memory hold (re.hi, re.lo, im.hi,
+// double-float policy: registers and shared memory hold (re.hi, im.hi, re.lo,
 // im.lo). Between the passes of one program HBM holds the same pairs (IO bit 0:
 // the input is in pair form, bit 1: the output is written in pair form); the
 // first pass of a run converts from IEEE doubles and the last one back, so the
@@ -238,7 +240,11 @@ struct PolDFT {
   // and states no further from 64 bits (12 layers and a transform, 2-norm, mean of three: 14 qubits
   // 1.7e-14 one by one, 1.5e-14 in runs; 22 qubits 2.4e-14, 2.0e-14). In FP32, reordered circuits
   // with runs were 10 to 20 % further off.
-  static constexpr bool kPhaseRuns = true;
+  static constexpr bool kPhaseRuns = !DENSE;
+  // programs with dense blocks are not planned and have no noise sites; with the code of both in
+  // them, a block of 5 qubits took 14 % longer (26 qubits, two layers: 142.6 and 161.6 ms)
+  static constexpr bool kMaps = !DENSE;
+  static constexpr bool kSites = !DENSE;
   __device__ static dfc minus(const dfc& x) { return dfc{-x.rh, -x.ih, -x.rl, -x.il}; }
   __device__ static dfc one() { return dfc{1.f, 0.f, 0.f, 0.f}; }
   __device__ static dfc factor(const KOp& op, const dfc& f);  // the phase of a record times f
@@ -647,7 +653,10 @@ __device__ __forceinline__ void phase_run(typename P::Reg (&r)[kRegs], const KOp
 // in the order of the record's halves (a bit at a time, and with the swizzle of every register's
 // slot taken here, a layout change cost about 150 integer instructions; 25 qubits complex64: 7.75
 // ms of passes, 7.47 ms with this; 10,000 noisy shots of 10 qubits, with the record heads: 4807 and 4664 us).
-struct ThreadBits {
+template <bool USED>
+struct ThreadBits {};
+template <>
+struct ThreadBits<true> {
   uint32_t w[5];
   __device__ __forceinline__ ThreadBits() {
 #pragma unroll
@@ -657,7 +666,7 @@ struct ThreadBits {
     for (int i = 0; i < 5; ++i) asm volatile("" : "+r"(w[i]));
   }
 };
-__device__ __forceinline__ uint32_t map_of_thread(const KOp& op, const ThreadBits& who, uint32_t (&e)[3]) {
+__device__ __forceinline__ uint32_t map_of_thread(const KOp& op, const ThreadBits<true>& who, uint32_t (&e)[3]) {
   const uint32_t* h = reinterpret_cast<const uint32_t*>(op.c + 8);
   uint32_t m = 0;
 #pragma unroll
@@ -683,21 +692,21 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
   uint32_t lt = 0, mapx = 0;
   // moved: registers were read from other threads' slots, so the next stores wait for all reads
   bool in_regs = false, raw = true, moved = false;
-  const ThreadBits who;
+  const ThreadBits<P::kMaps> who;
   for (int o = 0; o < nops; ++o) {
     const KOp* rec = sops + o;  // shared memory: a broadcast read
     uint4 head = *reinterpret_cast<const uint4*>(rec);  // code, tmask, tval, rmr
     int code = (int)head.x;
     if ((code & 0xFF) < 16) {
     const KOp& op = *rec;
-    if (code == KC_SITE) {
+    if (P::kSites && code == KC_SITE) {
       const uint32_t drawn = __ldg(sv.choices + head.z);
       if ((head.y >> drawn) & 1u) continue;  // the identity
       rec = sv.variants + ((size_t)head.z * 4 + drawn);
       head = *reinterpret_cast<const uint4*>(rec);
       code = (int)head.x;
     } else {
-    if (code == KC_MAPX) {
+    if (P::kMaps && code == KC_MAPX) {
       if ((base & op.gmask) == op.gmask) mapx ^= head.y;
       continue;
     }
@@ -708,13 +717,15 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
         continue;
       }
     }
-    if (code == KC_REMAP) {
-      uint32_t e[3];
-      const uint32_t m = map_of_thread(op, who, e) ^ mapx;
+    if constexpr (P::kMaps) {
+      if (code == KC_REMAP) {
+        uint32_t e[3];
+        const uint32_t m = map_of_thread(op, who, e) ^ mapx;
 #pragma unroll
-      for (int j = 0; j < kRegs; ++j) pos[j] = (int)map_slot(m, e, j);
-      moved = true;  // the slots are other threads' whatever the layout read
-      continue;
+        for (int j = 0; j < kRegs; ++j) pos[j] = (int)map_slot(m, e, j);
+        moved = true;  // the slots are other threads' whatever the layout read
+        continue;
+      }
     }
     if ((code & 0xFF) == KC_LAYOUT) {
       if (in_regs) {
@@ -732,11 +743,13 @@ __device__ void run_ops(unsigned char* buf, const KOp* __restrict__ sops, int no
       const int at = swz<E>((int)lt);
 #pragma unroll
       for (int j = 0; j < kRegs; ++j) pos[j] = at ^ __float_as_int(op.c[j]);
-      moved = (code & KF_MAP) != 0;
       uint32_t m = 0, e[3] = {0, 0, 0};
-      if (moved) {
-        m = map_of_thread(op, who, e) ^ mapx;
-        mapx = 0;
+      if constexpr (P::kMaps) {
+        moved = (code & KF_MAP) != 0;
+        if (moved) {
+          m = map_of_thread(op, who, e) ^ mapx;
+          mapx = 0;
+        }
       }
       auto from = [&](int j) { return moved ? (int)map_slot(m, e, j) : pos[j]; };
       if (raw) {
@@ -886,7 +899,7 @@ __device__ void run_ops2(unsigned char* buf0, unsigned char* buf1, const KOp* __
   uint32_t lt = 0, mapx0 = 0, mapx1 = 0;
   int apart = 0;  // the slots of tile 1 against tile 0's (a map's tile-conditioned parts)
   bool in_regs = false, moved = false;
-  const ThreadBits who;
+  const ThreadBits<true> who;
   for (int o = 0; o < nops; ++o) {
     const KOp* rec = sops + o;
     uint4 head = *reinterpret_cast<const uint4*>(rec);
