@@ -633,6 +633,7 @@ LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool t
   std::vector<char> taken(in.size(), 0);
   std::vector<int> grp;
   size_t first = 0;
+  const uint32_t all = (1u << k) - 1;
   LayoutMap map;  // permutations since the last layout
   bool pending = false;
   while (first < in.size() || pending) {
@@ -649,6 +650,7 @@ LayoutPlan plan_layouts_mode(const std::vector<PlanOp>& in, int k, int R, bool t
         } else {
           changed |= q.req;
           seen |= q.all;
+          if (seen == all) break;  // every permutation changes a bit
         }
       }
       while (first < in.size() && taken[first]) ++first;
