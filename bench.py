@@ -590,11 +590,11 @@ def main():
     mean_pass = statistics.mean(dom) if dom else float("nan")
     achieved = pass_bytes / (mean_pass / 1e3) / 1e9 if dom else float("nan")
     # DRAM bytes per tiled pass from an ncu capture of the same kernel on a 26-qubit state
-    # (dram__bytes_read.sum + dram__bytes_write.sum = 2.087e9 per c128 launch, 1.012e9 per c64
+    # (dram__bytes_read.sum + dram__bytes_write.sum = 2.086e9 per c128 launch, 1.012e9 per c64
     # launch), scaled by the amplitudes processed
     traffic, traffic_src = None, None
     if args.fusion == "tiled":
-        traffic = (2.087e9 if args.precision == "c128" else 1.012e9) * 2 ** (n - 26)
+        traffic = (2.086e9 if args.precision == "c128" else 1.012e9) * 2 ** (n - 26)
         traffic_src = "ncu capture at 26 qubits x 2^(n-26)"
     # time of the 40 random layers alone, per layer
     st.prepare(layers_only, fusion=args.fusion)
